@@ -33,24 +33,12 @@ struct AmdRing {
     }
 };
 
-// spacing quotients: a / (c(e) - c(e-1)) and a / (c(e) - c(e-1))^2, divided
-// as the reference does in FP64, multiplied by the stored reciprocal in FP32
+// Reciprocal spacings of one column and plane and their squares: faces (x, y,
+// z: the cell's own spacing) and centres on its two sides (g0 below, g1 above).
 template <typename T>
-struct Sp {
-    const T *c, *r;
-    __device__ __forceinline__ T q1(T a, int e) const {
-        if constexpr (sizeof(T) == 8) return a / (c[e] - c[e - 1]);
-        else return a * r[e];
-    }
-    __device__ __forceinline__ T q2(T a, int e) const {
-        if constexpr (sizeof(T) == 8) {
-            const T d = c[e] - c[e - 1];
-            return a / (d * d);
-        } else {
-            const T q = r[e];
-            return a * (q * q);
-        }
-    }
+struct AmdGeo {
+    T x, y, z, xg[2], yg[2], zg[2];
+    T x2, y2, z2, xg2[2], yg2[2], zg2[2];
 };
 
 // -C num/den at one canonical centre (subgrid.f90:658-868), clipped with
@@ -60,89 +48,62 @@ struct Sp {
 //   vx[a][b] = V(i+a, j+b-1) - V(i+a-1, j+b-1);  vz[b][c] = V(j+b-1, k+c) - V(j+b-1, k+c-1);
 //   wz = W(k)-W(k-1);  wx[a][c] = W(i+a, k+c-1) - W(i+a-1, k+c-1);
 //   wy[b][c] = W(j+b, k+c-1) - W(j+b-1, k+c-1).
-// compute_Sij (subgrid.f90:891-949) takes its edge values from the same
-// differences.
+// The reference only ever combines the two differences of one side (the two
+// faces of their component) as their sum (p) and the sum of their squares
+// (q); every term is formed from these twelve pairs:
+//   8 S12 = p(uy,0) ryg0 + p(uy,1) ryg1 + p(vx,0) rxg0 + p(vx,1) rxg1 (compute_Sij, subgrid.f90:891-949),
+//   den = (d r)^2 of the diagonal ones + 1/4 sum q r^2 of the others (subgrid.f90:662-763),
+//   num: S11 (ux^2 + 1/4 (q(uy) + q(uz))) and its like, and
+//   2 S12 (1/4 (p(vx) ux + p(uy) vy) + 1/8 (p(uz,0) p(vz,0) + p(uz,1) p(vz,1))) and its like
+//   (subgrid.f90:660-866).
+// About 150 operations a cell; the spacing quotients are products with
+// reciprocals formed once (54 of them per cell: as FP64 divisions they were
+// three quarters of the FP64 instructions, and FP64 instructions are what
+// the FP64 pass is bound by).
 template <typename T, typename A>
-__device__ __forceinline__ T amd_point(const Sp<T> &sx, const Sp<T> &sxg, const Sp<T> &sy, const Sp<T> &syg,
-                                       const Sp<T> &sz, const Sp<T> &szg, const A &U, const A &V, const A &W, int i,
-                                       int j, int k) {
-    const T h = T(0.5), q = T(0.25), two = T(2);
+__device__ __forceinline__ T amd_point(const AmdGeo<T> &g, const A &U, const A &V, const A &W, int i, int j, int k) {
+    const T q4 = T(0.25), two = T(2);
     const T ux = U(i, j, k) - U(i - 1, j, k);
     const T vy = V(i, j, k) - V(i, j - 1, k);
     const T wz = W(i, j, k) - W(i, j, k - 1);
-    T uy[2][2], uz[2][2], vx[2][2], vz[2][2], wx[2][2], wy[2][2];
+    // sums and sums of squares of the two differences of each side
+    T puy[2], puz[2], pvx[2], pvz[2], pwx[2], pwy[2], quy[2], quz[2], qvx[2], qvz[2], qwx[2], qwy[2];
+    auto pair = [](T a, T b, T &p, T &q) {
+        p = a + b;
+        q = a * a + b * b;
+    };
 #pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            uy[a][b] = U(i + a - 1, j + b, k) - U(i + a - 1, j + b - 1, k);
-            uz[a][b] = U(i + a - 1, j, k + b) - U(i + a - 1, j, k + b - 1);
-            vx[a][b] = V(i + a, j + b - 1, k) - V(i + a - 1, j + b - 1, k);
-            vz[a][b] = V(i, j + a - 1, k + b) - V(i, j + a - 1, k + b - 1);
-            wx[a][b] = W(i + a, j, k + b - 1) - W(i + a - 1, j, k + b - 1);
-            wy[a][b] = W(i, j + a, k + b - 1) - W(i, j + a - 1, k + b - 1);
-        }
-    auto av = [h](T p, T r) { return h * (p + r); };
-    // Sij at the centre
-    const T s11 = sx.q1(ux, i), s22 = sy.q1(vy, j), s33 = sz.q1(wz, k);
-    T e4[2][2], e5[2][2], e6[2][2];
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            e4[a][b] = h * (syg.q1(uy[a][b], j + b) + sxg.q1(vx[a][b], i + a));
-            e5[a][b] = h * (szg.q1(uz[a][b], k + b) + sxg.q1(wx[a][b], i + a));
-            e6[a][b] = h * (szg.q1(vz[a][b], k + b) + syg.q1(wy[a][b], j + a));
-        }
-    const T s12 = q * (e4[0][0] + e4[1][0] + e4[0][1] + e4[1][1]);
-    const T s13 = q * (e5[0][0] + e5[1][0] + e5[0][1] + e5[1][1]);
-    const T s23 = q * (e6[0][0] + e6[1][0] + e6[0][1] + e6[1][1]);
-
-    // (d_i u_j)(d_i u_j): term_4 (subgrid.f90:662-763)
-    T den = sx.q2(ux * ux, i);
-    den = den + av(av(syg.q2(uy[0][0] * uy[0][0], j), syg.q2(uy[1][0] * uy[1][0], j)),
-                   av(syg.q2(uy[0][1] * uy[0][1], j + 1), syg.q2(uy[1][1] * uy[1][1], j + 1)));
-    den = den + av(av(szg.q2(uz[0][0] * uz[0][0], k), szg.q2(uz[1][0] * uz[1][0], k)),
-                   av(szg.q2(uz[0][1] * uz[0][1], k + 1), szg.q2(uz[1][1] * uz[1][1], k + 1)));
-    den = den + sy.q2(vy * vy, j);
-    den = den + av(av(sxg.q2(vx[0][0] * vx[0][0], i), sxg.q2(vx[0][1] * vx[0][1], i)),
-                   av(sxg.q2(vx[1][0] * vx[1][0], i + 1), sxg.q2(vx[1][1] * vx[1][1], i + 1)));
-    den = den + av(av(szg.q2(vz[0][0] * vz[0][0], k), szg.q2(vz[1][0] * vz[1][0], k)),
-                   av(szg.q2(vz[0][1] * vz[0][1], k + 1), szg.q2(vz[1][1] * vz[1][1], k + 1)));
-    den = den + sz.q2(wz * wz, k);
-    den = den + av(av(sxg.q2(wx[0][0] * wx[0][0], i), sxg.q2(wx[0][1] * wx[0][1], i)),
-                   av(sxg.q2(wx[1][0] * wx[1][0], i + 1), sxg.q2(wx[1][1] * wx[1][1], i + 1)));
-    den = den + av(av(syg.q2(wy[0][0] * wy[0][0], j), syg.q2(wy[0][1] * wy[0][1], j)),
-                   av(syg.q2(wy[1][0] * wy[1][0], j + 1), syg.q2(wy[1][1] * wy[1][1], j + 1)));
-
-    // (d_hat_k u_i)(d_hat_k u_j) S_ij: nu_t_ (subgrid.f90:660-866)
-    auto s2 = [](T p) { return p * p; };
-    T num = s2(ux) * s11;
-    num = num + av(av(s2(uy[0][0]), s2(uy[1][0])), av(s2(uy[0][1]), s2(uy[1][1]))) * s11;
-    num = num + av(av(s2(uz[0][0]), s2(uz[1][0])), av(s2(uz[0][1]), s2(uz[1][1]))) * s11;
-    num = num + s2(vy) * s22;
-    num = num + av(av(s2(vx[0][0]), s2(vx[0][1])), av(s2(vx[1][0]), s2(vx[1][1]))) * s22;
-    num = num + av(av(s2(vz[0][0]), s2(vz[1][0])), av(s2(vz[0][1]), s2(vz[1][1]))) * s22;
-    num = num + s2(wz) * s33;
-    num = num + av(av(s2(wx[0][0]), s2(wx[0][1])), av(s2(wx[1][0]), s2(wx[1][1]))) * s33;
-    num = num + av(av(s2(wy[0][0]), s2(wy[0][1])), av(s2(wy[1][0]), s2(wy[1][1]))) * s33;
-    // S12 (subgrid.f90:769-800)
-    num = num + two * (av(av(vx[0][0], vx[0][1]), av(vx[1][0], vx[1][1])) * ux) * s12;
-    num = num + two * (av(av(uy[0][0], uy[1][0]), av(uy[0][1], uy[1][1])) * vy) * s12;
-    num = num + two * av(av(uz[0][0], uz[1][0]) * av(vz[0][0], vz[1][0]), av(uz[0][1], uz[1][1]) * av(vz[0][1], vz[1][1])) * s12;
-    // S13 (subgrid.f90:802-833)
-    num = num + two * (av(av(wx[0][0], wx[0][1]), av(wx[1][0], wx[1][1])) * ux) * s13;
-    num = num + two * (av(av(uz[0][0], uz[1][0]), av(uz[0][1], uz[1][1])) * wz) * s13;
-    num = num + two * av(av(uy[0][0], uy[1][0]) * av(wy[0][0], wy[0][1]), av(uy[0][1], uy[1][1]) * av(wy[1][0], wy[1][1])) * s13;
-    // S23 (subgrid.f90:835-866)
-    num = num + two * (av(av(wy[0][0], wy[0][1]), av(wy[1][0], wy[1][1])) * vy) * s23;
-    num = num + two * (av(av(vz[0][0], vz[1][0]), av(vz[0][1], vz[1][1])) * wz) * s23;
-    num = num + two * av(av(vx[0][0], vx[0][1]) * av(wx[0][0], wx[0][1]), av(vx[1][0], vx[1][1]) * av(wx[1][0], wx[1][1])) * s23;
+    for (int s = 0; s < 2; s++) {
+        pair(U(i - 1, j + s, k) - U(i - 1, j + s - 1, k), U(i, j + s, k) - U(i, j + s - 1, k), puy[s], quy[s]);
+        pair(U(i - 1, j, k + s) - U(i - 1, j, k + s - 1), U(i, j, k + s) - U(i, j, k + s - 1), puz[s], quz[s]);
+        pair(V(i + s, j - 1, k) - V(i + s - 1, j - 1, k), V(i + s, j, k) - V(i + s - 1, j, k), pvx[s], qvx[s]);
+        pair(V(i, j - 1, k + s) - V(i, j - 1, k + s - 1), V(i, j, k + s) - V(i, j, k + s - 1), pvz[s], qvz[s]);
+        pair(W(i + s, j, k - 1) - W(i + s - 1, j, k - 1), W(i + s, j, k) - W(i + s - 1, j, k), pwx[s], qwx[s]);
+        pair(W(i, j + s, k - 1) - W(i, j + s - 1, k - 1), W(i, j + s, k) - W(i, j + s - 1, k), pwy[s], qwy[s]);
+    }
+    const T ux2 = ux * ux, vy2 = vy * vy, wz2 = wz * wz;
+    T den = quy[0] * g.yg2[0] + quy[1] * g.yg2[1] + quz[0] * g.zg2[0] + quz[1] * g.zg2[1] + qvx[0] * g.xg2[0] +
+            qvx[1] * g.xg2[1] + qvz[0] * g.zg2[0] + qvz[1] * g.zg2[1] + qwx[0] * g.xg2[0] + qwx[1] * g.xg2[1] +
+            qwy[0] * g.yg2[0] + qwy[1] * g.yg2[1];
+    den = ux2 * g.x2 + vy2 * g.y2 + wz2 * g.z2 + q4 * den;
+    T num = (ux * g.x) * (ux2 + q4 * ((quy[0] + quy[1]) + (quz[0] + quz[1])));
+    num += (vy * g.y) * (vy2 + q4 * ((qvx[0] + qvx[1]) + (qvz[0] + qvz[1])));
+    num += (wz * g.z) * (wz2 + q4 * ((qwx[0] + qwx[1]) + (qwy[0] + qwy[1])));
+    // 8 S_ij of the mixed components times 8 times their factors
+    const T t12 = puy[0] * g.yg[0] + puy[1] * g.yg[1] + pvx[0] * g.xg[0] + pvx[1] * g.xg[1];
+    const T t13 = puz[0] * g.zg[0] + puz[1] * g.zg[1] + pwx[0] * g.xg[0] + pwx[1] * g.xg[1];
+    const T t23 = pvz[0] * g.zg[0] + pvz[1] * g.zg[1] + pwy[0] * g.yg[0] + pwy[1] * g.yg[1];
+    const T sUy = puy[0] + puy[1], sUz = puz[0] + puz[1], sVx = pvx[0] + pvx[1], sVz = pvz[0] + pvz[1],
+            sWx = pwx[0] + pwx[1], sWy = pwy[0] + pwy[1];
+    T off = t12 * (two * (sVx * ux + sUy * vy) + (puz[0] * pvz[0] + puz[1] * pvz[1]));
+    off += t13 * (two * (sWx * ux + sUz * wz) + (puy[0] * pwy[0] + puy[1] * pwy[1]));
+    off += t23 * (two * (sWy * vy + sVz * wz) + (pvx[0] * pwx[0] + pvx[1] * pwx[1]));
+    num += T(1.0 / 32.0) * off;
     const T v = -T(0.3) * num / den;
     return v > T(0) ? v : T(0);
 }
 
-template <typename T> struct AmdMinB { static constexpr int v = sizeof(T) == 4 ? 2 : 1; };
+template <typename T> struct AmdMinB { static constexpr int v = 2; };
 
 // nu_t at the canonical cells and at every duplicate / ghost position that
 // the periodic copies (boundary_conditions.f90:87-244) and the wall rule
@@ -161,7 +122,25 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int i = i0 + tx, j = j0 + ty;
     const bool on = i <= nxp + 1 && j <= nyg - 1;
-    const Sp<T> sx{g.x, rc.dx}, sxg{g.xg, rc.dxg}, sy{g.y, rc.dy}, syg{g.yg, rc.dyg}, sz{g.z, rc.dz}, szg{g.zg, rc.dzg};
+    // this column's reciprocal spacings (the last entries of the tables stand
+    // in for columns and rows past the field, whose results are not stored)
+    AmdGeo<T> ag;
+    {
+        const int ii = min(i, nx - 1), jj = min(j, nyg - 1);
+        ag.x = rc.dx[ii];
+        ag.y = rc.dy[jj];
+        ag.x2 = ag.x * ag.x;
+        ag.y2 = ag.y * ag.y;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            ag.xg[s] = rc.dxg[ii + s];
+            ag.yg[s] = rc.dyg[jj + s];
+            ag.xg2[s] = ag.xg[s] * ag.xg[s];
+            ag.yg2[s] = ag.yg[s] * ag.yg[s];
+        }
+        ag.zg[1] = rc.dzg[kb];
+        ag.zg2[1] = ag.zg[1] * ag.zg[1];
+    }
     // wall rule 2: -nu_t(2) + 2 0.38 dPdx^(1/2) (y(2)-y(1))/2
     T add = T(0);
     if (wall_rule == 2) add = (T)(2.0 * 0.38 * sqrt(ds->dPdx) * ((double)g.y[2] - (double)g.y[1]) / 2.0);
@@ -208,6 +187,13 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
     int sm1 = 0, s0 = 1, sp1 = 2;
     for (int k = kb; k <= ke; k++) {
         if (k + 1 <= ke) fetch(k + 2);  // in flight during this plane's work
+        // the spacings of plane k (the lower centre spacing carried)
+        ag.zg[0] = ag.zg[1];
+        ag.zg2[0] = ag.zg2[1];
+        ag.zg[1] = rc.dzg[k + 1];
+        ag.zg2[1] = ag.zg[1] * ag.zg[1];
+        ag.z = rc.dz[k];
+        ag.z2 = ag.z * ag.z;
         if (on) {
             AmdRing<T> aU, aV, aW;
             aU.b[0] = ring[sm1][0]; aU.b[1] = ring[s0][0]; aU.b[2] = ring[sp1][0];
@@ -216,7 +202,7 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
             aU.i0 = aV.i0 = aW.i0 = i0;
             aU.j0 = aV.j0 = aW.j0 = j0;
             aU.kc = aV.kc = aW.kc = k;
-            const T v = amd_point<T, AmdRing<T>>(sx, sxg, sy, syg, sz, szg, aU, aV, aW, i, j, k);
+            const T v = amd_point<T, AmdRing<T>>(ag, aU, aV, aW, i, j, k);
             if constexpr (sizeof(T) == 8) accd += v;
             else accf += v;
             const T gv = wall_rule == 0 ? v : -v + add;
