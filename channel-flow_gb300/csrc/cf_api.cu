@@ -333,6 +333,8 @@ static int tri_factor(cf_ctx *ctx) {
     CF_CUDA(cudaMemcpy(ctx->tri_fac, F.data(), F.size() * sizeof(double), cudaMemcpyHostToDevice));
     CF_CUDA(cudaMalloc(&ctx->tri_piv, piv.size()));
     CF_CUDA(cudaMemcpy(ctx->tri_piv, piv.data(), piv.size(), cudaMemcpyHostToDevice));
+    CF_CUDA(cudaMalloc(&ctx->tri_flag, NM));
+    CF_CUDA(cudaMemcpy(ctx->tri_flag, flag.data(), NM, cudaMemcpyHostToDevice));
     if (split) {
         // without pivoting zgtsv leaves du untouched: the Dyy upper diagonal
         std::vector<float> du32(nym);
@@ -347,8 +349,6 @@ static int tri_factor(cf_ctx *ctx) {
         CF_CUDA(cudaMemcpy(ctx->tri_ru32, ru32.data(), nf * sizeof(float), cudaMemcpyHostToDevice));
         CF_CUDA(cudaMalloc(&ctx->tri_du32, nym * sizeof(float)));
         CF_CUDA(cudaMemcpy(ctx->tri_du32, du32.data(), nym * sizeof(float), cudaMemcpyHostToDevice));
-        CF_CUDA(cudaMalloc(&ctx->tri_flag, NM));
-        CF_CUDA(cudaMemcpy(ctx->tri_flag, flag.data(), NM, cudaMemcpyHostToDevice));
         CF_CUDA(cudaMalloc(&ctx->tri_list, std::max<size_t>(1, list.size()) * sizeof(int)));
         if (!list.empty())
             CF_CUDA(cudaMemcpy(ctx->tri_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice));

@@ -251,11 +251,11 @@ struct cf_ctx {
     double *d_tri = nullptr;           // Dd, Dl, Du (nym each), kxx (nxp), kzz (nzp)
     double *tri_fac = nullptr;         // zgtsv factors [row][mode]: m, 1/d, du, dl
     unsigned char *tri_piv = nullptr;  // zgtsv pivot flags [row][mode]
+    unsigned char *tri_flag = nullptr; // 1: mode pivots somewhere
     // split path: FP32 LU factors of the modes whose elimination never pivots
     float *tri_l32 = nullptr;          // multipliers [row][mode]
     float *tri_ru32 = nullptr;         // 1/d [row][mode]
     float *tri_du32 = nullptr;         // Dyy upper diagonal [row] (shared by all modes)
-    unsigned char *tri_flag = nullptr; // 1: mode pivots somewhere (FP64 replay)
     int *tri_list = nullptr;           // the flagged modes
     int n_tri_list = 0;
     double *d_tw = nullptr;            // twiddles: x fwd, x bwd, z fwd, z bwd

@@ -908,67 +908,132 @@ struct TriFac {
     const unsigned char *piv;        // [nym][NM]
 };
 
-// FP64 replay, one 32-thread block per mode (all modes, or the modes of
-// `list`): the warp stages the mode's right-hand side and factors in shared
-// memory with independent loads, then lane 0 runs the serial recurrence out
-// of shared memory.
-template <typename T>
-__global__ void __launch_bounds__(32) k_tri_mode(typename C2<T>::t *__restrict__ spec, TriFac f, int nym, long NM,
-                                                 const int *__restrict__ list) {
-    typedef typename C2<T>::t C;
-    extern __shared__ double tsm[];
-    double *br = tsm, *bi = br + nym, *fm = bi + nym, *frd = fm + nym, *fdu = frd + nym, *fdl = fdu + nym;
-    unsigned char *fp = (unsigned char *)(fdl + nym);
-    const long mo = list ? list[blockIdx.x] : blockIdx.x;
-    for (int q = threadIdx.x; q < nym; q += 32) {
-        const long o = (long)q * NM + mo;
-        C v = spec[o];
-        br[q] = v.x;
-        bi[q] = v.y;
-        fm[q] = f.m[o];
-        frd[q] = f.rd[o];
-        fdu[q] = f.du[o];
-        fdl[q] = f.dl[o];
-        fp[q] = f.piv[o];
-    }
-    __syncwarp();
-    if (threadIdx.x == 0) {
-        double r0 = br[0], i0 = bi[0];
-        for (int q = 0; q < nym - 1; q++) {
-            double nre = br[q + 1], nim = bi[q + 1], m = fm[q];
-            if (fp[q]) {
-                br[q] = nre;
-                bi[q] = nim;
-                nre = r0 - m * nre;
-                nim = i0 - m * nim;
-            } else {
-                br[q] = r0;
-                bi[q] = i0;
-                nre = nre - m * r0;
-                nim = nim - m * i0;
+// FP64 replay, one thread per mode, 32 adjacent modes per block: a warp's
+// accesses to a row are coalesced, and the rows of the next TRI_RB are loaded
+// while the recurrence works on the current ones (a row costs one dependent
+// FP64 operation forward and two backward).  The eliminated right-hand side
+// stays in place in the spectrum.  PIV: some mode of the warp pivots; without,
+// zgtsv's elimination leaves the upper diagonal at Dyy's (duc, the same for
+// every mode), dl is zero and the flags need not be read, so that a mode and
+// row moves 80 bytes instead of 97.  Six FP64 instructions per mode and row
+// (2.4 M mode-rows at Re_tau 550: 23 us of the FP64 pipe); one lane per
+// 32-thread block running the recurrence issued as many per warp as this
+// does for 32 modes.
+constexpr int TRI_RB = 8;
+
+template <bool PIV>
+__device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const TriFac &f, const double *__restrict__ duc,
+                                           int nym, long NM, long mo) {
+    double2 *const sp = spec + mo;
+    const double *const fm = f.m + mo, *const frd = f.rd + mo, *const fdu = f.du + mo, *const fdl = f.dl + mo;
+    const unsigned char *const fp = f.piv + mo;
+    double2 nb[TRI_RB];
+    double nm[TRI_RB];
+    unsigned char np[TRI_RB];
+    // rows q0+1 .. q0+TRI_RB of the right-hand side and the multipliers above them
+    auto load_f = [&](int q0) {
+#pragma unroll
+        for (int r = 0; r < TRI_RB; r++) {
+            const int q = q0 + r;
+            if (q < nym - 1) {
+                nb[r] = sp[(long)(q + 1) * NM];
+                nm[r] = fm[(long)q * NM];
+                if constexpr (PIV) np[r] = fp[(long)q * NM];
             }
-            r0 = nre;
-            i0 = nim;
         }
-        double x1r = r0 * frd[nym - 1], x1i = i0 * frd[nym - 1], x2r = 0.0, x2i = 0.0;
-        br[nym - 1] = x1r;
-        bi[nym - 1] = x1i;
-        for (int q = nym - 2; q >= 0; q--) {
-            double yr = (br[q] - fdu[q] * x1r - fdl[q] * x2r) * frd[q];
-            double yi = (bi[q] - fdu[q] * x1i - fdl[q] * x2i) * frd[q];
-            br[q] = yr;
-            bi[q] = yi;
-            x2r = x1r;
-            x2i = x1i;
-            x1r = yr;
-            x1i = yi;
+    };
+    double2 c = sp[0];
+    load_f(0);
+    for (int q0 = 0; q0 < nym - 1; q0 += TRI_RB) {
+        double2 b[TRI_RB];
+        double m[TRI_RB];
+        unsigned char p[TRI_RB];
+#pragma unroll
+        for (int r = 0; r < TRI_RB; r++) {
+            b[r] = nb[r];
+            m[r] = nm[r];
+            if constexpr (PIV) p[r] = np[r];
+        }
+        load_f(q0 + TRI_RB);
+#pragma unroll
+        for (int r = 0; r < TRI_RB; r++) {
+            const int q = q0 + r;
+            if (q < nym - 1) {
+                double2 o = c, x = b[r];
+                if constexpr (PIV) {
+                    if (p[r]) {
+                        o = b[r];
+                        x = c;
+                    }
+                }
+                sp[(long)q * NM] = o;
+                c.x = x.x - m[r] * o.x;
+                c.y = x.y - m[r] * o.y;
+            }
         }
     }
-    __syncwarp();
-    for (int q = threadIdx.x; q < nym; q += 32) spec[(long)q * NM + mo] = cmk<C>(br[q], bi[q]);
+    double rl = frd[(long)(nym - 1) * NM];
+    double2 x1 = make_double2(c.x * rl, c.y * rl), x2 = make_double2(0.0, 0.0);
+    sp[(long)(nym - 1) * NM] = x1;
+    double nu[TRI_RB], nl[TRI_RB];
+    auto load_b = [&](int q0) {  // rows q0, q0 - 1, ..
+#pragma unroll
+        for (int r = 0; r < TRI_RB; r++) {
+            const int q = q0 - r;
+            if (q >= 0) {
+                nb[r] = sp[(long)q * NM];
+                nm[r] = frd[(long)q * NM];
+                if constexpr (PIV) {
+                    nu[r] = fdu[(long)q * NM];
+                    nl[r] = fdl[(long)q * NM];
+                } else {
+                    nu[r] = duc[q];
+                }
+            }
+        }
+    };
+    load_b(nym - 2);
+    for (int q0 = nym - 2; q0 >= 0; q0 -= TRI_RB) {
+        double2 b[TRI_RB];
+        double rd[TRI_RB], du[TRI_RB], dl[TRI_RB];
+#pragma unroll
+        for (int r = 0; r < TRI_RB; r++) {
+            b[r] = nb[r];
+            rd[r] = nm[r];
+            du[r] = nu[r];
+            if constexpr (PIV) dl[r] = nl[r];
+        }
+        load_b(q0 - TRI_RB);
+#pragma unroll
+        for (int r = 0; r < TRI_RB; r++) {
+            const int q = q0 - r;
+            if (q >= 0) {
+                double2 y;
+                if constexpr (PIV) {
+                    y.x = ((b[r].x - dl[r] * x2.x) - du[r] * x1.x) * rd[r];
+                    y.y = ((b[r].y - dl[r] * x2.y) - du[r] * x1.y) * rd[r];
+                    x2 = x1;
+                } else {
+                    y.x = (b[r].x - du[r] * x1.x) * rd[r];
+                    y.y = (b[r].y - du[r] * x1.y) * rd[r];
+                }
+                sp[(long)q * NM] = y;
+                x1 = y;
+            }
+        }
+    }
 }
 
-static size_t tri_mode_smem(int nym) { return (size_t)nym * (6 * sizeof(double) + 1); }
+__global__ void __launch_bounds__(32) k_tri_mode(double2 *__restrict__ spec, TriFac f,
+                                                 const unsigned char *__restrict__ flag,
+                                                 const double *__restrict__ duc, int nym, long NM) {
+    const long mo = (long)blockIdx.x * 32 + threadIdx.x;
+    const bool act = mo < NM;
+    const bool piv = __any_sync(0xffffffffu, act && flag[act ? mo : 0]);
+    if (!act) return;
+    if (piv) tri_replay<true>(spec, f, duc, nym, NM, mo);
+    else tri_replay<false>(spec, f, duc, nym, NM, mo);
+}
 
 // The tridiagonal systems of many channels in one launch (ensembles): the
 // FP64 replay of k_tri_mode (zgtsv's elimination with its recorded pivots)
@@ -1793,7 +1858,7 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
         else k_tri_split<32><<<nb, tb, sm, ctx->st>>>((float2 *)spec, tf, ts, nym, NM, npb, pw);
         count_launch(ctx, "k_tri_split");
     } else {
-        k_tri_mode<T><<<(unsigned)NM, 32, tri_mode_smem(nym), ctx->st>>>(spec, tf, nym, NM, nullptr);
+        k_tri_mode<<<(unsigned)cdiv(NM, 32), 32, 0, ctx->st>>>(spec, tf, ctx->tri_flag, ctx->d_tri + 2 * nym, nym, NM);
         count_launch(ctx, "k_tri_mode");
     }
     }
