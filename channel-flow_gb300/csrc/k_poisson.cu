@@ -1010,8 +1010,8 @@ __device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const Tri
             if (q >= 0) {
                 double2 y;
                 if constexpr (PIV) {
-                    y.x = ((b[r].x - dl[r] * x2.x) - du[r] * x1.x) * rd[r];
-                    y.y = ((b[r].y - dl[r] * x2.y) - du[r] * x1.y) * rd[r];
+                    y.x = ((b[r].x - du[r] * x1.x) - dl[r] * x2.x) * rd[r];
+                    y.y = ((b[r].y - du[r] * x1.y) - dl[r] * x2.y) * rd[r];
                     x2 = x1;
                 } else {
                     y.x = (b[r].x - du[r] * x1.x) * rd[r];
