@@ -211,9 +211,12 @@ __device__ __forceinline__ const C *stage_twiddles(const C *tw, C *sm_tw) {
 // threads per line of the x transforms (the host launch uses the same rule)
 __host__ __device__ constexpr int fft_x_threads(int n) { return n >= 128 ? 32 : 16; }
 
-// reciprocal face spacings 1/(x(i)-x(i-1)) etc., 1-based (split path)
+// reciprocal face spacings 1/(x(i)-x(i-1)) etc., 1-based.  Both precisions
+// multiply by them: an FP64 division is about a dozen FP64 instructions, and
+// the FP64 pipe (two lanes an SM) is what the FP64 kernels are bound by.
+template <typename T>
 struct RSp {
-    const float *rx, *ry, *rz;
+    const T *rx, *ry, *rz;
 };
 
 // ---------------------------------------------------------------------------
@@ -224,7 +227,7 @@ struct RSp {
 // ---------------------------------------------------------------------------
 template <typename T, int N>
 __global__ void k_fwd_x(GeoT<T> g, Fld<T> U, Fld<T> V, Fld<T> W, typename C2<T>::t *spec, FftPlan pl,
-                        const typename C2<T>::t *tw_g, int LP, RSp rs) {
+                        const typename C2<T>::t *tw_g, int LP, RSp<T> rs) {
     typedef typename C2<T>::t C;
     extern __shared__ unsigned char smraw[];
     C *sm = (C *)smraw;
@@ -246,17 +249,16 @@ __global__ void k_fwd_x(GeoT<T> g, Fld<T> U, Fld<T> V, Fld<T> W, typename C2<T>:
     // need not be filled before this kernel
     const int km = k == 2 ? nzp + 1 : k - 1;
     if (active) {
-        if constexpr (sizeof(T) == 4 && N > 0) {
-            // split path, compile-time length: reciprocal spacings instead of
-            // divisions; the loads of XB points are issued before any of them
+        if constexpr (N > 0) {
+            // compile-time length: the loads of XB points are issued before any of them
             // is used or stored (a shared-memory store would otherwise order
             // every later load of U, V, W behind it)
             constexpr int GX = fft_x_threads(N), NPT = N / GX, XB = NPT < 3 ? NPT : 3;
-            const float ry = rs.ry[j], rz0 = rs.rz[k], rz1 = rs.rz[k + 1];
+            const T ry = rs.ry[j], rz0 = rs.rz[k], rz1 = rs.rz[k + 1];
             const int k1 = k + 1;
 #pragma unroll
             for (int e0 = 0; e0 < NPT; e0 += XB) {
-                float ua[XB], uam[XB], ub[XB], ubm[XB], va[XB], vam[XB], vb[XB], vbm[XB], wa[XB], wb[XB], wm[XB], rx[XB];
+                T ua[XB], uam[XB], ub[XB], ubm[XB], va[XB], vam[XB], vb[XB], vbm[XB], wa[XB], wb[XB], wm[XB], rx[XB];
 #pragma unroll
                 for (int b = 0; b < XB; b++) {
                     const int i = tid + 2 + (e0 + b) * GX, im = i == 2 ? n + 1 : i - 1;
@@ -278,32 +280,16 @@ __global__ void k_fwd_x(GeoT<T> g, Fld<T> U, Fld<T> V, Fld<T> W, typename C2<T>:
                     }
                 }
             }
-        } else if constexpr (sizeof(T) == 4) {
-            // split path, run-time length
-            const float ry = rs.ry[j], rz0 = rs.rz[k], rz1 = rs.rz[k + 1];
+        } else {
+            const T ry = rs.ry[j], rz0 = rs.rz[k], rz1 = rs.rz[k + 1];
             for (int i = tid + 2; i <= n + 1; i += G) {
-                const float rx = rs.rx[i];
+                const T rx = rs.rx[i];
                 const int k1 = k + 1, im = i == 2 ? n + 1 : i - 1;
-                const float w0 = W(i, j, k), w1 = W(i, j, k1);
+                const T w0 = W(i, j, k), w1 = W(i, j, k1);
                 T d0 = (U(i, j, k) - U(im, j, k)) * rx + (V(i, j, k) - V(i, j - 1, k)) * ry +
                        (w0 - W(i, j, km)) * rz0;
                 T d1 = (U(i, j, k1) - U(im, j, k1)) * rx + (V(i, j, k1) - V(i, j - 1, k1)) * ry +
                        (w1 - w0) * rz1;
-                C z;
-                z.x = d0;
-                z.y = d1;
-                a[i - 2] = z;
-            }
-        } else {
-            for (int i = tid + 2; i <= n + 1; i += G) {
-                const int im = i == 2 ? n + 1 : i - 1;
-                T d0 = (U(i, j, k) - U(im, j, k)) / (g.x[i] - g.x[i - 1]) +
-                       (V(i, j, k) - V(i, j - 1, k)) / (g.y[j] - g.y[j - 1]) +
-                       (W(i, j, k) - W(i, j, km)) / (g.z[k] - g.z[k - 1]);
-                int k1 = k + 1;
-                T d1 = (U(i, j, k1) - U(im, j, k1)) / (g.x[i] - g.x[i - 1]) +
-                       (V(i, j, k1) - V(i, j - 1, k1)) / (g.y[j] - g.y[j - 1]) +
-                       (W(i, j, k1) - W(i, j, k1 - 1)) / (g.z[k1] - g.z[k1 - 1]);
                 C z;
                 z.x = d0;
                 z.y = d1;
@@ -668,7 +654,7 @@ constexpr int XR_FT = 32;  // threads per line pair of the forward x transform
 
 template <typename T, int N>
 __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, Fld<T> W, typename C2<T>::t *spec,
-                                                 const typename C2<T>::t *__restrict__ tw_g, RSp rs) {
+                                                 const typename C2<T>::t *__restrict__ tw_g, RSp<T> rs) {
     typedef typename C2<T>::t C;
     constexpr int R0 = xr_r(N, 0), R1 = xr_r(N, 1), R2 = xr_r(N, 2), G = XR_FT, LP = ZR_T / G, NB0 = N / R0;
     constexpr int RL = R2 > 1 ? R2 : R1, NSL = N / RL, NBL = N / RL;  // the last stage (span NSL)
@@ -691,12 +677,7 @@ __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, 
     // (U(1) = U(nxp+1), W(k=1) = W(nzp+1))
     const int km = k == 2 ? nzp + 1 : k - 1, k1 = k + 1;
     if (act) {
-        T ry = T(0), rz0 = T(0), rz1 = T(0);
-        if constexpr (sizeof(T) == 4) {
-            ry = rs.ry[j];
-            rz0 = rs.rz[k];
-            rz1 = rs.rz[k + 1];
-        }
+        const T ry = rs.ry[j], rz0 = rs.rz[k], rz1 = rs.rz[k + 1];
 #pragma unroll
         for (int e0 = 0; e0 < NPT; e0 += XB) {
             T ua[XB], uam[XB], ub[XB], ubm[XB], va[XB], vam[XB], vb[XB], vbm[XB], wa[XB], wb[XB], wm[XB];
@@ -714,16 +695,9 @@ __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, 
                 const int x = t + (e0 + b) * G, i = x + 2;
                 if (e0 + b < NPT && x < N) {
                     C z;
-                    if constexpr (sizeof(T) == 4) {
-                        const T rx = rs.rx[i];
-                        z.x = (ua[b] - uam[b]) * rx + (va[b] - vam[b]) * ry + (wa[b] - wm[b]) * rz0;
-                        z.y = (ub[b] - ubm[b]) * rx + (vb[b] - vbm[b]) * ry + (wb[b] - wa[b]) * rz1;
-                    } else {
-                        z.x = (ua[b] - uam[b]) / (g.x[i] - g.x[i - 1]) + (va[b] - vam[b]) / (g.y[j] - g.y[j - 1]) +
-                              (wa[b] - wm[b]) / (g.z[k] - g.z[k - 1]);
-                        z.y = (ub[b] - ubm[b]) / (g.x[i] - g.x[i - 1]) + (vb[b] - vbm[b]) / (g.y[j] - g.y[j - 1]) +
-                              (wb[b] - wa[b]) / (g.z[k1] - g.z[k1 - 1]);
-                    }
+                    const T rx = rs.rx[i];
+                    z.x = (ua[b] - uam[b]) * rx + (va[b] - vam[b]) * ry + (wa[b] - wm[b]) * rz0;
+                    z.y = (ub[b] - ubm[b]) * rx + (vb[b] - vbm[b]) * ry + (wb[b] - wa[b]) * rz1;
                     bl[xr_pos<N>(x)] = z;
                 }
             }
@@ -1549,11 +1523,6 @@ struct PhiView {
     }
 };
 
-// reciprocal spacings of the split path's projection
-struct RSpG {
-    const float *rxg, *ryg, *rzg;  // 1/(xg(i)-xg(i-1)) etc., 1-based
-};
-
 // planes per thread of the pressure store: every load of the thread is
 // issued before the first store
 constexpr int PROJ_KP = 2;
@@ -1565,8 +1534,7 @@ template <typename T>
 struct ProjArgs {
     T *u, *v, *w, *ul, *vl, *wl;
     const T *phi;
-    const float *rxg, *ryg, *rzg;
-    const T *xg, *yg, *zg;
+    const T *rxg, *ryg, *rzg;
     int nx, ny, nz, nxg, nyg, nzg, nxp, nym, nzp, ilim, klim;
 };
 
@@ -1662,14 +1630,7 @@ __global__ void __launch_bounds__(128) k_project3(const __grid_constant__ ProjAr
             wl[q] = dw && kin ? a.wl[iw + q * swz] : T(0);
         }
     }
-    T rx, ry;
-    if constexpr (sizeof(T) == 4) {
-        rx = du ? a.rxg[i + 1] : T(0);
-        ry = dv ? a.ryg[j + 1] : T(0);
-    } else {
-        rx = du ? T(1) / (a.xg[i + 1] - a.xg[i]) : T(0);
-        ry = dv ? T(1) / (a.yg[j + 1] - a.yg[j]) : T(0);
-    }
+    const T rx = du ? a.rxg[i + 1] : T(0), ry = dv ? a.ryg[j + 1] : T(0);
     auto upd = [&](T *F, T *Fl, int o, T f, T fl, T gr) {
         if constexpr (sizeof(T) == 4 && LO) {
             float hi = f, l = fl;
@@ -1684,19 +1645,8 @@ __global__ void __launch_bounds__(128) k_project3(const __grid_constant__ ProjAr
     for (int q = 0; q < KP; q++) {
         const int k = k0 + q;
         if (k > klim) break;
-        T gx, gy, gz;
-        if constexpr (sizeof(T) == 4) {
-            gx = (px[q] - p0[q]) * rx;
-            gy = (py[q] - p0[q]) * ry;
-            gz = k <= nz - 1 ? (p0[q + 1] - p0[q]) * a.rzg[k + 1] : T(0);
-        } else {
-            // projection.f90:209-223 divides by the spacings
-            gx = du ? (px[q] - p0[q]) / (a.xg[i + 1] - a.xg[i]) : T(0);
-            gy = dv ? (py[q] - p0[q]) / (a.yg[j + 1] - a.yg[j]) : T(0);
-            gz = k <= nz - 1 ? (p0[q + 1] - p0[q]) / (a.zg[k + 1] - a.zg[k]) : T(0);
-        }
-        (void)rx;
-        (void)ry;
+        const T gx = (px[q] - p0[q]) * rx, gy = (py[q] - p0[q]) * ry,
+                gz = k <= nz - 1 ? (p0[q + 1] - p0[q]) * a.rzg[k + 1] : T(0);
         if (du) upd(a.u, a.ul, iu + q * suz, u[q], ul[q], gx);
         if (dv) upd(a.v, a.vl, iv + q * svz, v[q], vl[q], gy);
         if (k <= nz - 1) upd(a.w, a.wl, iw + q * swz, w[q], wl[q], gz);
@@ -1745,10 +1695,10 @@ __global__ void __launch_bounds__(128) k_store_p(Fld<T> P, const T *__restrict__
         const int kc = min(max(k0 + q, 2), nzg - 1);
         v[q] = k0 + q <= nzg ? phi[pv(ic, jc, kc)] : T(0);
     }
-    const T den = ds_dt<T>(ds) * c11;
+    const T rden = T(1) / (ds_dt<T>(ds) * c11);
 #pragma unroll
     for (int q = 0; q < KP; q++)
-        if (k0 + q <= nzg) P(i, j, k0 + q) = v[q] / den;
+        if (k0 + q <= nzg) P(i, j, k0 + q) = v[q] * rden;
 }
 
 template <typename T>
@@ -1788,10 +1738,8 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
     int LB = 16;  // with Gz = 16: FFTZ_KZS elements apart per thread in the copies
     while (LB > 1 && smem_pairs<T>(nzp, LB) + (LB + nzp) * sizeof(C) > 96 * 1024) LB /= 2;
     const size_t shz = smem_pairs<T>(nzp, LB) + (LB + nzp) * sizeof(C);
-    RSp rs;
-    rs.rx = ctx->d_rgeo_f + ctx->rgeo_off[0];
-    rs.ry = ctx->d_rgeo_f + ctx->rgeo_off[2];
-    rs.rz = ctx->d_rgeo_f + ctx->rgeo_off[4];
+    const RcpT<T> rc = rcp_of<T>(ctx);
+    const RSp<T> rs = {rc.dx, rc.dy, rc.dz};
 #define CF_FFT_SIZES(X) X(16) X(32) X(64) X(96) X(128) X(192) X(256) X(384) X(512)
 #define CF_FWDX(N) case N: \
     if constexpr (xr_r(N, 0) > 0) k_fwd_xr<T, N><<<cdiv(npairs, ZR_T / XR_FT), ZR_T, xr_fwd_smem<T, N>(), ctx->st>>>(g, U, V, W, spec, twxf, rs); \
@@ -1832,7 +1780,7 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
     tf.du = ctx->tri_fac + 2 * nf;
     tf.dl = ctx->tri_fac + 3 * nf;
     tf.piv = ctx->tri_piv;
-    if (sizeof(T) == 4) {
+    if constexpr (sizeof(T) == 4) {
         TriSplit ts;
         ts.l = ctx->tri_l32;
         ts.ru = ctx->tri_ru32;
@@ -1901,10 +1849,7 @@ int launch_projection(cf_ctx *ctx, int b, bool store_p, bool lo, bool canon, int
     pv.nxp = nxp; pv.nym = nym; pv.nzp = nzp;
     dim3 blk(32, 4, 1);
     {
-        RSpG rg;
-        rg.rxg = ctx->d_rgeo_f + ctx->rgeo_off[1];
-        rg.ryg = ctx->d_rgeo_f + ctx->rgeo_off[3];
-        rg.rzg = ctx->d_rgeo_f + ctx->rgeo_off[5];
+        const RcpT<T> rc = rcp_of<T>(ctx);
         const int ilim = canon ? ctx->nxp + 1 : ctx->nxg - 1, klim = canon ? ctx->nzp + 1 : ctx->nzg - 1;
         // the boundary conditions as ghost copies written by the projection
         // itself: canonical cells, no-slip walls
@@ -1915,8 +1860,7 @@ int launch_projection(cf_ctx *ctx, int b, bool store_p, bool lo, bool canon, int
         pa.vl = lo ? (T *)ctx->Vlo[b] : nullptr;
         pa.wl = lo ? (T *)ctx->Wlo[b] : nullptr;
         pa.phi = phi;
-        pa.rxg = rg.rxg; pa.ryg = rg.ryg; pa.rzg = rg.rzg;
-        pa.xg = g.xg; pa.yg = g.yg; pa.zg = g.zg;
+        pa.rxg = rc.dxg; pa.ryg = rc.dyg; pa.rzg = rc.dzg;
         pa.nx = ctx->nx; pa.ny = ctx->ny; pa.nz = ctx->nz;
         pa.nxg = ctx->nxg; pa.nyg = ctx->nyg; pa.nzg = ctx->nzg;
         pa.nxp = nxp; pa.nym = nym; pa.nzp = nzp;
