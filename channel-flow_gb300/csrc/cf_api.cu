@@ -10,8 +10,8 @@
 int fft_setup_attrs();
 int dsm_fused_setup();
 int dsm_b_setup();
-int dsm_b_plan(int esz, int nxp, int nym, int nzp, int sms);
-int dsm_fused_plan(int esz, int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
+int dsm_b_plan(int nxp, int nym, int nzp, int sms);
+int dsm_fused_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
 
 static thread_local std::string g_last_error;  // failures without a context
 
@@ -496,7 +496,13 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
         dsm_fused_setup();
         dsm_b_setup();
-        dsm_fused_plan(p->precision == CF_PREC_SPLIT ? 4 : 8, nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_fused);
+        if (ctx->esz == 4) {
+            dsm_fused_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_fused);
+            ctx->dsmb_nkc = dsm_b_plan(nxp, ctx->nym, nzp, dev_sms);
+        } else {
+            dsm64_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_fused);
+            nch_fused = (size_t)dsm64_slots(nxp, nzp, 1);  // any chunk length
+        }
         ctx->use_fused_dsm = !p->dsm_unfused;
         // fused RHS: 32 x 8 column tiles, z chunks for ~4 resident blocks per SM
         long rt = (long)cdiv(ctx->nxp, 32) * cdiv(ctx->nyg - 2, 8);
@@ -512,10 +518,9 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
         }
         ctx->rhs_nkc = (int)best;
         if (p->LES_model == 3) amd_plan(p->precision == CF_PREC_SPLIT ? 4 : 8, nxp, ctx->nym, nzp, dev_sms, &ctx->amd_nkc, &amd_parts);
-        ctx->dsmb_nkc = dsm_b_plan(p->precision == CF_PREC_SPLIT ? 4 : 8, nxp, ctx->nym, nzp, dev_sms);
     }
     // (with the wall model the one-pass kernel's slots are followed by the seam band's)
-    size_t nch = std::max({(size_t)ctx->dsm_nblk, nch_fused + (p->iwall_model == 3 ? dsm_seam_slots_max() : 0),
+    size_t nch = std::max({(size_t)ctx->dsm_nblk, nch_fused + (ctx->esz == 4 && p->iwall_model == 3 ? dsm_seam_slots_max() : 0),
                            (size_t)cdiv(amd_parts, 2), (size_t)cdiv(nxp, 32) * (size_t)ctx->dsmb_nkc});
     CF_CUDA(cudaMalloc(&ctx->dsm_part, (size_t)2 * ctx->nym * nch * sizeof(double)));
     ctx->dsm_part_nch = nch;
@@ -1156,7 +1161,7 @@ static int step_eager(cf_ctx *ctx) { return DISPATCH(enqueue_step<double>(ctx), 
 // Each member's launches are those of enqueue_seg in the same order.
 // ---------------------------------------------------------------------------
 static bool dsm_batchable(const cf_ctx *c) {
-    return c->prm.LES_model == 2 && c->use_fused_dsm && c->prm.iwall_model == 0 && c->state_periodic && c->use_rhs3;
+    return c->esz == 4 && c->prm.LES_model == 2 && c->use_fused_dsm && c->prm.iwall_model == 0 && c->state_periodic && c->use_rhs3;
 }
 
 static void ens_bufs(const cf_ctx *c, int s, int *src, int *dst) {
@@ -1639,8 +1644,7 @@ static int capture_batched_step(cf_ensemble *e, int *extra) {
                 std::vector<cf_ctx *> &mm = pass ? dm2 : dm;
                 std::vector<int> &bb = pass ? db2 : db;
                 if (mm.empty()) continue;
-                rc = esz == 8 ? launch_dsm_batch<double>(e->st, mm.data(), bb.data(), (int)mm.size())
-                              : launch_dsm_batch<float>(e->st, mm.data(), bb.data(), (int)mm.size());
+                rc = launch_dsm_batch<float>(e->st, mm.data(), bb.data(), (int)mm.size());
                 *extra += 2;
             }
             if (!rc && !rm.empty()) {
@@ -1894,13 +1898,13 @@ static int tune_t(cf_ctx *ctx, int reps, double *rep) {
     if (!rc && ctx->prm.LES_model == 2 && ctx->use_fused_dsm && ctx->state_periodic &&
         (ctx->prm.iwall_model == 0 || ctx->prm.iwall_model == 3)) {
         const int keep = ctx->dsm_kc;
-        const int ntx = cdiv(ctx->nxp, sizeof(T) == 4 ? 32 : 16);
-        const size_t nseam = ctx->prm.iwall_model == 3 ? (size_t)dsm_seam_slots_max() : 0;
+        const size_t nseam = sizeof(T) == 4 && ctx->prm.iwall_model == 3 ? (size_t)dsm_seam_slots_max() : 0;
         double best = 1e300;
         int best_kc = keep, last_len = -1;
         for (int nn = cdiv(nzp, DSM_ZMAX_HOST); nn <= std::max(1, nzp / 4) && !rc; nn++) {
             const int len = cdiv(nzp, nn);
-            if (len == last_len || (size_t)ntx * cdiv(nzp, len) + nseam > ctx->dsm_part_nch) continue;
+            const size_t slots = sizeof(T) == 4 ? (size_t)cdiv(ctx->nxp, 32) * cdiv(nzp, len) : (size_t)dsm64_slots(ctx->nxp, nzp, len);
+            if (len == last_len || slots + nseam > ctx->dsm_part_nch) continue;
             last_len = len;
             ctx->dsm_kc = len;
             double us = 0;

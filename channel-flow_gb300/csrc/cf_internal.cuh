@@ -214,7 +214,7 @@ struct cf_ctx {
     double *dsm_part = nullptr;        // plane partial sums
     double *avg_nu_t = nullptr;        // (nyg) device
     int dsm_nblk = 0;
-    int dsm_kc = 0;                    // z-chunk length of the fused pass
+    int dsm_kc = 0;                    // z-chunk length of the fused pass (FP32) or of the FP64 pass
     int dsm_nchunk_fused = 0;          // plane-partial slots per row of the last one-pass launch
     int dsm_nchunk_base = 0;           // of them, the one-pass kernel's (the seam band's follow)
     bool use_fused_dsm = true;
@@ -305,8 +305,11 @@ int rhs3_blocks_per_sm(int esz);
 template <typename T> int launch_rhs_update(cf_ctx *ctx, int s, int src, int dst);  // fused RHS + RK update
 template <typename T> int launch_rk_update(cf_ctx *ctx, int s);            // from stored F slots
 template <typename T> int launch_dsm(cf_ctx *ctx, int buf);                // eddy viscosity
-template <typename T> int launch_dsm_fused(cf_ctx *ctx, int buf);          // fused pass (periodic state)
-template <typename T> int launch_dsm_fused_wm(cf_ctx *ctx, int buf);       // fused pass + seam band (wall model)
+template <typename T> int launch_dsm_fused(cf_ctx *ctx, int buf);          // FP32 fused pass (periodic state)
+template <typename T> int launch_dsm_fused_wm(cf_ctx *ctx, int buf);       // FP32 fused pass + seam band (wall model)
+int launch_dsm64(cf_ctx *ctx, int buf, int *nchunk);                       // FP64 pass: |S| and the plane partials
+void dsm64_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
+int dsm64_slots(int nxp, int nzp, int kc);                                 // its partials per row with chunks of kc planes
 int dsm_seam_slots_max();                                                  // partial slots the seam band may take
 constexpr int CF_ENS_MAXM = 32;  // channels per batched ensemble launch at most
 // fused pass + <LM>/<MM> rows of n channels in two launches (ensembles)

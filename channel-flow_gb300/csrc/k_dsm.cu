@@ -1,4 +1,7 @@
-// k_dsm.cu -- dynamic Smagorinsky eddy viscosity, subgrid.f90:376-538.
+// k_dsm.cu -- dynamic Smagorinsky eddy viscosity, subgrid.f90:376-538: the
+// multi-pass kernels of the FP32 path (a state whose ghosts are not yet
+// filled), the plane coefficients and nu_t from them; the other passes are
+// in k_dsm_fused.cu (FP32) and k_dsm64.cu (FP64).
 //
 // Quantities the reference keeps only as periodic copies are computed at the
 // canonical cells (i = 2..nx-1, j = 2..nyg-1, k = 2..nz-1) and read through
@@ -61,18 +64,16 @@ __global__ void k_dsm_a(GeoT<T> g, RcpT<T> rc, Fld<T> U, Fld<T> V, Fld<T> W, T *
 // (subgrid.f90:429-513).  A block owns a DB_X x DB_Y tile of (i, j) and
 // marches along z over a chunk of planes: each plane of the 15 quantities
 // (tile plus one halo cell, periodic in x, rows clamped to the interior) is
-// gathered into a shared-memory buffer while an earlier one is filtered; the
-// FP32 kernel filters it in y by a column pass and in x at its point (the
-// FP64 kernel with a 9-point stencil at its point) and spreads the result
+// gathered into a shared-memory buffer while an earlier one is filtered, then
+// filtered in y by a column pass and in x at the point, and the result spread
 // over the z accumulators of planes r-1, r, r+1 (weights 1/6, 2/3, 1/6), so
 // that plane r-1 is complete once plane r is in.  The filtered velocities
 // Uf, Vf, Wf (stage C) are read at their actual indices, while the next
-// plane's copies are in flight.  The plane sums (float-float in the FP32
-// kernel) count the duplicate column and plane as weight 2 on i = 2 and
+// plane's copies are in flight.  The plane sums (float-float) count the duplicate column and plane as weight 2 on i = 2 and
 // k = 2 (the reference's loops run over i = 2..nxg-1, k = 2..nzg-1).
 //
-// Two gathers: per-element cp.async copies into two buffers (any nxp, FP64
-// and FP32), and for FP32 with nxp a multiple of 4 one tensor copy (TMA) per
+// Two gathers: per-element cp.async copies into two buffers (any nxp), and
+// with nxp a multiple of 4 one tensor copy (TMA) per
 // plane into three buffers, two planes in flight.  The tensor copy is a 4D
 // box of x 40, y 10, z 1 and all 15 quantities; its x origin is 4 columns
 // before the tile's halo column (16-byte aligned), its y origin the row
@@ -126,22 +127,23 @@ __device__ __forceinline__ bool dbt_wait(uint32_t mb, uint32_t parity) {
     return false;
 }
 // dynamic shared memory of k_dsm_b: the plane buffers of the 15 quantities
-template <typename T, bool TMA>
+template <bool TMA>
 constexpr size_t dsm_b_smem() {
-    return TMA ? (size_t)DBT_NB * DBT_STRIDE + 128 : (size_t)2 * DB_NQ * (DB_X + 2) * (DB_Y + 2) * sizeof(T);
+    return TMA ? (size_t)DBT_NB * DBT_STRIDE + 128 : (size_t)2 * DB_NQ * (DB_X + 2) * (DB_Y + 2) * sizeof(float);
 }
 
-// TMA: the tensor-copy gather (FP32, nxp a multiple of 4; tm maps the 15
+// TMA: the tensor-copy gather (nxp a multiple of 4; tm maps the 15
 // quantities of q as x nxp, y nym, z nzp, quantity 15).  skip_first (a test
 // hook): plane kb-1 is not copied, so its wait expires and the block stops.
 // A wait that expired is counted in ds->n_wait; the block's copies still in
 // flight are waited for (with the same limit) before it returns.
-template <typename T, bool TMA>
-__global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CUtensorMap tm, const T *__restrict__ q,
-                                                      GeoT<T> g, RcpT<T> rc, Fld<T> Uf, Fld<T> Vf, Fld<T> Wf, Can c,
+template <bool TMA>
+__global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CUtensorMap tm, const float *__restrict__ q,
+                                                      GeoT<float> g, RcpT<float> rc, Fld<float> Uf, Fld<float> Vf,
+                                                      Fld<float> Wf, Can c,
                                                       int nyg, int kc_len, double *part, int nchunk, DevScal *ds,
                                                       int skip_first) {
-    static_assert(!TMA || sizeof(T) == 4, "the tensor-copy gather is the FP32 kernel's");
+    typedef float T;
     constexpr int SX = DB_X + 2, SY = DB_Y + 2, NP = SX * SY;
     // a buffer: DB_NQ quantities of PQ elements, rows of pitch PX, halo
     // column 0 at column OX
@@ -151,11 +153,8 @@ __global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CU
     // tensor-copy destinations are 128-byte aligned
     T *plb = (T *)(dsmb_raw + (TMA ? (128 - (sh_u32(dsmb_raw) & 127)) & 127 : 0));  // [NB][DB_NQ][PQ]
     __shared__ __align__(8) uint64_t bar[NB];
-    // the plane filtered in y, rows of the tile (FP32: within 48 KB of static
-    // shared memory with the plane; the FP64 kernel filters from the plane)
-    constexpr bool COLS = sizeof(T) == 4;
-    __shared__ T cl[COLS ? DB_NQ : 1][DB_Y][SX];
-    __shared__ double red[2][DB_X * DB_Y];
+    // the plane filtered in y, rows of the tile
+    __shared__ T cl[DB_NQ][DB_Y][SX];
     const int tx = threadIdx.x % DB_X, ty = threadIdx.x / DB_X;
     const int i0 = 2 + blockIdx.x * DB_X, j0 = 2 + blockIdx.y * DB_Y;
     const int kb = 2 + blockIdx.z * kc_len, ke = min(kb + kc_len - 1, c.nzp + 1);
@@ -167,9 +166,8 @@ __global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CU
     T accp[DB_NQ], accc[DB_NQ];  // planes r-1 (two contributions in) and r (one)
 #pragma unroll
     for (int qq = 0; qq < DB_NQ; qq++) accp[qq] = accc[qq] = T(0);
-    // plane sums of this thread: FP64 in the FP64 path, float-float in the
-    // split path (an FP64 instruction per cell costs dozens of FP32 ones here)
-    double sl = 0.0, smm = 0.0;
+    // plane sums of this thread in float-float (an FP64 instruction per cell
+    // costs dozens of FP32 ones here)
     float slh = 0.f, sll = 0.f, smh = 0.f, sml = 0.f;
     // gather of plane r into buffer b: one tensor copy issued by thread 0
     // (TMA), or one group of per-element asynchronous copies (tile plus one
@@ -278,7 +276,6 @@ __global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CU
         }
         // y filter, one (quantity, column) per task: the column's SY values
         // give the DB_Y filtered rows (one-sided at rows 2 and nyg-1)
-        if constexpr (COLS) {
         for (int t = threadIdx.x; t < DB_NQ * SX; t += DB_X * DB_Y) {
             const int qq = t / SX, sx = t - qq * SX;
             T col[SY];
@@ -292,20 +289,13 @@ __global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CU
             }
         }
         __syncthreads();
-        }
         if (!own) continue;
-        // y weights of this row for the FP64 kernel (one-sided at rows 2 and nyg-1)
-        const T wm = j == 2 ? T(0) : (j == nyg - 1 ? f13 : f6), wp = j == 2 ? f13 : (j == nyg - 1 ? T(0) : f6);
-        const int e = (ty + 1) * PX + tx + 1 + OX;
         T fq[DB_NQ];
 #pragma unroll
         for (int qq = 0; qq < DB_NQ; qq++) {
             T a = T(0);
 #pragma unroll
-            for (int d = -1; d <= 1; d++) {
-                if constexpr (COLS) a += fw[d + 1] * cl[qq][ty][tx + 1 + d];
-                else a += fw[d + 1] * (wm * pl[qq][e + d - PX] + f23 * pl[qq][e + d] + wp * pl[qq][e + d + PX]);
-            }
+            for (int d = -1; d <= 1; d++) a += fw[d + 1] * cl[qq][ty][tx + 1 + d];
             fq[qq] = accp[qq] + f6 * a;  // plane r-1, complete
             accp[qq] = accc[qq] + f23 * a;
             accc[qq] = f6 * a;
@@ -321,15 +311,9 @@ __global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CU
         }
         const T lm = (L[0] * M[0] + L[1] * M[1] + L[2] * M[2] + T(2) * (L[3] * M[3] + L[4] * M[4] + L[5] * M[5]));
         const T mm = (M[0] * M[0] + M[1] * M[1] + M[2] * M[2] + T(2) * (M[3] * M[3] + M[4] * M[4] + M[5] * M[5]));
-        if constexpr (sizeof(T) == 4) {
-            const float wgt = (i == 2 ? 2.f : 1.f) * (k == 2 ? 2.f : 1.f);  // exact: lm, mm times 1, 2 or 4
-            ff_add(slh, sll, wgt * lm);
-            ff_add(smh, sml, wgt * mm);
-        } else {
-            const double wgt = (i == 2 ? 2.0 : 1.0) * (k == 2 ? 2.0 : 1.0);
-            sl += wgt * (double)lm;
-            smm += wgt * (double)mm;
-        }
+        const float wgt = (i == 2 ? 2.f : 1.f) * (k == 2 ? 2.f : 1.f);  // exact: lm, mm times 1, 2 or 4
+        ff_add(slh, sll, wgt * lm);
+        ff_add(smh, sml, wgt * mm);
     }
     if constexpr (TMA) {
         if (rfail) {
@@ -345,36 +329,19 @@ __global__ void __launch_bounds__(DB_X *DB_Y) k_dsm_b(const __grid_constant__ CU
             return;
         }
     }
-    if constexpr (sizeof(T) == 4) {
-        // one warp per row (DB_X = 32): float-float shuffle tree, lane 0
-        // writes (L.M hi, lo, M.M hi, lo)
-        if (!own) slh = sll = smh = sml = 0.f;
+    // one warp per row (DB_X = 32): float-float shuffle tree, lane 0
+    // writes (L.M hi, lo, M.M hi, lo)
+    if (!own) slh = sll = smh = sml = 0.f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float a1 = __shfl_down_sync(0xffffffffu, slh, o), a2 = __shfl_down_sync(0xffffffffu, sll, o);
-            const float b1 = __shfl_down_sync(0xffffffffu, smh, o), b2 = __shfl_down_sync(0xffffffffu, sml, o);
-            ff_add2(slh, sll, a1, a2);
-            ff_add2(smh, sml, b1, b2);
-        }
-        if (tx == 0 && j <= nyg - 1) {
-            const long chunk = (long)blockIdx.z * gridDim.x + blockIdx.x;
-            ((float4 *)part)[(long)(j - 2) * nchunk + chunk] = make_float4(slh, sll, smh, sml);
-        }
-        return;
+    for (int o = 16; o > 0; o >>= 1) {
+        const float a1 = __shfl_down_sync(0xffffffffu, slh, o), a2 = __shfl_down_sync(0xffffffffu, sll, o);
+        const float b1 = __shfl_down_sync(0xffffffffu, smh, o), b2 = __shfl_down_sync(0xffffffffu, sml, o);
+        ff_add2(slh, sll, a1, a2);
+        ff_add2(smh, sml, b1, b2);
     }
-    // plane partials of this block for row j: the sum over the tile's DB_X threads of the row
-    red[0][threadIdx.x] = sl;
-    red[1][threadIdx.x] = smm;
-    __syncthreads();
     if (tx == 0 && j <= nyg - 1) {
-        double a = 0.0, b = 0.0;
-        for (int t = 0; t < DB_X; t++) {
-            a += red[0][ty * DB_X + t];
-            b += red[1][ty * DB_X + t];
-        }
         const long chunk = (long)blockIdx.z * gridDim.x + blockIdx.x;
-        part[((long)(j - 2) * nchunk + chunk) * 2] = a;
-        part[((long)(j - 2) * nchunk + chunk) * 2 + 1] = b;
+        ((float4 *)part)[(long)(j - 2) * nchunk + chunk] = make_float4(slh, sll, smh, sml);
     }
 }
 
@@ -642,89 +609,86 @@ bool dsmb_tma(cf_ctx *ctx) {
     return ctx->dsmb_map_state == 1 && ctx->prm.dsm_unfused != 2;
 }
 
-template <typename T>
-int launch_dsm(cf_ctx *ctx, int b) {
-    int dir = ctx->prm.Dirichlet_nu_t == 1;
-    Can c;
-    c.nxp = ctx->nxp; c.nym = ctx->nym; c.nzp = ctx->nzp; c.n = (long)ctx->nCan;
-    dim3 blk(32, 4, 1);
-    if (ctx->use_fused_dsm && ctx->state_periodic && (ctx->prm.iwall_model == 0 || ctx->prm.iwall_model == 3)) {
-        // one pass: |S| and the plane partial sums (k_dsm_fused.cu); with the
-        // wall model the seam band is computed by k_dsm_seam
-        int rc = ctx->prm.iwall_model == 0 ? launch_dsm_fused<T>(ctx, b) : launch_dsm_fused_wm<T>(ctx, b);
-        if (rc) return rc;
-        const int nch = ctx->dsm_nchunk_fused, nb = ctx->dsm_nchunk_base;
-        if (sizeof(T) == 4)  // float-float partials of the FP32 kernel
-            k_dsm_e_ff<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>((const float4 *)ctx->dsm_part, nch, ctx->nyg,
-                                                                ctx->avg_nu_t, dir, nb);
-        else
-            k_dsm_e<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>(ctx->dsm_part, nch, ctx->nyg, ctx->avg_nu_t, dir, nb);
-        count_launch(ctx, "k_dsm_e");
-        ctx->nut_lazy = true;  // nu_t = max(-C(j)|S|/2, 0) is formed by its readers
-        CF_CUDA(cudaGetLastError());
-        return 0;
-    }
-    ctx->nut_lazy = false;
-    GeoT<T> g = geo_of<T>(ctx);
-    Fld<T> U = make_fld<T>(ctx->U[b], ctx->nx, ctx->nyg);
-    Fld<T> V = make_fld<T>(ctx->V[b], ctx->nxg, ctx->ny);
-    Fld<T> W = make_fld<T>(ctx->W[b], ctx->nxg, ctx->nyg);
-    T *q = (T *)ctx->dsm_q;
-    const RcpT<T> rc = rcp_of<T>(ctx);
-    dim3 grdc(cdiv(ctx->nxp, 32), cdiv(ctx->nym, 4), ctx->nzp);
-    k_dsm_a<T><<<grdc, blk, 0, ctx->st>>>(g, rc, U, V, W, q, c);
-    count_launch(ctx, "k_dsm_a");
-    Fld<T> Uf = make_fld<T>(ctx->Uf, ctx->nx, ctx->nyg);
-    Fld<T> Vf = make_fld<T>(ctx->Vf, ctx->nxg, ctx->ny);
-    Fld<T> Wf = make_fld<T>(ctx->Wf, ctx->nxg, ctx->nyg);
-    {
-        // z chunks of 16 canonical planes
-        const int kc = 16, nkc = cdiv(ctx->nzp, kc), ntx = cdiv(ctx->nxp, 32);
-        k_dsm_c_t<T><<<dim3(ntx, cdiv(ctx->nyg, 8), nkc), 256, 0, ctx->st>>>(U, Uf, ctx->nx, ctx->nyg, ctx->nzg, ctx->nxp, ctx->nzp, kc);
-        k_dsm_c_t<T><<<dim3(ntx, cdiv(ctx->ny, 8), nkc), 256, 0, ctx->st>>>(V, Vf, ctx->nxg, ctx->ny, ctx->nzg, ctx->nxp, ctx->nzp, kc);
-        k_dsm_c_t<T><<<dim3(ntx, cdiv(ctx->nyg, 8), nkc), 256, 0, ctx->st>>>(W, Wf, ctx->nxg, ctx->nyg, ctx->nz, ctx->nxp, ctx->nzp, kc);
-    }
-    count_launch(ctx, "k_dsm_c_t"); count_launch(ctx, "k_dsm_c_t"); count_launch(ctx, "k_dsm_c_t");
-    int nchunk;
-    {
-        // z chunks planned at context creation (dsm_b_plan), within the plane-partial slots
-        const int ntx = cdiv(ctx->nxp, DB_X);
-        long nkc = std::max(1L, std::min((long)std::max(ctx->dsmb_nkc, 1), (long)ctx->dsm_part_nch / ntx));
-        const int kc_len = cdiv(ctx->nzp, nkc);
-        const int nz_chunks = cdiv(ctx->nzp, kc_len);
-        nchunk = ntx * nz_chunks;
-        const dim3 grd(ntx, cdiv(ctx->nym, DB_Y), nz_chunks);
-        CUtensorMap tm;
-        if (dsmb_tma(ctx)) {
-            std::memcpy(&tm, ctx->dsmb_map, sizeof(tm));
-            k_dsm_b<float, true><<<grd, DB_X * DB_Y, dsm_b_smem<float, true>(), ctx->st>>>(
-                tm, (const float *)q, geo_of<float>(ctx), rcp_of<float>(ctx), make_fld<float>(ctx->Uf, ctx->nx, ctx->nyg),
-                make_fld<float>(ctx->Vf, ctx->nxg, ctx->ny), make_fld<float>(ctx->Wf, ctx->nxg, ctx->nyg), c, ctx->nyg,
-                kc_len, ctx->dsm_part, nchunk, ctx->ds, ctx->dsmb_skip_first);
-        } else {
-            std::memset(&tm, 0, sizeof(tm));  // not read by the per-element gather
-            k_dsm_b<T, false><<<grd, DB_X * DB_Y, dsm_b_smem<T, false>(), ctx->st>>>(
-                tm, q, g, rc, Uf, Vf, Wf, c, ctx->nyg, kc_len, ctx->dsm_part, nchunk, ctx->ds, 0);
-        }
-        count_launch(ctx, "k_dsm_b");
-    }
-    if (sizeof(T) == 4)  // float-float partials of the FP32 kernel
-        k_dsm_e_ff<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>((const float4 *)ctx->dsm_part, nchunk, ctx->nyg,
-                                                            ctx->avg_nu_t, dir, nchunk);
+// The plane coefficients <LM>/<MM> from nch partials per row (of them nbase
+// outside the seam band's rows): float-float ones of the FP32 kernels, FP64
+// ones of the FP64 pass.  nu_t = max(-C(j)|S|/2, 0) (stage F) is left to its
+// readers: the fused RHS forms it in its loader, the others (eqwm, statistics,
+// downloads) materialise it first.
+static int launch_dsm_e(cf_ctx *ctx, int nch, int nbase) {
+    const int dir = ctx->prm.Dirichlet_nu_t == 1;
+    if (ctx->esz == 4)
+        k_dsm_e_ff<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>((const float4 *)ctx->dsm_part, nch, ctx->nyg, ctx->avg_nu_t,
+                                                            dir, nbase);
     else
-        k_dsm_e<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>(ctx->dsm_part, nchunk, ctx->nyg, ctx->avg_nu_t, dir, nchunk);
+        k_dsm_e<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>(ctx->dsm_part, nch, ctx->nyg, ctx->avg_nu_t, dir, nbase);
     count_launch(ctx, "k_dsm_e");
-    // stage F (nu_t = max(-C(j)|S|/2, 0) everywhere) is left to the readers,
-    // as after the one-pass kernel: |S| sits in the same canonical slot, the
-    // fused RHS forms nu_t in its loader and the other readers (eqwm,
-    // statistics, downloads) materialise it first
     ctx->nut_lazy = true;
     CF_CUDA(cudaGetLastError());
     return 0;
 }
 
-template int launch_dsm<double>(cf_ctx *, int);
-template int launch_dsm<float>(cf_ctx *, int);
+// FP64: two kernels that read U, V, W at actual indices, whatever the state
+// of the ghosts and with either wall treatment (k_dsm64.cu).
+template <>
+int launch_dsm<double>(cf_ctx *ctx, int b) {
+    int nch;
+    if (int rc = launch_dsm64(ctx, b, &nch)) return rc;
+    return launch_dsm_e(ctx, nch, nch);
+}
+
+template <>
+int launch_dsm<float>(cf_ctx *ctx, int b) {
+    Can c;
+    c.nxp = ctx->nxp; c.nym = ctx->nym; c.nzp = ctx->nzp; c.n = (long)ctx->nCan;
+    if (ctx->use_fused_dsm && ctx->state_periodic && (ctx->prm.iwall_model == 0 || ctx->prm.iwall_model == 3)) {
+        // one pass: |S| and the plane partial sums (k_dsm_fused.cu); with the
+        // wall model the seam band is computed by k_dsm_seam
+        int rc = ctx->prm.iwall_model == 0 ? launch_dsm_fused<float>(ctx, b) : launch_dsm_fused_wm<float>(ctx, b);
+        if (rc) return rc;
+        return launch_dsm_e(ctx, ctx->dsm_nchunk_fused, ctx->dsm_nchunk_base);
+    }
+    GeoT<float> g = geo_of<float>(ctx);
+    Fld<float> U = make_fld<float>(ctx->U[b], ctx->nx, ctx->nyg);
+    Fld<float> V = make_fld<float>(ctx->V[b], ctx->nxg, ctx->ny);
+    Fld<float> W = make_fld<float>(ctx->W[b], ctx->nxg, ctx->nyg);
+    float *q = (float *)ctx->dsm_q;
+    const RcpT<float> rc = rcp_of<float>(ctx);
+    const dim3 blk(32, 4, 1), grdc(cdiv(ctx->nxp, 32), cdiv(ctx->nym, 4), ctx->nzp);
+    k_dsm_a<float><<<grdc, blk, 0, ctx->st>>>(g, rc, U, V, W, q, c);
+    count_launch(ctx, "k_dsm_a");
+    Fld<float> Uf = make_fld<float>(ctx->Uf, ctx->nx, ctx->nyg);
+    Fld<float> Vf = make_fld<float>(ctx->Vf, ctx->nxg, ctx->ny);
+    Fld<float> Wf = make_fld<float>(ctx->Wf, ctx->nxg, ctx->nyg);
+    {
+        // z chunks of 16 canonical planes
+        const int kc = 16, nkc = cdiv(ctx->nzp, kc), ntx = cdiv(ctx->nxp, 32);
+        k_dsm_c_t<float><<<dim3(ntx, cdiv(ctx->nyg, 8), nkc), 256, 0, ctx->st>>>(U, Uf, ctx->nx, ctx->nyg, ctx->nzg, ctx->nxp, ctx->nzp, kc);
+        k_dsm_c_t<float><<<dim3(ntx, cdiv(ctx->ny, 8), nkc), 256, 0, ctx->st>>>(V, Vf, ctx->nxg, ctx->ny, ctx->nzg, ctx->nxp, ctx->nzp, kc);
+        k_dsm_c_t<float><<<dim3(ntx, cdiv(ctx->nyg, 8), nkc), 256, 0, ctx->st>>>(W, Wf, ctx->nxg, ctx->nyg, ctx->nz, ctx->nxp, ctx->nzp, kc);
+    }
+    count_launch(ctx, "k_dsm_c_t"); count_launch(ctx, "k_dsm_c_t"); count_launch(ctx, "k_dsm_c_t");
+    // z chunks planned at context creation (dsm_b_plan), within the plane-partial slots
+    const int ntx = cdiv(ctx->nxp, DB_X);
+    const long nkc = std::max(1L, std::min((long)std::max(ctx->dsmb_nkc, 1), (long)ctx->dsm_part_nch / ntx));
+    const int kc_len = cdiv(ctx->nzp, nkc);
+    const int nz_chunks = cdiv(ctx->nzp, kc_len);
+    const int nchunk = ntx * nz_chunks;
+    const dim3 grd(ntx, cdiv(ctx->nym, DB_Y), nz_chunks);
+    CUtensorMap tm;
+    if (dsmb_tma(ctx)) {
+        std::memcpy(&tm, ctx->dsmb_map, sizeof(tm));
+        k_dsm_b<true><<<grd, DB_X * DB_Y, dsm_b_smem<true>(), ctx->st>>>(tm, q, g, rc, Uf, Vf, Wf, c, ctx->nyg, kc_len,
+                                                                         ctx->dsm_part, nchunk, ctx->ds,
+                                                                         ctx->dsmb_skip_first);
+    } else {
+        std::memset(&tm, 0, sizeof(tm));  // not read by the per-element gather
+        k_dsm_b<false><<<grd, DB_X * DB_Y, dsm_b_smem<false>(), ctx->st>>>(tm, q, g, rc, Uf, Vf, Wf, c, ctx->nyg, kc_len,
+                                                                           ctx->dsm_part, nchunk, ctx->ds, 0);
+    }
+    count_launch(ctx, "k_dsm_b");
+    return launch_dsm_e(ctx, nchunk, nchunk);
+}
+
 template int launch_nut_zero<double>(cf_ctx *);
 template int launch_nut_materialize<double>(cf_ctx *);
 template int launch_nut_materialize<float>(cf_ctx *);
@@ -735,13 +699,9 @@ template int launch_nut_zero<float>(cf_ctx *);
 // z chunks of the multi-pass filter kernel: the count that minimises (waves
 // of resident blocks) x (planes per chunk + the 2 halo planes a chunk loads
 // again); its plane partials take ceil(nxp / 32) x nkc slots per row
-int dsm_b_plan(int esz, int nxp, int nym, int nzp, int sms) {
+int dsm_b_plan(int nxp, int nym, int nzp, int sms) {
     int per = 1;
-    if (esz == 4)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dsm_b<float, true>, DB_X * DB_Y, dsm_b_smem<float, true>());
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dsm_b<double, false>, DB_X * DB_Y,
-                                                      dsm_b_smem<double, false>());
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dsm_b<true>, DB_X * DB_Y, dsm_b_smem<true>());
     const long tiles = (long)cdiv(nxp, DB_X) * cdiv(nym, DB_Y), res = (long)(per < 1 ? 1 : per) * sms;
     long best = 1;
     double best_cost = 1e300;
@@ -759,11 +719,7 @@ int dsm_b_plan(int esz, int nxp, int nym, int nzp, int sms) {
 // shared-memory opt-in of the multi-pass filter kernel (two planes in dynamic
 // shared memory; called at context creation)
 int dsm_b_setup() {
-    cudaFuncSetAttribute(k_dsm_b<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)dsm_b_smem<float, true>());
-    cudaFuncSetAttribute(k_dsm_b<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)dsm_b_smem<float, false>());
-    cudaFuncSetAttribute(k_dsm_b<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)dsm_b_smem<double, false>());
+    cudaFuncSetAttribute(k_dsm_b<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm_b_smem<true>());
+    cudaFuncSetAttribute(k_dsm_b<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm_b_smem<false>());
     return 0;
 }

@@ -541,28 +541,20 @@ static int launch_fused_cfg(cf_ctx *ctx, int b, int kc_len) {
     return 0;
 }
 
-// tile shapes: FP32 32 x 8, FP64 16 x 8 (the FP64 kernel needs more registers
-// and twice the shared memory per tile).  32 x 16 FP32 tiles (one 512-thread
+// tile shape 32 x 8.  32 x 16 tiles (one 512-thread
 // block per SM, 144 KB) do less halo work but run about 5 % slower at
 // 192 x 128 x 192 cells (fewer blocks to hide each other's barriers); three
 // 32 x 8 blocks per SM neither fit in shared memory nor in 80 registers.
 template <typename T> struct DsmCfg;
 template <> struct DsmCfg<float> { static constexpr int TX = 32, TY = 8; };
-template <> struct DsmCfg<double> { static constexpr int TX = 16, TY = 8; };
 
 int dsm_fused_setup() {
     cudaFuncSetAttribute(k_dsm_fused_batch<float, DsmCfg<float>::TX, DsmCfg<float>::TY>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)DsmSmem<float, DsmCfg<float>::TX, DsmCfg<float>::TY>::bytes);
-    cudaFuncSetAttribute(k_dsm_fused_batch<double, DsmCfg<double>::TX, DsmCfg<double>::TY>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)DsmSmem<double, DsmCfg<double>::TX, DsmCfg<double>::TY>::bytes);
     cudaFuncSetAttribute(k_dsm_fused<float, DsmCfg<float>::TX, DsmCfg<float>::TY>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)DsmSmem<float, DsmCfg<float>::TX, DsmCfg<float>::TY>::bytes);
-    cudaFuncSetAttribute(k_dsm_fused<double, DsmCfg<double>::TX, DsmCfg<double>::TY>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)DsmSmem<double, DsmCfg<double>::TX, DsmCfg<double>::TY>::bytes);
     return 0;
 }
 
@@ -584,8 +576,8 @@ static int plan_t(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
     return 0;
 }
 
-int dsm_fused_plan(int esz, int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
-    return esz == 8 ? plan_t<double>(nxp, nym, nzp, sms, kc, nchunk) : plan_t<float>(nxp, nym, nzp, sms, kc, nchunk);
+int dsm_fused_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
+    return plan_t<float>(nxp, nym, nzp, sms, kc, nchunk);
 }
 
 template <typename T>
@@ -593,7 +585,6 @@ int launch_dsm_fused(cf_ctx *ctx, int b) {
     return launch_fused_cfg<T, DsmCfg<T>::TX, DsmCfg<T>::TY>(ctx, b, ctx->dsm_kc);
 }
 
-template int launch_dsm_fused<double>(cf_ctx *, int);
 template int launch_dsm_fused<float>(cf_ctx *, int);
 
 // ---------------------------------------------------------------------------
@@ -849,7 +840,6 @@ int launch_dsm_fused_wm(cf_ctx *ctx, int b) {
     return launch_seam<T>(ctx, b, chunk0, a.nchunk);
 }
 
-template int launch_dsm_fused_wm<double>(cf_ctx *, int);
 template int launch_dsm_fused_wm<float>(cf_ctx *, int);
 
 __global__ void __launch_bounds__(256) k_dsm_e_batch(const __grid_constant__ DsmEBatch B) {
@@ -935,5 +925,4 @@ int launch_dsm_batch(cudaStream_t st, cf_ctx *const *m, const int *buf, int n) {
     return cudaGetLastError() == cudaSuccess ? 0 : CF_ERR_CUDA;
 }
 
-template int launch_dsm_batch<double>(cudaStream_t, cf_ctx *const *, const int *, int);
 template int launch_dsm_batch<float>(cudaStream_t, cf_ctx *const *, const int *, int);

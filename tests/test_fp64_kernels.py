@@ -43,3 +43,32 @@ def test_projection_edges(dims):
     assert_close(g["P"], f["P"], 1e-11, "P")
     ch.close()
     o.close()
+
+
+@pytest.mark.parametrize("dims,wall,kw", [((6, 5, 6), 0, {}), ((18, 6, 8), 0, {}), ((22, 9, 34), 0, {"dirichlet": 1}),
+                                          ((34, 17, 12), 0, {}), ((50, 7, 18), 0, {}), ((66, 12, 20), 0, {}),
+                                          ((18, 17, 18), 3, {}), ((34, 8, 22), 3, {}), ((50, 13, 10), 3, {})])
+def test_dsm_segments_and_chunks(dims, wall, kw):
+    """The FP64 dynamic Smagorinsky pass with one and several row segments of
+    16 and 32 lanes, full and ragged, rows packed in pairs (odd and even row
+    counts), chunks of one plane and more; with the wall model after an eqwm
+    boundary update, whose wall ghosts are not periodic at the seams.  nu_t
+    and the plane coefficients within the per-routine 1e-12."""
+    if wall:
+        case = channel_case(*dims, stretch=0.0, wall=3, retau=2000.0, profile="plug", jref=2, ncv=30)
+    else:
+        case = channel_case(*dims)
+    if "dirichlet" in kw:
+        case["prm"]["Dirichlet_nu_t"] = kw["dirichlet"]
+    o, ch = pair(case)
+    for d in (o, ch):
+        d.apply_boundary_conditions()
+        d.compute_eddy_viscosity()
+        if wall:
+            d.compute_wall_model()
+            d.apply_boundary_conditions()
+            d.compute_eddy_viscosity()
+    assert_close(ch.download()["nu_t"], o.fields()["nu_t"], 1e-12, "nu_t")
+    assert_close(ch.avg_nu_t()[1:-1], o.array("avg_nu_t").ravel()[1:-1], 1e-12, "avg_nu_t")
+    ch.close()
+    o.close()
