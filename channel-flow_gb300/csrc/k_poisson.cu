@@ -29,6 +29,13 @@ template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
     return r;
 }
 template <typename C> __device__ __forceinline__ C cconj(C a) { a.y = -a.y; return a; }
+// a times -i (forward transforms) or +i (inverse): a swap and a sign, no arithmetic
+template <bool INV, typename C> __device__ __forceinline__ C crot(C a) {
+    C r;
+    r.x = INV ? -a.y : a.y;
+    r.y = INV ? a.x : -a.x;
+    return r;
+}
 
 struct FftPlan {
     int n, nrad, rad[8];
@@ -36,7 +43,7 @@ struct FftPlan {
 
 // One line of length n held in smem a (ping) / b (pong); the G threads of a
 // group (index tid) cooperate; returns the buffer holding the result.
-template <typename C>
+template <bool INV, typename C>
 __device__ C *fft_smem(C *a, C *b, const FftPlan &pl, const C *tw, int tid, int G) {
     const int n = pl.n;
     int Ns = 1;
@@ -56,9 +63,8 @@ __device__ C *fft_smem(C *a, C *b, const FftPlan &pl, const C *tw, int tid, int 
                 v[0] = cadd(t0, v[1]);
                 v[1] = csub(t0, v[1]);
             } else if (R == 4) {
-                C w = tw[n / 4];  // sign*i
                 C s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-                C s13 = cadd(v[1], v[3]), d13 = cmul(csub(v[1], v[3]), w);
+                C s13 = cadd(v[1], v[3]), d13 = crot<INV>(csub(v[1], v[3]));
                 v[0] = cadd(s02, s13);
                 v[2] = csub(s02, s13);
                 v[1] = cadd(d02, d13);
@@ -124,16 +130,15 @@ constexpr int fft_rad(int n, int s) {
     return 1;
 }
 
-template <int R, int N, typename C>
+template <int R, int N, bool INV, typename C>
 __device__ __forceinline__ void butterfly(C *v, const C *tw) {
     if constexpr (R == 2) {
         C t0 = v[0];
         v[0] = cadd(t0, v[1]);
         v[1] = csub(t0, v[1]);
     } else if constexpr (R == 4) {
-        const C w = tw[N / 4];  // sign*i
         C s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-        C s13 = cadd(v[1], v[3]), d13 = cmul(csub(v[1], v[3]), w);
+        C s13 = cadd(v[1], v[3]), d13 = crot<INV>(csub(v[1], v[3]));
         v[0] = cadd(s02, s13);
         v[2] = csub(s02, s13);
         v[1] = cadd(d02, d13);
@@ -165,7 +170,7 @@ __device__ __forceinline__ void butterfly(C *v, const C *tw) {
     }
 }
 
-template <int N, int S, int NS, typename C>
+template <int N, int S, int NS, bool INV, typename C>
 __device__ __forceinline__ C *fft_fixed(C *a, C *b, const C *tw, int tid, int G) {
     if constexpr (S == fft_nrad(N)) {
         return a;
@@ -180,21 +185,21 @@ __device__ __forceinline__ C *fft_fixed(C *a, C *b, const C *tw, int tid, int G)
 #pragma unroll
                 for (int r = 1; r < R; r++) v[r] = cmul(v[r], tw[r * k * step]);
             }
-            butterfly<R, N>(v, tw);
+            butterfly<R, N, INV>(v, tw);
             const int d = (j / NS) * NS * R + k;
 #pragma unroll
             for (int r = 0; r < R; r++) b[d + r * NS] = v[r];
         }
         __syncthreads();
-        return fft_fixed<N, S + 1, NS * R, C>(b, a, tw, tid, G);
+        return fft_fixed<N, S + 1, NS * R, INV, C>(b, a, tw, tid, G);
     }
 }
 
 // One line: the compile-time transform when N > 0, else the plan's.
-template <int N, typename C>
+template <int N, bool INV, typename C>
 __device__ __forceinline__ C *fft_line(C *a, C *b, const FftPlan &pl, const C *tw, int tid, int G) {
-    if constexpr (N > 0) return fft_fixed<N, 0, 1, C>(a, b, tw, tid, G);
-    else return fft_smem<C>(a, b, pl, tw, tid, G);
+    if constexpr (N > 0) return fft_fixed<N, 0, 1, INV, C>(a, b, tw, tid, G);
+    else return fft_smem<INV, C>(a, b, pl, tw, tid, G);
 }
 
 // Copies the twiddle table to shared memory (compile-time sizes only).
@@ -298,7 +303,7 @@ __global__ void k_fwd_x(GeoT<T> g, Fld<T> U, Fld<T> V, Fld<T> W, typename C2<T>:
         }
     }
     __syncthreads();
-    C *r = fft_line<N, C>(a, b, pl, tw, tid, G);
+    C *r = fft_line<N, false, C>(a, b, pl, tw, tid, G);
     if (!active) return;
     const int nh = n / 2 + 1;
     C *o0 = spec + ((long)(j - 2) * nzp + (k - 2)) * nh;
@@ -325,7 +330,7 @@ __global__ void k_fwd_x(GeoT<T> g, Fld<T> U, Fld<T> V, Fld<T> W, typename C2<T>:
 // thread copies every 16th element of its line
 constexpr int FFTZ_KZS = 16;
 
-template <typename T, int N>
+template <typename T, int N, bool INV>
 __global__ void k_fft_z(typename C2<T>::t *spec, FftPlan pl, const typename C2<T>::t *tw_g, int nlines, int nh, int LB) {
     typedef typename C2<T>::t C;
     extern __shared__ unsigned char smraw[];
@@ -357,7 +362,7 @@ __global__ void k_fft_z(typename C2<T>::t *spec, FftPlan pl, const typename C2<T
     __syncthreads();
     const int l = threadIdx.x / G, tid = threadIdx.x % G;
     C *a = sm + (long)l * LS, *b = a + n;
-    C *r = fft_line<N, C>(a, b, pl, tw, tid, G);
+    C *r = fft_line<N, INV, C>(a, b, pl, tw, tid, G);
     // r is a or b for every line alike (same number of stages)
     long roff = r - a;
     if (lact)
@@ -391,10 +396,10 @@ constexpr int ZR_T = 256;  // threads per block
 // roots W_R^m = tw[(N/R) m] from the length-N table.
 template <int R> constexpr int reg_ra() { return R % 4 == 0 ? 4 : (R % 2 == 0 ? 2 : (R % 3 == 0 ? 3 : 5)); }
 
-template <int R, int N, typename C>
+template <int R, int N, bool INV, typename C>
 __device__ __forceinline__ void reg_dft(C *v, const C *tw) {
     if constexpr (R == 2 || R == 3 || R == 4 || R == 5) {
-        butterfly<R, N>(v, tw);
+        butterfly<R, N, INV>(v, tw);
     } else if constexpr (R > 5) {
         constexpr int Ra = reg_ra<R>(), Rb = R / Ra;
         C u[R];
@@ -403,23 +408,23 @@ __device__ __forceinline__ void reg_dft(C *v, const C *tw) {
             C s[Ra];
 #pragma unroll
             for (int ra = 0; ra < Ra; ra++) s[ra] = v[Rb * ra + rb];
-            reg_dft<Ra, N>(s, tw);
+            reg_dft<Ra, N, INV>(s, tw);
 #pragma unroll
-            for (int qa = 0; qa < Ra; qa++) u[rb * Ra + qa] = (rb * qa) ? cmul(s[qa], tw[(N / R) * rb * qa]) : s[qa];
+            for (int qa = 0; qa < Ra; qa++) u[rb * Ra + qa] = (rb * qa) == 0 ? s[qa] : (4 * rb * qa == R ? crot<INV>(s[qa]) : cmul(s[qa], tw[(N / R) * rb * qa]));
         }
 #pragma unroll
         for (int qa = 0; qa < Ra; qa++) {
             C s[Rb];
 #pragma unroll
             for (int rb = 0; rb < Rb; rb++) s[rb] = u[rb * Ra + qa];
-            reg_dft<Rb, N>(s, tw);
+            reg_dft<Rb, N, INV>(s, tw);
 #pragma unroll
             for (int qb = 0; qb < Rb; qb++) v[qa + Ra * qb] = s[qb];
         }
     }
 }
 
-template <typename T, int N>
+template <typename T, int N, bool INV>
 __global__ void __launch_bounds__(ZR_T) k_fft_zr(typename C2<T>::t *__restrict__ spec,
                                                  const typename C2<T>::t *__restrict__ tw_g, int nlines, int nh) {
     typedef typename C2<T>::t C;
@@ -452,7 +457,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr(typename C2<T>::t *__restrict__
         // one stage (N = R0): the DFT of the line, stored in natural order
 #pragma unroll
         for (int it = 0; it < I0; it++) {
-            reg_dft<R0, N>(v[it], stw);
+            reg_dft<R0, N, INV>(v[it], stw);
             if (act && t + it * G < NB0) {
 #pragma unroll
                 for (int r = 0; r < R0; r++) spec[gb + (long)r * nh] = v[it][r];
@@ -464,7 +469,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr(typename C2<T>::t *__restrict__
         for (int it = 0; it < I0; it++) {
             const int j = t + it * G;
             if (j < NB0) {
-                reg_dft<R0, N>(v[it], stw);
+                reg_dft<R0, N, INV>(v[it], stw);
 #pragma unroll
                 for (int r = 0; r < R0; r++) bl[j * R0 + r] = v[it][r];
             }
@@ -481,7 +486,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr(typename C2<T>::t *__restrict__
                 for (int r = 0; r < R1; r++) w[r] = bl[j + r * NB1];
 #pragma unroll
                 for (int r = 1; r < R1; r++) w[r] = cmul(w[r], stw[r * j]);
-                reg_dft<R1, N>(w, stw);
+                reg_dft<R1, N, INV>(w, stw);
                 if (act) {
 #pragma unroll
                     for (int r = 0; r < R1; r++) spec[gb + (long)(j + r * R0) * nh] = w[r];
@@ -498,7 +503,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr(typename C2<T>::t *__restrict__
 constexpr int zr3_r(int n, int s) { return n == 384 ? (s < 2 ? 8 : 6) : (n == 512 ? 8 : 0); }
 constexpr int ZR3_G = 32;  // threads per line (two or fewer butterflies of each stage per thread)
 
-template <typename T, int N>
+template <typename T, int N, bool INV>
 __global__ void __launch_bounds__(ZR_T) k_fft_zr3(typename C2<T>::t *__restrict__ spec,
                                                   const typename C2<T>::t *__restrict__ tw_g, int nlines, int nh) {
     typedef typename C2<T>::t C;
@@ -533,7 +538,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr3(typename C2<T>::t *__restrict_
         for (int it = 0; it < I0; it++) {
             const int j = t + it * G;
             if (j < NB0) {
-                reg_dft<R0, N>(v[it], stw);
+                reg_dft<R0, N, INV>(v[it], stw);
 #pragma unroll
                 for (int r = 0; r < R0; r++) bl[j * R0 + r] = v[it][r];
             }
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr3(typename C2<T>::t *__restrict_
         for (int it = 0; it < I1; it++) {
             const int j = t + it * G, k = j % NS1;
             if (j < NB1) {
-                reg_dft<R1, N>(w[it], stw);
+                reg_dft<R1, N, INV>(w[it], stw);
                 const int d = (j / NS1) * NS1 * R1 + k;
 #pragma unroll
                 for (int r = 0; r < R1; r++) bl[d + r * NS1] = w[it][r];
@@ -576,7 +581,7 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr3(typename C2<T>::t *__restrict_
             for (int r = 0; r < R2; r++) w[r] = bl[j + r * NB2];
 #pragma unroll
             for (int r = 1; r < R2; r++) w[r] = cmul(w[r], stw[r * j]);
-            reg_dft<R2, N>(w, stw);
+            reg_dft<R2, N, INV>(w, stw);
             if (act) {
 #pragma unroll
                 for (int r = 0; r < R2; r++) spec[gb + (long)(j + r * NS2) * nh] = w[r];
@@ -618,7 +623,7 @@ template <int N> constexpr int xr_ls() { return N + N / xr_r(N, 0); }
 // A middle Stockham stage (span NS, radix R) of a padded line in place:
 // every thread reads its butterflies' inputs and applies the twiddles, a
 // barrier, then the DFTs and the writes (G threads per line, thread t).
-template <int N, int R, int NS, int G, typename C>
+template <int N, int R, int NS, int G, bool INV, typename C>
 __device__ __forceinline__ void xr_mid_stage(C *bl, const C *stw, int t) {
     constexpr int NB = N / R, I = (NB + G - 1) / G, ST = N / (NS * R);
     C w[I][R];
@@ -637,7 +642,7 @@ __device__ __forceinline__ void xr_mid_stage(C *bl, const C *stw, int t) {
     for (int it = 0; it < I; it++) {
         const int j = t + it * G, k = j % NS;
         if (j < NB) {
-            reg_dft<R, N>(w[it], stw);
+            reg_dft<R, N, INV>(w[it], stw);
             const int d = (j / NS) * NS * R + k;
 #pragma unroll
             for (int r = 0; r < R; r++) bl[xr_pos<N>(d + r * NS)] = w[it][r];
@@ -713,7 +718,7 @@ __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, 
         if (jb < NB0) {
 #pragma unroll
             for (int r = 0; r < R0; r++) v[it][r] = bl[xr_pos<N>(jb + NB0 * r)];
-            reg_dft<R0, N>(v[it], stw);
+            reg_dft<R0, N, false>(v[it], stw);
         }
     }
     __syncthreads();
@@ -727,7 +732,7 @@ __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, 
     }
     if constexpr (R2 > 1) {
         __syncthreads();
-        xr_mid_stage<N, R1, R0, G>(bl, stw, t);
+        xr_mid_stage<N, R1, R0, G, false>(bl, stw, t);
     }
     if constexpr (R1 > 1) {
         __syncthreads();
@@ -742,7 +747,7 @@ __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, 
                 for (int r = 0; r < RL; r++) w[r] = bl[xr_pos<N>(jb + r * NSL)];
 #pragma unroll
                 for (int r = 1; r < RL; r++) w[r] = cmul(w[r], stw[r * jb]);
-                reg_dft<RL, N>(w, stw);
+                reg_dft<RL, N, false>(w, stw);
 #pragma unroll
                 for (int r = 0; r < RL; r++) bl[xr_pos<N>(jb + r * NSL)] = w[r];
             }
@@ -810,7 +815,7 @@ __global__ void __launch_bounds__(ZR_T) k_inv_xr(const typename C2<T>::t *__rest
     __syncthreads();
     T *p0 = phi + (long)N * (jj + (long)nym * kk), *p1 = phi + (long)N * (jj + (long)nym * (kk + 1));
     if constexpr (R1 == 1) {
-        reg_dft<R0, N>(v[0], stw);
+        reg_dft<R0, N, true>(v[0], stw);
         if (act) {
 #pragma unroll
             for (int r = 0; r < R0; r++) {
@@ -824,14 +829,14 @@ __global__ void __launch_bounds__(ZR_T) k_inv_xr(const typename C2<T>::t *__rest
         for (int it = 0; it < I0; it++) {
             const int jb = t + it * G;
             if (jb < NB0) {
-                reg_dft<R0, N>(v[it], stw);
+                reg_dft<R0, N, true>(v[it], stw);
 #pragma unroll
                 for (int r = 0; r < R0; r++) bl[xr_pos<N>(jb * R0 + r)] = v[it][r];
             }
         }
         __syncthreads();
         if constexpr (R2 > 1) {
-            xr_mid_stage<N, R1, R0, G>(bl, stw, t);
+            xr_mid_stage<N, R1, R0, G, true>(bl, stw, t);
             __syncthreads();
         }
         // last stage (span NSL = NBL, twiddle step 1): phi stored directly
@@ -844,7 +849,7 @@ __global__ void __launch_bounds__(ZR_T) k_inv_xr(const typename C2<T>::t *__rest
                 for (int r = 0; r < RL; r++) w[r] = bl[xr_pos<N>(jb + r * NSL)];
 #pragma unroll
                 for (int r = 1; r < RL; r++) w[r] = cmul(w[r], stw[r * jb]);
-                reg_dft<RL, N>(w, stw);
+                reg_dft<RL, N, true>(w, stw);
                 if (act) {
 #pragma unroll
                     for (int r = 0; r < RL; r++) {
@@ -1498,7 +1503,7 @@ __global__ void k_inv_x(const typename C2<T>::t *spec, T *phi, FftPlan pl, const
         }
     }
     __syncthreads();
-    C *r = fft_line<N, C>(a, b, pl, tw, tid, G);
+    C *r = fft_line<N, true, C>(a, b, pl, tw, tid, G);
     if (!active) return;
     long base0 = (long)n * (jj + (long)nym * kk), base1 = (long)n * (jj + (long)nym * (kk + 1));
 #pragma unroll
@@ -1745,13 +1750,13 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
     if constexpr (xr_r(N, 0) > 0) k_fwd_xr<T, N><<<cdiv(npairs, ZR_T / XR_FT), ZR_T, xr_fwd_smem<T, N>(), ctx->st>>>(g, U, V, W, spec, twxf, rs); \
     else k_fwd_x<T, N><<<cdiv(npairs, LP), LP * Gx, shx, ctx->st>>>(g, U, V, W, spec, px, twxf, LP, rs); \
     break;
-#define CF_FFTZ(N, TW) case N: \
-    if constexpr (zr_r0(N) > 0) k_fft_zr<T, N><<<cdiv(nlines, ZR_T / zr_threads(N)), ZR_T, zr_smem<T, N>(), ctx->st>>>(spec, TW, (int)nlines, nh); \
-    else if constexpr (zr3_r(N, 0) > 0) k_fft_zr3<T, N><<<cdiv(nlines, ZR_T / ZR3_G), ZR_T, zr3_smem<T, N>(), ctx->st>>>(spec, TW, (int)nlines, nh); \
-    else k_fft_z<T, N><<<cdiv(nlines, LB), LB * Gz, shz, ctx->st>>>(spec, pz, TW, (int)nlines, nh, LB); \
+#define CF_FFTZ(N, TW, INV) case N: \
+    if constexpr (zr_r0(N) > 0) k_fft_zr<T, N, INV><<<cdiv(nlines, ZR_T / zr_threads(N)), ZR_T, zr_smem<T, N>(), ctx->st>>>(spec, TW, (int)nlines, nh); \
+    else if constexpr (zr3_r(N, 0) > 0) k_fft_zr3<T, N, INV><<<cdiv(nlines, ZR_T / ZR3_G), ZR_T, zr3_smem<T, N>(), ctx->st>>>(spec, TW, (int)nlines, nh); \
+    else k_fft_z<T, N, INV><<<cdiv(nlines, LB), LB * Gz, shz, ctx->st>>>(spec, pz, TW, (int)nlines, nh, LB); \
     break;
-#define CF_FFTZF(N) CF_FFTZ(N, twzf)
-#define CF_FFTZB(N) CF_FFTZ(N, twzb)
+#define CF_FFTZF(N) CF_FFTZ(N, twzf, false)
+#define CF_FFTZB(N) CF_FFTZ(N, twzb, true)
 #define CF_INVX(N) case N: \
     if constexpr (xr_r(N, 0) > 0) k_inv_xr<T, N><<<cdiv(npairs, ZR_T / xr_threads(N)), ZR_T, xr_smem<T, N>(), ctx->st>>>(spec, phi, twxb, nym, nzp, scale); \
     else k_inv_x<T, N><<<cdiv(npairs, LP), LP * Gx, shx, ctx->st>>>(spec, phi, px, twxb, nym, nzp, LP, scale); \
@@ -1766,7 +1771,7 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
     // forward z
     switch (nzp) {
         CF_FFT_SIZES(CF_FFTZF)
-        default: k_fft_z<T, 0><<<cdiv(nlines, LB), LB * Gz, shz, ctx->st>>>(spec, pz, twzf, (int)nlines, nh, LB);
+        default: k_fft_z<T, 0, false><<<cdiv(nlines, LB), LB * Gz, shz, ctx->st>>>(spec, pz, twzf, (int)nlines, nh, LB);
     }
     count_launch(ctx, "k_fft_z");
     }
@@ -1814,7 +1819,7 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
     // inverse z
     switch (nzp) {
         CF_FFT_SIZES(CF_FFTZB)
-        default: k_fft_z<T, 0><<<cdiv(nlines, LB), LB * Gz, shz, ctx->st>>>(spec, pz, twzb, (int)nlines, nh, LB);
+        default: k_fft_z<T, 0, true><<<cdiv(nlines, LB), LB * Gz, shz, ctx->st>>>(spec, pz, twzb, (int)nlines, nh, LB);
     }
     count_launch(ctx, "k_fft_z");
     // inverse x
@@ -2006,15 +2011,18 @@ template <typename T, int N>
 static void fft_attrs_one() {
     cudaFuncSetAttribute(k_fwd_x<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     cudaFuncSetAttribute(k_inv_x<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    cudaFuncSetAttribute(k_fft_z<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    cudaFuncSetAttribute(k_fft_z<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    cudaFuncSetAttribute(k_fft_z<T, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     if constexpr (zr3_r(N, 0) > 0) {
-        cudaFuncSetAttribute(k_fft_zr3<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zr3_smem<T, N>());
+        cudaFuncSetAttribute(k_fft_zr3<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zr3_smem<T, N>());
+        cudaFuncSetAttribute(k_fft_zr3<T, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zr3_smem<T, N>());
         cudaFuncSetAttribute(k_fwd_xr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xr_fwd_smem<T, N>());
         cudaFuncSetAttribute(k_inv_xr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xr_smem<T, N>());
     }
     if constexpr (zr_r0(N) > 0) {
         // exactly what the launches request (up to 110 KB: FP64, length 96)
-        cudaFuncSetAttribute(k_fft_zr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zr_smem<T, N>());
+        cudaFuncSetAttribute(k_fft_zr<T, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zr_smem<T, N>());
+        cudaFuncSetAttribute(k_fft_zr<T, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zr_smem<T, N>());
         cudaFuncSetAttribute(k_fwd_xr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xr_fwd_smem<T, N>());
         cudaFuncSetAttribute(k_inv_xr<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xr_smem<T, N>());
     }
