@@ -99,6 +99,9 @@ static int alloc_all(cf_ctx *ctx) {
         TRY(alloc<T>(ctx, &ctx->Uf, ctx->nU));
         TRY(alloc<T>(ctx, &ctx->Vf, ctx->nV));
         TRY(alloc<T>(ctx, &ctx->Wf, ctx->nW));
+        // in the filtered quantities' place, which are no longer read when nu_t is wanted
+        // (12 nCan >= nC from the smallest grid on)
+        if (sizeof(T) == 8) ctx->nut_rhs = (T *)ctx->dsm_q + 3 * ctx->nCan;
     }
     TRY(alloc<T>(ctx, &ctx->phi, ctx->nCan));
     TRY(alloc<T>(ctx, &ctx->spec, 2 * ctx->nSpec));
@@ -504,19 +507,23 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
             nch_fused = (size_t)dsm64_slots(nxp, nzp, 1);  // any chunk length
         }
         ctx->use_fused_dsm = !p->dsm_unfused;
-        // fused RHS: 32 x 8 column tiles, z chunks for ~4 resident blocks per SM
-        long rt = (long)cdiv(ctx->nxp, 32) * cdiv(ctx->nyg - 2, 8);
-        // z chunks: the count that minimises (waves of resident blocks) x
-        // (planes per chunk + the 2 halo planes a chunk loads again)
-        const long res = (long)rhs3_blocks_per_sm(p->precision == CF_PREC_SPLIT ? 4 : 8) * dev_sms;
-        long best = 1;
-        double best_cost = 1e300;
-        for (long n = 1; n <= std::max(1L, (long)ctx->nzp / 4); n++) {
-            const double waves = (double)((rt * n + res - 1) / res);
-            const double cost = waves * ((double)cdiv(ctx->nzp, n) + 2.0);
-            if (cost < best_cost - 1e-9) { best_cost = cost; best = n; }
+        if (ctx->esz == 8) {
+            ctx->rhs_nkc = rhs64_plan(nxp, ctx->nym, nzp, dev_sms);
+        } else {
+            // fused RHS: 32 x 8 column tiles; z chunks: the count that
+            // minimises (waves of resident blocks) x (planes per chunk + the
+            // 2 halo planes a chunk loads again)
+            long rt = (long)cdiv(ctx->nxp, 32) * cdiv(ctx->nyg - 2, 8);
+            const long res = (long)rhs3_blocks_per_sm() * dev_sms;
+            long best = 1;
+            double best_cost = 1e300;
+            for (long n = 1; n <= std::max(1L, (long)ctx->nzp / 4); n++) {
+                const double waves = (double)((rt * n + res - 1) / res);
+                const double cost = waves * ((double)cdiv(ctx->nzp, n) + 2.0);
+                if (cost < best_cost - 1e-9) { best_cost = cost; best = n; }
+            }
+            ctx->rhs_nkc = (int)best;
         }
-        ctx->rhs_nkc = (int)best;
         if (p->LES_model == 3) amd_plan(p->precision == CF_PREC_SPLIT ? 4 : 8, nxp, ctx->nym, nzp, dev_sms, &ctx->amd_nkc, &amd_parts);
     }
     // (with the wall model the one-pass kernel's slots are followed by the seam band's)
@@ -1161,7 +1168,7 @@ static int step_eager(cf_ctx *ctx) { return DISPATCH(enqueue_step<double>(ctx), 
 // Each member's launches are those of enqueue_seg in the same order.
 // ---------------------------------------------------------------------------
 static bool dsm_batchable(const cf_ctx *c) {
-    return c->esz == 4 && c->prm.LES_model == 2 && c->use_fused_dsm && c->prm.iwall_model == 0 && c->state_periodic && c->use_rhs3;
+    return c->esz == 4 && c->prm.LES_model == 2 && c->use_fused_dsm && c->prm.iwall_model == 0 && c->state_periodic;
 }
 
 static void ens_bufs(const cf_ctx *c, int s, int *src, int *dst) {
@@ -1648,9 +1655,15 @@ static int capture_batched_step(cf_ensemble *e, int *extra) {
                 *extra += 2;
             }
             if (!rc && !rm.empty()) {
-                rc = esz == 8 ? launch_rhs3_batch<double>(e->st, rm.data(), s, rs.data(), rd.data(), (int)rm.size())
-                              : launch_rhs3_batch<float>(e->st, rm.data(), s, rs.data(), rd.data(), (int)rm.size());
-                *extra += 1;
+                if (esz == 4) {
+                    rc = launch_rhs3_batch<float>(e->st, rm.data(), s, rs.data(), rd.data(), (int)rm.size());
+                    *extra += 1;
+                } else {  // FP64 members: their own launches, one after the other
+                    for (size_t q = 0; q < rm.size() && !rc; q++) {
+                        *extra += 1;
+                        rc = launch_rhs64(rm[q], e->st, s, rs[q], rd[q]);
+                    }
+                }
             }
         }
         if (rc) break;

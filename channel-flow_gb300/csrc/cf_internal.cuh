@@ -47,6 +47,12 @@ __host__ __device__ static inline Fld<T> make_fld(void *p, int n1, int n2) {
     return f;
 }
 
+// one field per velocity component
+template <typename T>
+struct Trio {
+    Fld<T> u, v, w;
+};
+
 // Grid geometry (device pointers, 1-based: x[1..nx]); T = double or float.
 template <typename T>
 struct GeoT {
@@ -207,6 +213,7 @@ struct cf_ctx {
     void *Ulo[3] = {}, *Vlo[3] = {}, *Wlo[3] = {};  // split path: low words
     int cur = 0, old = 0;              // current state and Uo buffers
     void *nut = nullptr, *P = nullptr;
+    void *nut_rhs = nullptr;           // FP64 dynamic model: nu_t as the fused right-hand side reads it
     void *F[3][3] = {};                // [slot 0..2][comp]
     // eddy viscosity
     void *dsm_q = nullptr;             // 16 canonical arrays
@@ -226,7 +233,6 @@ struct cf_ctx {
     alignas(64) unsigned char dsmb_map[128] = {};
     int dsmb_map_state = 0;
     int dsmb_skip_first = 0;
-    bool use_rhs3 = true;              // one fused RHS + update launch per substep
     int rhs_nkc = 1;                   // z chunks of the fused RHS
     int amd_nkc = 1;                   // z chunks of the AMD pass
     int seg_base = 0;                  // buffer a step in segments started from
@@ -301,7 +307,10 @@ int cf_fail(cf_ctx *ctx, int code, const std::string &msg);
 template <typename T> int launch_bc(cf_ctx *ctx, int buf, bool lo = true);  // apply_boundary_conditions (lo: low words too)
 template <typename T> int check_bc(cf_ctx *ctx, int buf, bool *ok);      // ghosts already as the BCs leave them?
 template <typename T> int launch_rhs(cf_ctx *ctx, int comp, int slot);     // store F slot
-int rhs3_blocks_per_sm(int esz);
+int rhs3_blocks_per_sm();
+int rhs64_plan(int nxp, int nym, int nzp, int sms);                        // z chunks of the FP64 right-hand side
+int launch_rhs64(cf_ctx *ctx, cudaStream_t st, int s, int src, int dst);    // FP64 RHS + RK update
+int launch_rhs64_comp(cf_ctx *ctx, int comp, int slot);                     // one FP64 right-hand side into slot
 template <typename T> int launch_rhs_update(cf_ctx *ctx, int s, int src, int dst);  // fused RHS + RK update
 template <typename T> int launch_rk_update(cf_ctx *ctx, int s);            // from stored F slots
 template <typename T> int launch_dsm(cf_ctx *ctx, int buf);                // eddy viscosity
@@ -314,10 +323,11 @@ int dsm_seam_slots_max();                                                  // pa
 constexpr int CF_ENS_MAXM = 32;  // channels per batched ensemble launch at most
 // fused pass + <LM>/<MM> rows of n channels in two launches (ensembles)
 template <typename T> int launch_dsm_batch(cudaStream_t st, cf_ctx *const *m, const int *buf, int n);
-// fused right-hand sides + RK update of substep s of n channels in one launch
+// fused right-hand sides + RK update of substep s of n split-path channels in one launch
 template <typename T> int launch_rhs3_batch(cudaStream_t st, cf_ctx *const *m, int s, const int *src, const int *dst, int n);
 template <typename T> int launch_nut_zero(cf_ctx *ctx);
 template <typename T> int launch_nut_materialize(cf_ctx *ctx);       // fill nut if held lazily
+int launch_nut_rhs64(cf_ctx *ctx, cudaStream_t st, void **field);    // nu_t for the FP64 right-hand side
 template <typename T> int launch_nut_wall_rows(cf_ctx *ctx);         // its rows 1, 2, nyg-1, nyg only (stays lazy)
 // canon: project the canonical cells only (the boundary conditions that
 // follow rewrite the periodic duplicates)

@@ -401,72 +401,10 @@ __device__ __forceinline__ void rhs_zflux_dn(const GeoT<T> &g, const RC &rc, con
     }
 }
 
-// RK3 stage update of one point (time_integration.f90:108-110, 124-126,
-// 140-145) with F2 never reused (rk_coef(3,2) = 0, initialization.f90:416).
-// The split path keeps u^n as hi + lo; substep 3 writes the new low word.
-template <typename T>
-__device__ __forceinline__ void rk_store(T r, int i, int j, int k, const Fld<T> &out, const Fld<T> &F1,
-                                         const Fld<T> &Uo, const Fld<T> &Uolo, const Fld<T> &Unlo, int s,
-                                         const RkCoef &rk, T dt) {
-    T inc;
-    if (s == 1) {
-        F1(i, j, k) = r;
-        inc = dt * T(rk.c[1][1]) * r;
-    } else if (s == 2) {
-        inc = dt * (T(rk.c[2][1]) * F1(i, j, k) + T(rk.c[2][2]) * r);
-    } else {
-        inc = dt * (T(rk.c[3][1]) * F1(i, j, k) + T(rk.c[3][3]) * r);
-    }
-    if constexpr (sizeof(T) == 4) {
-        if (Uolo.p) {
-            float hi = Uo(i, j, k), lo = Uolo(i, j, k);
-            if (Unlo.p) {
-                ff_add(hi, lo, inc);
-                out(i, j, k) = hi;
-                Unlo(i, j, k) = lo;
-            } else {
-                out(i, j, k) = hi + (lo + inc);
-            }
-            return;
-        }
-    }
-    out(i, j, k) = Uo(i, j, k) + inc;
-}
-
-// The same update with its operands already loaded (f1 = F1 for s > 1, uo and
-// uolo = the old state and its low word) and the substep's coefficients in T
-// (ca: of F1 -- or of r when s = 1 --, cb: of r).
-template <typename T>
-__device__ __forceinline__ void rk_apply(T r, T f1, T uo, T uolo, bool has_lo, int i, int j, int k, const Fld<T> &out,
-                                         const Fld<T> &F1, const Fld<T> &Unlo, int s, T ca, T cb, T dt) {
-    T inc;
-    if (s == 1) {
-        F1(i, j, k) = r;
-        inc = dt * ca * r;
-    } else {
-        inc = dt * (ca * f1 + cb * r);
-    }
-    if constexpr (sizeof(T) == 4) {
-        if (has_lo) {
-            float hi = uo, lo = uolo;
-            if (Unlo.p) {
-                ff_add(hi, lo, inc);
-                out(i, j, k) = hi;
-                Unlo(i, j, k) = lo;
-            } else {
-                out(i, j, k) = hi + (lo + inc);
-            }
-            return;
-        }
-    }
-    out(i, j, k) = uo + inc;
-}
-
-// mode: 0 = store F(slot); 1 = fused update from Uo with F1 (s = 1 stores F1)
+// one right-hand side into its slot
 template <typename T, int COMP>
 __global__ void k_rhs(GeoT<T> g, RcpT<T> rc, Fld<T> U, Fld<T> V, Fld<T> W, Fld<T> nt, const DevScal *ds, T nu, T Om, int rot,
-                      Fld<T> out, Fld<T> F1, Fld<T> Uo, Fld<T> Uolo, Fld<T> Unlo, int mode, int s, RkCoef rk,
-                      int i1, int j1, int k1) {
+                      Fld<T> out, int i1, int j1, int k1) {
     int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z + 2;
@@ -475,13 +413,8 @@ __global__ void k_rhs(GeoT<T> g, RcpT<T> rc, Fld<T> U, Fld<T> V, Fld<T> W, Fld<T
     if (COMP == 0) r = rhs_u_point<T, Fld<T>>(g, rc, U, V, W, nt, nu, ds_dpdx<T>(ds), Om, rot, i, j, k);
     else if (COMP == 1) r = rhs_v_point<T, Fld<T>>(g, rc, U, V, W, nt, nu, Om, rot, i, j, k);
     else r = rhs_w_point<T, Fld<T>>(g, rc, U, V, W, nt, nu, ds_dpdz<T>(ds), i, j, k);
-    if (mode == 0) {
-        out(i, j, k) = r;
-        return;
-    }
-    rk_store<T>(r, i, j, k, out, F1, Uo, Uolo, Unlo, s, rk, ds_dt<T>(ds));
+    out(i, j, k) = r;
 }
-
 
 static RkCoef rk_coefs() {
     RkCoef c = {};
@@ -495,44 +428,25 @@ static RkCoef rk_coefs() {
 }
 
 template <typename T>
-static int rhs_launch(cf_ctx *ctx, int comp, int src, int mode, int s, int slot, int dst) {
+static int rhs_launch(cf_ctx *ctx, int comp, int slot) {
     if (int rc = launch_nut_materialize<T>(ctx)) return rc;
-    GeoT<T> g = geo_of<T>(ctx);
-    Fld<T> U = make_fld<T>(ctx->U[src], ctx->nx, ctx->nyg);
-    Fld<T> V = make_fld<T>(ctx->V[src], ctx->nxg, ctx->ny);
-    Fld<T> W = make_fld<T>(ctx->W[src], ctx->nxg, ctx->nyg);
-    Fld<T> nt = make_fld<T>(ctx->nut, ctx->nxg, ctx->nyg);
+    const GeoT<T> g = geo_of<T>(ctx);
+    const int b = ctx->cur;
+    const Fld<T> U = make_fld<T>(ctx->U[b], ctx->nx, ctx->nyg), V = make_fld<T>(ctx->V[b], ctx->nxg, ctx->ny),
+                 W = make_fld<T>(ctx->W[b], ctx->nxg, ctx->nyg), nt = make_fld<T>(ctx->nut, ctx->nxg, ctx->nyg);
     int i1, j1, k1, n1, n2;
-    void *outp, *uo, *uolo = nullptr, *unlo = nullptr;
     if (comp == 0) { i1 = ctx->nx - 1; j1 = ctx->nyg - 1; k1 = ctx->nzg - 1; n1 = ctx->nx; n2 = ctx->nyg; }
     else if (comp == 1) { i1 = ctx->nxg - 1; j1 = ctx->ny - 1; k1 = ctx->nzg - 1; n1 = ctx->nxg; n2 = ctx->ny; }
     else { i1 = ctx->nxg - 1; j1 = ctx->nyg - 1; k1 = ctx->nz - 1; n1 = ctx->nxg; n2 = ctx->nyg; }
-    void **cur = comp == 0 ? ctx->U : comp == 1 ? ctx->V : ctx->W;
-    void **lo = comp == 0 ? ctx->Ulo : comp == 1 ? ctx->Vlo : ctx->Wlo;
-    if (mode == 0) {
-        outp = ctx->F[slot][comp];
-        uo = nullptr;
-    } else {
-        outp = cur[dst];
-        uo = cur[ctx->old];
-        if (lo[ctx->old]) {
-            uolo = lo[ctx->old];
-            if (s == 3) unlo = lo[dst];
-        }
-    }
     // F arrays use the full field extents (interior written)
-    Fld<T> out = make_fld<T>(outp, n1, n2);
-    Fld<T> F1 = make_fld<T>(ctx->F[0][comp], n1, n2);
-    Fld<T> Uo = make_fld<T>(uo, n1, n2);
-    Fld<T> Uolo = make_fld<T>(uolo, n1, n2);
-    Fld<T> Unlo = make_fld<T>(unlo, n1, n2);
-    dim3 blk(32, 4, 1), grd(cdiv(i1 - 1, 32), cdiv(j1 - 1, 4), k1 - 1);
-    T nu = (T)ctx->prm.nu, Om = (T)ctx->omega_z;
+    const Fld<T> out = make_fld<T>(ctx->F[slot][comp], n1, n2);
+    const dim3 blk(32, 4, 1), grd(cdiv(i1 - 1, 32), cdiv(j1 - 1, 4), k1 - 1);
+    const T nu = (T)ctx->prm.nu, Om = (T)ctx->omega_z;
     const int rot = fabs(ctx->omega_z) > 1e-6;  // equations.f90:169, 334
-    RkCoef rk = rk_coefs();
-    if (comp == 0) k_rhs<T, 0><<<grd, blk, 0, ctx->st>>>(g, rcp_of<T>(ctx), U, V, W, nt, ctx->ds, nu, Om, rot, out, F1, Uo, Uolo, Unlo, mode, s, rk, i1, j1, k1);
-    else if (comp == 1) k_rhs<T, 1><<<grd, blk, 0, ctx->st>>>(g, rcp_of<T>(ctx), U, V, W, nt, ctx->ds, nu, Om, rot, out, F1, Uo, Uolo, Unlo, mode, s, rk, i1, j1, k1);
-    else k_rhs<T, 2><<<grd, blk, 0, ctx->st>>>(g, rcp_of<T>(ctx), U, V, W, nt, ctx->ds, nu, Om, rot, out, F1, Uo, Uolo, Unlo, mode, s, rk, i1, j1, k1);
+    const RcpT<T> rc = rcp_of<T>(ctx);
+    if (comp == 0) k_rhs<T, 0><<<grd, blk, 0, ctx->st>>>(g, rc, U, V, W, nt, ctx->ds, nu, Om, rot, out, i1, j1, k1);
+    else if (comp == 1) k_rhs<T, 1><<<grd, blk, 0, ctx->st>>>(g, rc, U, V, W, nt, ctx->ds, nu, Om, rot, out, i1, j1, k1);
+    else k_rhs<T, 2><<<grd, blk, 0, ctx->st>>>(g, rc, U, V, W, nt, ctx->ds, nu, Om, rot, out, i1, j1, k1);
     count_launch(ctx, "k_rhs");
     CF_CUDA(cudaGetLastError());
     return 0;
@@ -553,11 +467,6 @@ struct RingAcc {
     __device__ __forceinline__ T operator()(int i, int j, int k) const {
         return b[k - kc + 1][(j - j0 + 1) * SX + (i - i0 + 1)];
     }
-};
-
-template <typename T>
-struct Trio {
-    Fld<T> u, v, w;
 };
 
 // nu_t held as |S| on canonical cells and the plane coefficient C(j):
@@ -922,7 +831,7 @@ int launch_rhs3(cf_ctx *ctx, int s, int src, int dst) {
     return 0;
 }
 
-// The fused right-hand sides + RK update of substep s of n channels (state
+// The fused right-hand sides + RK update of substep s of n split-path channels (state
 // buffers src[q] -> dst[q]) in one launch: per channel exactly the
 // arithmetic of launch_rhs3.
 template <typename T>
@@ -955,29 +864,31 @@ int launch_rhs3_batch(cudaStream_t st, cf_ctx *const *m, int s, const int *src, 
 }
 
 // resident fused-RHS blocks per SM (for the z-chunk plan)
-int rhs3_blocks_per_sm(int esz) {
+int rhs3_blocks_per_sm() {
     int n = 1;
-    if (esz == 4) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_rhs3<float, 32, 8, 2, true>, 256, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_rhs3<double, 32, 8, 2, false>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_rhs3<float, 32, 8, 2, true>, 256, 0);
     return n < 1 ? 1 : n;
 }
 
 template <typename T>
 int launch_rhs(cf_ctx *ctx, int comp, int slot) {
-    return rhs_launch<T>(ctx, comp, ctx->cur, 0, 0, slot, 0);
+    if constexpr (sizeof(T) == 8) {
+        if (int rc = launch_nut_materialize<double>(ctx)) return rc;
+        return launch_rhs64_comp(ctx, comp, slot);
+    } else {
+        return rhs_launch<T>(ctx, comp, slot);
+    }
 }
 
 template <typename T>
-int launch_rhs3(cf_ctx *ctx, int s, int src, int dst);
-
-template <typename T>
 int launch_rhs_update(cf_ctx *ctx, int s, int src, int dst) {
-    if (ctx->use_rhs3) return launch_rhs3<T>(ctx, s, src, dst);
-    for (int c = 0; c < 3; c++) {
-        int rc = rhs_launch<T>(ctx, c, src, 1, s, 0, dst);
-        if (rc) return rc;
+    if constexpr (sizeof(T) == 8) {
+        if (int rc = launch_rhs64(ctx, ctx->st, s, src, dst)) return rc;
+        count_launch(ctx, "k_rhs64");
+        return 0;
+    } else {
+        return launch_rhs3<T>(ctx, s, src, dst);
     }
-    return 0;
 }
 
 // RK update from stored slots (time_integration.f90:108-146), U = Uo + dt*sum
@@ -988,11 +899,13 @@ __global__ void k_rk_update(Fld<T> U, Fld<T> Uo, Fld<T> F1, Fld<T> F2, Fld<T> F3
     int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
     int k = blockIdx.z + 2;
     if (i > i1 || j > j1 || k > k1) return;
-    double dt = ds->dt, f;
-    if (s == 1) f = dt * rk.c[1][1] * (double)F1(i, j, k);
-    else if (s == 2) f = dt * (rk.c[2][1] * (double)F1(i, j, k) + rk.c[2][2] * (double)F2(i, j, k));
-    else f = dt * (rk.c[3][1] * (double)F1(i, j, k) + rk.c[3][2] * (double)F2(i, j, k) + rk.c[3][3] * (double)F3(i, j, k));
-    U(i, j, k) = (T)((double)Uo(i, j, k) + f);
+    // rk_coef(3,2) = 0 (initialization.f90:416); the order of the fused update
+    const double dt = ds->dt, uo = (double)Uo(i, j, k), f1 = (double)F1(i, j, k);
+    double u;
+    if (s == 1) u = fma(dt * rk.c[1][1], f1, uo);
+    else if (s == 2) u = fma(dt * rk.c[2][1], f1, fma(dt * rk.c[2][2], (double)F2(i, j, k), uo));
+    else u = fma(dt * rk.c[3][1], f1, fma(dt * rk.c[3][3], (double)F3(i, j, k), uo));
+    U(i, j, k) = (T)u;
 }
 
 template <typename T>
@@ -1608,7 +1521,6 @@ int check_bc(cf_ctx *ctx, int b, bool *ok) {
 }
 
 #define INST(T)                                                      \
-    template int launch_rhs3_batch<T>(cudaStream_t, cf_ctx *const *, int, const int *, const int *, int); \
     template int check_bc<T>(cf_ctx *, int, bool *);                 \
     template int launch_bc<T>(cf_ctx *, int, bool);                  \
     template int launch_rhs<T>(cf_ctx *, int, int);                  \
@@ -1622,3 +1534,4 @@ int check_bc(cf_ctx *ctx, int b, bool *ok) {
     template int launch_div_check<T>(cf_ctx *, int, double *);
 INST(double)
 INST(float)
+template int launch_rhs3_batch<float>(cudaStream_t, cf_ctx *const *, int, const int *, const int *, int);

@@ -520,20 +520,33 @@ __global__ void k_fill(T *p, long n, T v) {
     if (t < n) p[t] = v;
 }
 
-// Fills nut from |S| and the plane coefficient when it is held lazily.
+// nu_t on the full extents from |S| and the plane coefficient into dst.
+template <typename T>
+static int launch_nut_field(cf_ctx *ctx, cudaStream_t st, void *dst) {
+    Can c;
+    c.nxp = ctx->nxp; c.nym = ctx->nym; c.nzp = ctx->nzp; c.n = (long)ctx->nCan;
+    k_dsm_f<T><<<dim3(cdiv(ctx->nxg, 32), cdiv(ctx->nyg, 4), ctx->nzg), dim3(32, 4, 1), 0, st>>>(
+        make_fld<T>(dst, ctx->nxg, ctx->nyg), (T *)ctx->dsm_q + Q_S * c.n, ctx->avg_nu_t, c, ctx->nxg, ctx->nyg, ctx->nzg,
+        ctx->prm.Dirichlet_nu_t == 1, 0);
+    count_launch(ctx, "k_dsm_f");
+    CF_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// Fills nut when it is held lazily.
 template <typename T>
 int launch_nut_materialize(cf_ctx *ctx) {
     if (!ctx->nut_lazy) return 0;
-    Can c;
-    c.nxp = ctx->nxp; c.nym = ctx->nym; c.nzp = ctx->nzp; c.n = (long)ctx->nCan;
-    Fld<T> nt = make_fld<T>(ctx->nut, ctx->nxg, ctx->nyg);
-    T *q = (T *)ctx->dsm_q;
-    k_dsm_f<T><<<dim3(cdiv(ctx->nxg, 32), cdiv(ctx->nyg, 4), ctx->nzg), dim3(32, 4, 1), 0, ctx->st>>>(
-        nt, q + Q_S * c.n, ctx->avg_nu_t, c, ctx->nxg, ctx->nyg, ctx->nzg, ctx->prm.Dirichlet_nu_t == 1, 0);
-    count_launch(ctx, "k_dsm_f");
+    if (int rc = launch_nut_field<T>(ctx, ctx->st, ctx->nut)) return rc;
     ctx->nut_lazy = false;
-    CF_CUDA(cudaGetLastError());
     return 0;
+}
+
+// The field the FP64 right-hand side reads: nut, or, held lazily, its own
+// copy (nut itself stays lazy for its other readers).
+int launch_nut_rhs64(cf_ctx *ctx, cudaStream_t st, void **field) {
+    *field = ctx->nut_lazy ? ctx->nut_rhs : ctx->nut;
+    return ctx->nut_lazy ? launch_nut_field<double>(ctx, st, ctx->nut_rhs) : 0;
 }
 
 // nu_t of the wall rows and their neighbours (j = 1, 2, nyg-1, nyg), the

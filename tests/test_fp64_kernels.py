@@ -72,3 +72,42 @@ def test_dsm_segments_and_chunks(dims, wall, kw):
     assert_close(ch.avg_nu_t()[1:-1], o.array("avg_nu_t").ravel()[1:-1], 1e-12, "avg_nu_t")
     ch.close()
     o.close()
+
+
+@pytest.mark.parametrize("dims,les,wall,vary,kw", [((6, 5, 6), 0, 0, True, {}), ((18, 9, 10), 2, 0, False, {}),
+                                                   ((34, 16, 8), 3, 0, True, {}),
+                                                   ((22, 17, 66), 2, 0, False, dict(Rossby_plus=2.0)),
+                                                   ((50, 33, 14), 2, 0, False, {}), ((66, 10, 12), 2, 3, False, {}),
+                                                   ((98, 23, 6), 0, 0, True, dict(Rossby_plus=2.0)),
+                                                   ((18, 10, 130), 3, 0, True, {})])
+def test_rhs_segments_rows_and_chunks(dims, les, wall, vary, kw):
+    """The FP64 fused right-hand side through one whole step: segments of 16
+    and 32 lanes, full and ragged, one and several row tiles with full and
+    partial last tiles, one and several chunks, with rotation, with and
+    without eddy viscosity and wall model.  vary: x and z spacings that
+    change from cell to cell, where the reference's upper- and lower-face
+    formulas differ (not with the dynamic model, whose plane sums the library
+    takes with the duplicate column as a copy, which it is on uniform x and z
+    only).  U, V, W after the step within the per-routine 1e-12."""
+    nx, ny, nz = dims
+    case = channel_case(*dims, les=les, wall=wall, stretch=0.0 if wall else 1.5, retau=2000.0 if wall else 180.0,
+                        profile="plug" if wall else "laminar", jref=2, ncv=30)
+    if vary:
+        for c, n in (("x", nx), ("z", nz)):
+            d = np.diff(case[c])
+            d *= 1.0 + 0.2 * np.cos(2 * np.pi * np.arange(n - 1) / (n - 2))  # periodic over the n - 2 cells
+            case[c] = np.concatenate([[0.0], np.cumsum(d)])
+    case["prm"].update(kw)
+    o, ch = pair(case)
+    for d in (o, ch):
+        d.init_mass_flow()
+        d.apply_boundary_conditions()
+    o.compute_dt()
+    o.time_step_rk3()
+    ch.time_step_rk3(1)
+    g, f = ch.download(), o.fields()
+    for n in ("U", "V", "W"):
+        assert_close(g[n], f[n], 1e-12, n)
+    ch.close()
+    o.close()
+
