@@ -8,10 +8,9 @@
 #include "cf_internal.cuh"
 
 int fft_setup_attrs();
-int dsm_fused_setup();
 int dsm_b_setup();
+int dsm32_setup();
 int dsm_b_plan(int nxp, int nym, int nzp, int sms);
-int dsm_fused_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
 
 static thread_local std::string g_last_error;  // failures without a context
 
@@ -490,23 +489,22 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
     ctx->esz = p->precision == CF_PREC_SPLIT ? 4 : 8;
     if (ctx->esz == 8) { TRY(alloc_all<double>(ctx)); TRY(upload_twiddles<double>(ctx)); }
     else { TRY(alloc_all<float>(ctx)); TRY(upload_twiddles<float>(ctx)); }
-    ctx->dsm_nblk = std::max(1, std::min(64, (int)((long)nxp * nzp / 2048)));
-    size_t nch_fused = 0;
+    size_t nch_dsm = 0;
     int amd_parts = 0;
     {
-        // fused pass: column tiles marching in z; chunks sized for one wave
         int dev_sms = 152;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
-        dsm_fused_setup();
         dsm_b_setup();
+        dsm32_setup();
+        // eddy viscosity: chunks of planes; room for the partials of any chunk length
         if (ctx->esz == 4) {
-            dsm_fused_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_fused);
+            dsm32_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_dsm);
+            nch_dsm = (size_t)dsm32_slots(nxp, nzp, 1);
             ctx->dsmb_nkc = dsm_b_plan(nxp, ctx->nym, nzp, dev_sms);
         } else {
-            dsm64_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_fused);
-            nch_fused = (size_t)dsm64_slots(nxp, nzp, 1);  // any chunk length
+            dsm64_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_dsm);
+            nch_dsm = (size_t)dsm64_slots(nxp, nzp, 1);
         }
-        ctx->use_fused_dsm = !p->dsm_unfused;
         if (ctx->esz == 8) {
             ctx->rhs_nkc = rhs64_plan(nxp, ctx->nym, nzp, dev_sms);
         } else {
@@ -526,9 +524,7 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
         }
         if (p->LES_model == 3) amd_plan(p->precision == CF_PREC_SPLIT ? 4 : 8, nxp, ctx->nym, nzp, dev_sms, &ctx->amd_nkc, &amd_parts);
     }
-    // (with the wall model the one-pass kernel's slots are followed by the seam band's)
-    size_t nch = std::max({(size_t)ctx->dsm_nblk, nch_fused + (ctx->esz == 4 && p->iwall_model == 3 ? dsm_seam_slots_max() : 0),
-                           (size_t)cdiv(amd_parts, 2), (size_t)cdiv(nxp, 32) * (size_t)ctx->dsmb_nkc});
+    const size_t nch = std::max({nch_dsm, (size_t)cdiv(amd_parts, 2), (size_t)cdiv(nxp, 32) * (size_t)ctx->dsmb_nkc});
     CF_CUDA(cudaMalloc(&ctx->dsm_part, (size_t)2 * ctx->nym * nch * sizeof(double)));
     ctx->dsm_part_nch = nch;
     // avg_nu_t (1..nyg) in FP64, followed by an FP32 copy
@@ -569,7 +565,6 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
     TRY(push_scal(ctx));
     TRY(setup_eqwm(ctx));
     fft_setup_attrs();
-    dsm_fused_setup();
     CF_CUDA(cudaStreamSynchronize(ctx->st));
     CF_CUDA(cudaGetLastError());
     return CF_OK;
@@ -681,11 +676,7 @@ extern "C" int cf_upload_fields(cf_ctx *ctx, const double *U, const double *V, c
     TRY(put(ctx, ctx->V[b], ctx->Vlo[b], V, ctx->nV));
     TRY(put(ctx, ctx->W[b], ctx->Wlo[b], W, ctx->nW));
     ctx->old = ctx->cur;
-    // do the ghosts already hold what apply_boundary_conditions would put
-    // there? (checked on the device copy; synchronises the stream)
-    bool ok = false;
-    TRY(DISPATCH(check_bc<double>(ctx, b, &ok), check_bc<float>(ctx, b, &ok)));
-    ctx->state_periodic = ok;
+    CF_CUDA(cudaStreamSynchronize(ctx->st));  // the host arrays may be reused
     return CF_OK;
 }
 
@@ -1151,26 +1142,20 @@ static int step_seg(cf_ctx *ctx, int seg, bool tri) {
 static int step_eager(cf_ctx *ctx) { return DISPATCH(enqueue_step<double>(ctx), enqueue_step<float>(ctx)); }
 
 // ---------------------------------------------------------------------------
-// The same step cut for an ensemble whose fused dynamic Smagorinsky passes
-// and fused right-hand sides run as one launch over all members.  Per
+// The same step cut for an ensemble whose fused right-hand sides run as one
+// launch over all split-path members.  Per
 // substep s, with buffers as in enqueue_seg (X the starting state,
 // a = X+1, b = X+2 mod 3):
 //   pre(s):  s = 1: dt; s > 1: inverse transforms of substep s-1's
-//            projection and the boundary conditions; the eddy viscosity of a
-//            member that does not take the batched pass (and at s = 1 the
-//            wall model)
-//   [batched fused DSM pass of the members that take it -- twice at s = 1
-//    when sgs_recompute -- and batched fused right-hand sides + RK update]
+//            projection and the boundary conditions; the eddy viscosity
+//            (and at s = 1 the wall model)
+//   [batched fused right-hand sides + RK update]
 //   post(s): forward transforms of substep s's projection (with the
 //            member's own tridiagonal solve unless the ensemble solves them)
 //   fin:     inverse transforms of substep 3's projection, boundary
 //            conditions, mass-flow forcing.
 // Each member's launches are those of enqueue_seg in the same order.
 // ---------------------------------------------------------------------------
-static bool dsm_batchable(const cf_ctx *c) {
-    return c->esz == 4 && c->prm.LES_model == 2 && c->use_fused_dsm && c->prm.iwall_model == 0 && c->state_periodic;
-}
-
 static void ens_bufs(const cf_ctx *c, int s, int *src, int *dst) {
     const int X = c->seg_base, a = (X + 1) % 3, b = (X + 2) % 3;
     *src = s == 1 ? X : (s == 2 ? a : b);
@@ -1178,29 +1163,22 @@ static void ens_bufs(const cf_ctx *c, int s, int *src, int *dst) {
 }
 
 template <typename T>
-static int ens_pre_t(cf_ctx *ctx, int s, bool batched_dsm) {
+static int ens_pre_t(cf_ctx *ctx, int s) {
     const bool canon = true;
     if (s == 1) {
         const int X = ctx->cur;
         ctx->seg_base = X;
         ctx->old = X;
         TRY(launch_dt<T>(ctx, X, true));
-        if (!batched_dsm) {
-            TRY(eddy(ctx, X));
-            if (ctx->prm.iwall_model == 3) {
-                TRY(wall_model(ctx, X));
-                if (ctx->prm.sgs_recompute) TRY(eddy(ctx, X));
-            } else if (ctx->prm.sgs_recompute) {
-                TRY(eddy(ctx, X));
-            }
-        }
+        TRY(eddy(ctx, X));
+        if (ctx->prm.iwall_model == 3) TRY(wall_model(ctx, X));
+        if (ctx->prm.sgs_recompute) TRY(eddy(ctx, X));
         return 0;
     }
     const int X = ctx->seg_base, a = (X + 1) % 3, b = (X + 2) % 3;
     const int p = s == 2 ? a : b;  // the state the previous substep's projection acts on
     TRY(launch_projection<T>(ctx, p, s == 2, false, canon, POISSON_INV, true));
-    if (!batched_dsm) TRY(eddy(ctx, p));
-    return 0;
+    return eddy(ctx, p);
 }
 
 template <typename T>
@@ -1228,7 +1206,7 @@ static int ens_fin_t(cf_ctx *ctx) {
     return 0;
 }
 
-static int ens_pre(cf_ctx *ctx, int s, bool bd) { return DISPATCH(ens_pre_t<double>(ctx, s, bd), ens_pre_t<float>(ctx, s, bd)); }
+static int ens_pre(cf_ctx *ctx, int s) { return DISPATCH(ens_pre_t<double>(ctx, s), ens_pre_t<float>(ctx, s)); }
 static int ens_post(cf_ctx *ctx, int s, bool tri) { return DISPATCH(ens_post_t<double>(ctx, s, tri), ens_post_t<float>(ctx, s, tri)); }
 static int ens_fin(cf_ctx *ctx) { return DISPATCH(ens_fin_t<double>(ctx), ens_fin_t<float>(ctx)); }
 
@@ -1237,14 +1215,6 @@ extern "C" int cf_time_step_rk3(cf_ctx *ctx, int nsteps, int sync) {
     CF_CUDA(cudaSetDevice(ctx->dev));
     for (int s = 0; s < nsteps; s++) {
         int X = ctx->cur;
-        if (!ctx->state_periodic) {
-            // ghosts not yet filled by apply_boundary_conditions: run this
-            // step without a graph (its first eddy viscosity takes the
-            // multi-pass route), later steps are captured
-            int rc = step_eager(ctx);
-            if (rc) return rc;
-            continue;
-        }
         if (!ctx->graphs[X]) {
             // first step from this buffer: count launches eagerly-captured
             cudaGraph_t g = nullptr;
@@ -1622,37 +1592,20 @@ static int capture_batched_step(cf_ensemble *e, int *extra) {
         }
         return !rc && ce == cudaSuccess;
     };
-    std::vector<char> bd(n);
-    for (int q = 0; q < n; q++) bd[q] = dsm_batchable(e->m[q]);
     for (int s = 1; s <= 3; s++) {
-        if (!branches([&](int q, cf_ctx *c) { return ens_pre(c, s, bd[q] != 0); })) break;
+        if (!branches([&](int, cf_ctx *c) { return ens_pre(c, s); })) break;
         // batched passes, per precision
         for (int esz : {4, 8}) {
-            std::vector<cf_ctx *> dm, dm2, rm;
-            std::vector<int> db, db2, rs, rd;
+            std::vector<cf_ctx *> rm;
+            std::vector<int> rs, rd;
             for (int q = 0; q < n; q++) {
                 cf_ctx *c = e->m[q];
                 if (c->esz != esz) continue;
                 int src, dst;
                 ens_bufs(c, s, &src, &dst);
-                if (bd[q]) {
-                    dm.push_back(c);
-                    db.push_back(src);
-                    if (s == 1 && c->prm.sgs_recompute) {
-                        dm2.push_back(c);
-                        db2.push_back(src);
-                    }
-                }
                 rm.push_back(c);
                 rs.push_back(src);
                 rd.push_back(dst);
-            }
-            for (int pass = 0; pass < 2 && !rc; pass++) {
-                std::vector<cf_ctx *> &mm = pass ? dm2 : dm;
-                std::vector<int> &bb = pass ? db2 : db;
-                if (mm.empty()) continue;
-                rc = launch_dsm_batch<float>(e->st, mm.data(), bb.data(), (int)mm.size());
-                *extra += 2;
             }
             if (!rc && !rm.empty()) {
                 if (esz == 4) {
@@ -1700,22 +1653,6 @@ extern "C" int cf_ensemble_step(cf_ensemble *e, int nsteps, int sync) {
     ENS_CUDA(cudaSetDevice(e->dev));
     const int n = (int)e->m.size();
     for (int s = 0; s < nsteps; s++) {
-        // members whose ghosts are not yet filled take their first step alone
-        // (as cf_time_step_rk3 does), ordered after the ensemble's work
-        bool eager = false;
-        for (cf_ctx *c : e->m)
-            if (!c->state_periodic) eager = true;
-        if (eager) {
-            ENS_CUDA(cudaEventRecord(e->fork, e->st));
-            for (int q = 0; q < n; q++) {
-                cf_ctx *c = e->m[q];
-                ENS_CUDA(cudaStreamWaitEvent(c->st, e->fork, 0));
-                if (int rc = cf_time_step_rk3(c, 1, 0)) return ens_fail(e, rc, "member step: " + c->err);
-                ENS_CUDA(cudaEventRecord(e->join[q], c->st));
-                ENS_CUDA(cudaStreamWaitEvent(e->st, e->join[q], 0));
-            }
-            continue;
-        }
         std::vector<int> key(n);
         for (int q = 0; q < n; q++) key[q] = e->m[q]->cur;
         auto it = e->graphs.find(key);
@@ -1795,21 +1732,18 @@ extern "C" int cf_ensemble_autotune(cf_ensemble *e, int steps, double *report, i
     if (!e || steps < 1) return ens_fail(e, CF_ERR_INVALID, "cf_ensemble_autotune: bad argument");
     ENS_CUDA(cudaSetDevice(e->dev));
     const int n = (int)e->m.size();
-    std::vector<int> kc0(n), nkc0(n);
+    std::vector<int> nkc0(n);
     for (int q = 0; q < n; q++) {
-        kc0[q] = e->m[q]->dsm_kc;
         nkc0[q] = e->m[q]->rhs_nkc;
     }
     auto apply = [&](int cand) {
         for (int q = 0; q < n; q++) {
             cf_ctx *c = e->m[q];
-            const int lo_rhs = cdiv(c->nzp, RHS_ZMAX_HOST), lo_dsm = cdiv(c->nzp, DSM_ZMAX_HOST);
+            const int lo_rhs = cdiv(c->nzp, RHS_ZMAX_HOST);
             if ((cand & 3) <= 1) {
-                c->dsm_kc = kc0[q];
                 c->rhs_nkc = nkc0[q];
             } else {
                 const int parts = (cand & 3) == 2 ? 1 : 2;
-                c->dsm_kc = cdiv(c->nzp, std::max(parts, lo_dsm));
                 c->rhs_nkc = std::max(parts, lo_rhs);
             }
             for (auto &g : c->graphs)
@@ -1908,16 +1842,13 @@ static int tune_t(cf_ctx *ctx, int reps, double *rep) {
         rep[1] = best;
     }
     // the eddy-viscosity pass
-    if (!rc && ctx->prm.LES_model == 2 && ctx->use_fused_dsm && ctx->state_periodic &&
-        (ctx->prm.iwall_model == 0 || ctx->prm.iwall_model == 3)) {
+    if (!rc && ctx->prm.LES_model == 2 && (sizeof(T) == 8 || !ctx->prm.dsm_unfused)) {
         const int keep = ctx->dsm_kc;
-        const size_t nseam = sizeof(T) == 4 && ctx->prm.iwall_model == 3 ? (size_t)dsm_seam_slots_max() : 0;
         double best = 1e300;
         int best_kc = keep, last_len = -1;
-        for (int nn = cdiv(nzp, DSM_ZMAX_HOST); nn <= std::max(1, nzp / 4) && !rc; nn++) {
+        for (int nn = 1; nn <= std::max(1, nzp / 4) && !rc; nn++) {
             const int len = cdiv(nzp, nn);
-            const size_t slots = sizeof(T) == 4 ? (size_t)cdiv(ctx->nxp, 32) * cdiv(nzp, len) : (size_t)dsm64_slots(ctx->nxp, nzp, len);
-            if (len == last_len || slots + nseam > ctx->dsm_part_nch) continue;
+            if (len == last_len) continue;
             last_len = len;
             ctx->dsm_kc = len;
             double us = 0;

@@ -128,22 +128,6 @@ __host__ __device__ __forceinline__ int wrapc(int i, int np) {
 
 static inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
-// The seam band of the wall-model configurations.  With the equilibrium wall
-// model the wall ghost rows of U and W (j = 1, nyg) are not periodic copies at
-// the seam columns and planes (their Neumann values use alpha at the ghost's
-// own position).  The reference reads those entries themselves in the
-// stencils of the canonical centres next to a seam and the canonical twin's
-// values where it fills ghost points (subgrid.f90:448-458), while this pass
-// reads every halo through the periodic wrap.  A centre's L.M, M.M and |S|
-// read U, V, W within two cells of it (through its neighbours' quantities and
-// the filtered velocities), so the centres that can see a wall ghost entry
-// outside the canonical columns and planes -- rows 2, 3, nyg-2, nyg-1 at
-// columns 2, 3, nxp, nxp+1 or planes 2, 3, nzp, nzp+1 -- are computed by
-// k_dsm_seam with the reference's readings.
-__host__ __device__ __forceinline__ bool seam_row(int j, int nyg) { return j <= 3 || j >= nyg - 2; }
-__host__ __device__ __forceinline__ bool seam_line(int i, int np) { return i <= 3 || i >= np; }
-
-
 // compute_Sij at one centre (subgrid.f90:891-949) from arrays at actual
 // indices (any accessor with operator()(i, j, k)); the spacing quotients are
 // products with the stored reciprocal spacings rc (27 divisions a centre
@@ -217,14 +201,10 @@ struct cf_ctx {
     void *F[3][3] = {};                // [slot 0..2][comp]
     // eddy viscosity
     void *dsm_q = nullptr;             // 16 canonical arrays
-    void *Uf = nullptr, *Vf = nullptr, *Wf = nullptr;
+    void *Uf = nullptr, *Vf = nullptr, *Wf = nullptr;  // filtered velocities (layout of the pass that wrote them)
     double *dsm_part = nullptr;        // plane partial sums
     double *avg_nu_t = nullptr;        // (nyg) device
-    int dsm_nblk = 0;
-    int dsm_kc = 0;                    // z-chunk length of the fused pass (FP32) or of the FP64 pass
-    int dsm_nchunk_fused = 0;          // plane-partial slots per row of the last one-pass launch
-    int dsm_nchunk_base = 0;           // of them, the one-pass kernel's (the seam band's follow)
-    bool use_fused_dsm = true;
+    int dsm_kc = 0;                    // z-chunk length of the eddy-viscosity pass
     int dsmb_nkc = 0;                  // z chunks of the multi-pass DSM filter kernel
     // tensor map (a CUtensorMap) of the 15 filter quantities of dsm_q for the
     // filter kernel's tensor-copy gather; state 0 not tried, 1 encoded, -1 not
@@ -239,11 +219,7 @@ struct cf_ctx {
     size_t dsm_part_nch = 0;           // plane-partial slots per row allocated in dsm_part
     int amd_nparts = 0;                // partial sums per row of the last AMD pass
     bool amd_avg_pending = false;      // avg_nu_t not yet formed from them
-    // U, V, W hold the ghosts apply_boundary_conditions gives them: periodic
-    // copies in x and z (with the wall model: except the wall ghost rows of U
-    // and W at the seams) and the wall rule
-    bool state_periodic = false;
-    // After the one-pass eddy viscosity, nu_t is held as |S| (canonical) and
+    // After the eddy viscosity, nu_t is held as |S| (canonical) and
     // the plane coefficient <LM>/<MM>: the fused RHS forms nu_t on the fly and
     // the nut buffer is filled only when another reader needs it.
     bool nut_lazy = false;
@@ -305,7 +281,6 @@ int cf_fail(cf_ctx *ctx, int code, const std::string &msg);
 
 // ---- launchers (kernels in the .cu files), all enqueue on ctx->st -------
 template <typename T> int launch_bc(cf_ctx *ctx, int buf, bool lo = true);  // apply_boundary_conditions (lo: low words too)
-template <typename T> int check_bc(cf_ctx *ctx, int buf, bool *ok);      // ghosts already as the BCs leave them?
 template <typename T> int launch_rhs(cf_ctx *ctx, int comp, int slot);     // store F slot
 int rhs3_blocks_per_sm();
 int rhs64_plan(int nxp, int nym, int nzp, int sms);                        // z chunks of the FP64 right-hand side
@@ -314,15 +289,13 @@ int launch_rhs64_comp(cf_ctx *ctx, int comp, int slot);                     // o
 template <typename T> int launch_rhs_update(cf_ctx *ctx, int s, int src, int dst);  // fused RHS + RK update
 template <typename T> int launch_rk_update(cf_ctx *ctx, int s);            // from stored F slots
 template <typename T> int launch_dsm(cf_ctx *ctx, int buf);                // eddy viscosity
-template <typename T> int launch_dsm_fused(cf_ctx *ctx, int buf);          // FP32 fused pass (periodic state)
-template <typename T> int launch_dsm_fused_wm(cf_ctx *ctx, int buf);       // FP32 fused pass + seam band (wall model)
+int launch_dsm32(cf_ctx *ctx, int buf, int *nchunk);                       // FP32 pass: |S| and the plane partials
+void dsm32_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
+int dsm32_slots(int nxp, int nzp, int kc);                                 // its partials per row with chunks of kc planes
 int launch_dsm64(cf_ctx *ctx, int buf, int *nchunk);                       // FP64 pass: |S| and the plane partials
 void dsm64_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
 int dsm64_slots(int nxp, int nzp, int kc);                                 // its partials per row with chunks of kc planes
-int dsm_seam_slots_max();                                                  // partial slots the seam band may take
 constexpr int CF_ENS_MAXM = 32;  // channels per batched ensemble launch at most
-// fused pass + <LM>/<MM> rows of n channels in two launches (ensembles)
-template <typename T> int launch_dsm_batch(cudaStream_t st, cf_ctx *const *m, const int *buf, int n);
 // fused right-hand sides + RK update of substep s of n split-path channels in one launch
 template <typename T> int launch_rhs3_batch(cudaStream_t st, cf_ctx *const *m, int s, const int *src, const int *dst, int n);
 template <typename T> int launch_nut_zero(cf_ctx *ctx);
@@ -357,7 +330,6 @@ template <typename T> int launch_amd(cf_ctx *ctx, int buf);  // AMD eddy viscosi
 void amd_plan(int esz, int nxp, int nym, int nzp, int sms, int *nkc, int *nparts);  // z chunks of the AMD pass
 int launch_avg_nu_t_flush(cf_ctx *ctx);  // AMD plane means of the last pass, if not formed yet
 int amd_partials_for(cf_ctx *ctx, int nkc);  // plane partials per row of an AMD pass with nkc z chunks
-constexpr int DSM_ZMAX_HOST = 256;           // planes per z chunk of the fused DSM pass at most
 constexpr int RHS_ZMAX_HOST = 256;           // planes per z chunk of the fused RHS at most
 template <typename T> int launch_div_check(cf_ctx *ctx, int buf, double *d_out);
 template <typename T> int launch_mass_flow(cf_ctx *ctx, int buf, int mode, bool ghosts = false);  // 1: x mass flow, 2: centre-line, 3: y

@@ -1,7 +1,7 @@
 // k_dsm.cu -- dynamic Smagorinsky eddy viscosity, subgrid.f90:376-538: the
-// multi-pass kernels of the FP32 path (a state whose ghosts are not yet
-// filled), the plane coefficients and nu_t from them; the other passes are
-// in k_dsm_fused.cu (FP32) and k_dsm64.cu (FP64).
+// multi-pass kernels of the FP32 path (cf_params.dsm_unfused, the
+// cross-check), the plane coefficients and nu_t from them.  The passes a step
+// takes are in k_dsm32.cu (split path) and k_dsm64.cu (FP64).
 //
 // Quantities the reference keeps only as periodic copies are computed at the
 // canonical cells (i = 2..nx-1, j = 2..nyg-1, k = 2..nz-1) and read through
@@ -425,16 +425,12 @@ __global__ void __launch_bounds__(256) k_dsm_c_t(Fld<T> A, Fld<T> Af, int n1, in
 // Stage E: avg_nu_t(j) = <LM>/<MM> (subgrid.f90:516-518) and its ghosts.
 // <LM>/<MM> per row from the block partial sums: one warp per row, lanes
 // over chunks in a fixed order, then the ghost rows (subgrid.f90:515-519).
-// nbase: the slots of a row outside the wall-model seam band (the seam
-// kernel's slots follow them only in the band's rows; nbase = nchunk when
-// there are none)
-__global__ void k_dsm_e(const double *part, int nchunk, int nyg, double *avg, int dirichlet, int nbase) {
+__global__ void k_dsm_e(const double *part, int nchunk, int nyg, double *avg, int dirichlet) {
     const int lane = threadIdx.x & 31;
     const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) + 2;
     if (j > nyg - 1) return;
-    const int nread = seam_row(j, nyg) ? nchunk : nbase;
     double a = 0.0, b = 0.0;
-    for (int q = lane; q < nread; q += 32) {
+    for (int q = lane; q < nchunk; q += 32) {
         a += part[((long)(j - 2) * nchunk + q) * 2];
         b += part[((long)(j - 2) * nchunk + q) * 2 + 1];
     }
@@ -457,15 +453,14 @@ __global__ void k_dsm_e(const double *part, int nchunk, int nyg, double *avg, in
         }
     }
 }
-// The same from float-float partials (L.M hi, lo, M.M hi, lo) of the one-pass
-// FP32 kernel: the sums in float-float, FP64 only for lane 0's quotient.
-__global__ void k_dsm_e_ff(const float4 *part, int nchunk, int nyg, double *avg, int dirichlet, int nbase) {
+// The same from float-float partials (L.M hi, lo, M.M hi, lo) of the FP32
+// kernels: the sums in float-float, FP64 only for lane 0's quotient.
+__global__ void k_dsm_e_ff(const float4 *part, int nchunk, int nyg, double *avg, int dirichlet) {
     const int lane = threadIdx.x & 31;
     const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) + 2;
     if (j > nyg - 1) return;
-    const int nread = seam_row(j, nyg) ? nchunk : nbase;
     float ah = 0.f, al = 0.f, bh = 0.f, bl = 0.f;
-    for (int q = lane; q < nread; q += 32) {
+    for (int q = lane; q < nchunk; q += 32) {
         const float4 v = part[(long)(j - 2) * nchunk + q];
         ff_add2(ah, al, v.x, v.y);
         ff_add2(bh, bl, v.z, v.w);
@@ -622,18 +617,17 @@ bool dsmb_tma(cf_ctx *ctx) {
     return ctx->dsmb_map_state == 1 && ctx->prm.dsm_unfused != 2;
 }
 
-// The plane coefficients <LM>/<MM> from nch partials per row (of them nbase
-// outside the seam band's rows): float-float ones of the FP32 kernels, FP64
-// ones of the FP64 pass.  nu_t = max(-C(j)|S|/2, 0) (stage F) is left to its
+// The plane coefficients <LM>/<MM> from nch partials per row: float-float
+// ones of the FP32 kernels, FP64 ones of the FP64 pass.  nu_t = max(-C(j)|S|/2, 0) (stage F) is left to its
 // readers: the fused RHS forms it in its loader, the others (eqwm, statistics,
 // downloads) materialise it first.
-static int launch_dsm_e(cf_ctx *ctx, int nch, int nbase) {
+static int launch_dsm_e(cf_ctx *ctx, int nch) {
     const int dir = ctx->prm.Dirichlet_nu_t == 1;
     if (ctx->esz == 4)
         k_dsm_e_ff<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>((const float4 *)ctx->dsm_part, nch, ctx->nyg, ctx->avg_nu_t,
-                                                            dir, nbase);
+                                                            dir);
     else
-        k_dsm_e<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>(ctx->dsm_part, nch, ctx->nyg, ctx->avg_nu_t, dir, nbase);
+        k_dsm_e<<<cdiv(ctx->nym, 8), 256, 0, ctx->st>>>(ctx->dsm_part, nch, ctx->nyg, ctx->avg_nu_t, dir);
     count_launch(ctx, "k_dsm_e");
     ctx->nut_lazy = true;
     CF_CUDA(cudaGetLastError());
@@ -646,20 +640,19 @@ template <>
 int launch_dsm<double>(cf_ctx *ctx, int b) {
     int nch;
     if (int rc = launch_dsm64(ctx, b, &nch)) return rc;
-    return launch_dsm_e(ctx, nch, nch);
+    return launch_dsm_e(ctx, nch);
 }
 
 template <>
 int launch_dsm<float>(cf_ctx *ctx, int b) {
     Can c;
     c.nxp = ctx->nxp; c.nym = ctx->nym; c.nzp = ctx->nzp; c.n = (long)ctx->nCan;
-    if (ctx->use_fused_dsm && ctx->state_periodic && (ctx->prm.iwall_model == 0 || ctx->prm.iwall_model == 3)) {
-        // one pass: |S| and the plane partial sums (k_dsm_fused.cu); with the
-        // wall model the seam band is computed by k_dsm_seam
-        int rc = ctx->prm.iwall_model == 0 ? launch_dsm_fused<float>(ctx, b) : launch_dsm_fused_wm<float>(ctx, b);
-        if (rc) return rc;
-        return launch_dsm_e(ctx, ctx->dsm_nchunk_fused, ctx->dsm_nchunk_base);
+    if (!ctx->prm.dsm_unfused) {
+        int nch;
+        if (int rc = launch_dsm32(ctx, b, &nch)) return rc;
+        return launch_dsm_e(ctx, nch);
     }
+    // dsm_unfused: the multi-pass kernels (the cross-check)
     GeoT<float> g = geo_of<float>(ctx);
     Fld<float> U = make_fld<float>(ctx->U[b], ctx->nx, ctx->nyg);
     Fld<float> V = make_fld<float>(ctx->V[b], ctx->nxg, ctx->ny);
@@ -699,7 +692,7 @@ int launch_dsm<float>(cf_ctx *ctx, int b) {
                                                                            ctx->dsm_part, nchunk, ctx->ds, 0);
     }
     count_launch(ctx, "k_dsm_b");
-    return launch_dsm_e(ctx, nchunk, nchunk);
+    return launch_dsm_e(ctx, nchunk);
 }
 
 template int launch_nut_zero<double>(cf_ctx *);

@@ -1883,8 +1883,7 @@ int launch_projection(cf_ctx *ctx, int b, bool store_p, bool lo, bool canon, int
             else k_project3<T, false, false><<<grd, blk, 0, ctx->st>>>(pa);
         }
         count_launch(ctx, "k_project3");
-        if (img) ctx->state_periodic = true;  // as launch_bc: holds for every later launch on the stream
-        else if (bc) {
+        if (bc && !img) {
             if (int rc = launch_bc<T>(ctx, b, lo)) return rc;
         }
     }

@@ -1,0 +1,55 @@
+"""Split-path kernels at the sizes where their tilings, chunks and tails end,
+against the FP64 path on the same inputs."""
+import numpy as np
+import pytest
+
+from conftest import channel_case, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def run_pair(case, calls, **extra):
+    """The same calls on an FP64 and a split-path channel; both channels."""
+    import channelflow as cf
+    out = []
+    for prec in (cf.PREC_FP64, cf.PREC_SPLIT):
+        kw = dict(case["prm"])
+        kw.update(extra)
+        ch = cf.Channel(case["x"], case["y"], case["z"], precision=prec, **kw)
+        ch.upload(case["U"], case["V"], case["W"])
+        calls(ch)
+        out.append(ch)
+    return out
+
+
+@pytest.mark.parametrize("dims,wall,dirichlet", [((6, 5, 6), 0, 0), ((18, 6, 8), 0, 0), ((20, 9, 34), 0, 1),
+                                                 ((34, 17, 12), 0, 0), ((50, 7, 18), 0, 0), ((66, 12, 20), 0, 0),
+                                                 ((98, 14, 10), 0, 0), ((130, 10, 8), 0, 1), ((102, 13, 38), 0, 0),
+                                                 ((18, 17, 18), 3, 0), ((34, 8, 22), 3, 0), ((130, 11, 10), 3, 0)])
+def test_dsm_segments_and_chunks(dims, wall, dirichlet):
+    """The FP32 dynamic Smagorinsky pass with segments of 16, 32 and 64
+    columns, full and ragged, several rows to a warp, chunks of one plane and
+    more, ghosts unfilled at the first call; with the wall model after an eqwm
+    boundary update.  The velocities (up to 1.5) are rounded to FP32 and the
+    strain rates are differences of neighbours of order 0.1: relative errors of
+    1e-6 per difference; C(j) and nu_t are held to the 2e-4 the split path's
+    eddy viscosity is held to elsewhere."""
+    if wall:
+        case = channel_case(*dims, stretch=0.0, wall=3, retau=2000.0, profile="plug", jref=2, ncv=30)
+    else:
+        case = channel_case(*dims)
+    case["prm"]["Dirichlet_nu_t"] = dirichlet
+
+    def calls(ch):
+        ch.apply_boundary_conditions()
+        ch.compute_eddy_viscosity()
+        if wall:
+            ch.compute_wall_model()
+            ch.apply_boundary_conditions()
+            ch.compute_eddy_viscosity()
+
+    a, b = run_pair(case, calls)
+    assert rel_err(b.avg_nu_t()[1:-1], a.avg_nu_t()[1:-1]) <= 2e-4
+    assert rel_err(b.download()["nu_t"], a.download()["nu_t"]) <= 2e-4
+    a.close()
+    b.close()
