@@ -10,6 +10,7 @@
 int fft_setup_attrs();
 int dsm_b_setup();
 int dsm32_setup();
+int eqwm_setup();
 int dsm_b_plan(int nxp, int nym, int nzp, int sms);
 
 static thread_local std::string g_last_error;  // failures without a context
@@ -496,6 +497,7 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
         dsm_b_setup();
         dsm32_setup();
+        eqwm_setup();
         // eddy viscosity: chunks of planes; room for the partials of any chunk length
         if (ctx->esz == 4) {
             dsm32_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_dsm);

@@ -4,12 +4,8 @@
 // W at the matching row is moved to the U location with the 3-point Lagrange
 // interpolations of interpolation.f90:114-252; their stencil choice depends
 // only on indices, so the host precomputes (jj, w0, w1, w2) per output index
-// with the reference's formulas.  One thread solves the ODE of one wall
-// point: Picard iteration on tau_w (<= 101 passes, tol 1e-7), each pass a
-// tridiagonal solve over the ncv cells.  The solve eliminates from the top
-// (the Dirichlet row, x_ncv = |u|) down to the wall row, so x_1 -- the only
-// unknown the stress needs (eqwm.f90:198) -- comes out of one register
-// recurrence without storing the Thomas coefficients of eqwm.f90:52-88.
+// with the reference's formulas.  The ODE of a wall point is solved by Picard
+// iteration on tau_w (<= 101 passes, tol 1e-7; k_eq_solve below).
 #include "cf_internal.cuh"
 
 // temp_1 = interpolate_z_2nd of W(:, jw, :) at both walls: (nxg, 2, nzg)
@@ -30,7 +26,6 @@ __global__ void k_eq_zinterp_t(Fld<T> W, int jref, int nxg, int nyg, int nzg, co
 struct EqParams {
     int ncv, jref, nx, nxg, nyg, nzg;
     double nu, h_wm, tau_mean;
-    int mixed;  // split path: FP32 Picard passes before the FP64 ones
 };
 
 // |u| at the matching row of wall point t = (i, wall, k) (wallmodel.f90:
@@ -86,252 +81,278 @@ struct WmState {
     double *tau_eq;
 };
 
-// Largest ncv for which the split path keeps each point's exponentials of
-// the last FP64 pass in shared memory (128 threads x (ncv-1) doubles: 45 KB).
-constexpr int EQ_EXP_NCV = 45;
-// offset (in doubles) of the kept exponentials: past the grid arrays
-__host__ __device__ __forceinline__ int eq_exp_off(int ncv) {
-    return (2 * ncv + 3) + ((2 * ncv + 4) * (int)sizeof(float) + 7) / 8;
-}
+// ---------------------------------------------------------------------------
+// solve_u_eqwm (eqwm.f90:90-223) for every wall point.
+//
+// The ODE's tridiagonal system (eqwm.f90:152-205) says that the flux
+// mu (u_{q+1} - u_q) / (y_cv(q+1) - y_cv(q)) is the same through every face
+// between the wall and the top cell, whose velocity is given, so the stress
+// of a pass is that of resistances in series,
+//   tau = u_les / sum_q g_q / mu_q,
+// g_0 = y_cv(1) - y_fa(1) with mu = nu and g_q = y_cv(q+1) - y_cv(q) with the
+// mixing-length viscosity of face q+1.  The sum is kept as a quotient
+// (N, D) <- (N mu + g D, D mu) with mu in units of nu: three operations a
+// cell and one division a pass, every term positive.  P lanes share a point's
+// cells and add their sums by shuffles: the FP64 pipe of each of an SM's
+// sub-partitions issues one warp instruction per 64 clocks whether or not
+// others have work, so that a wall with few points is spread over all of
+// them (66 x 66 x 2 points of 100 cells: 270 warps for 608 sub-partitions).
+//
+// exp(-y cd) of a pass is the last pass's value (kept per thread in shared
+// memory) times exp(-y dcd) as its Taylor polynomial where |y dcd| <= 2e-2
+// (degree 7; 4 up to 1e-3, 2 up to 1e-6: truncation below 1e-17 relative),
+// 16 FP64 instructions otherwise.
+//
+// Split path: the Picard passes in FP32 (at most 50, until the change is below
+// 1e-5 of tau), which also give the slope of the fixed-point map, G'(tau) =
+// (1/2r) sum g c y D (D + 2 x E) / mu^2; then one FP64 pass and the Newton
+// step t0 + (t1 - t0)/(1 - G'), whose error is that of the slope, about 1e-5
+// of a correction of 1e-6; then the reference's FP64 passes to its criterion,
+// which the first of them meets.  (Two passes and Aitken's extrapolation
+// instead needed a third FP64 pass, and a pass took a continuant recurrence
+// with seven operations a cell: 567 us per call against 340 at Re_tau 2000,
+// 258 x 258 x 2 points of 30 cells; all-FP64 4.62 ms against 2.32.)
+// ---------------------------------------------------------------------------
+constexpr int EQ_T = 128;                 // threads per block
+constexpr size_t EQ_SMEM = 100 * 1024;    // shared memory of a block at most
+__host__ __device__ __forceinline__ int eq_grid_doubles(int ncv) { return 2 * ncv + (ncv + 1); }
 
-// solve_u_eqwm (eqwm.f90:90-223) inline, grid in shared memory:
-// yfa[1..ncv+1], idcv[i] = 1/(y_cv(i+1)-y_cv(i)) (i = 1..ncv-1),
-// rw = 1/(y_cv(1)-y_fa(1)); grid[1..ncv] = y_cv, grid[ncv+1..2ncv+1] = y_fa.
-// With the learned stress (mode 1) the network's value stands for the solve
-// at points inside its training envelope; on checked calls the solve runs for
-// every point and its result is kept in tau_eq for the error record.
-__global__ void k_eq_solve(const Fld<double> Ud, const float *Uf32, int use_f32, int sy, int sz, const double *t1,
-                           const int *xst, const double *xw, const double *grid, EqParams ep, const double *nut,
-                           int nut_f32, double *tau0, double *alpha_x, double *alpha_zt, int *counters, WmState wm) {
+template <int P, bool MIXED>
+__global__ void __launch_bounds__(EQ_T) k_eq_solve(const Fld<double> Ud, const float *Uf32, int sy, int sz,
+                                                   const double *t1, const int *xst, const double *xw,
+                                                   const double *grid, EqParams ep, const void *nut, int keep_ex,
+                                                   double *tau0, double *alpha_x, double *alpha_zt, int *counters,
+                                                   WmState wm) {
     extern __shared__ double sg[];
-    const int ncv = ep.ncv;
-    // grid: yfa[1..ncv+1], idcv[1..ncv-1], rw; FP32 copies after them; then
-    // (split path, ncv <= EQ_EXP_NCV) this thread's exponentials of the
-    // last FP64 pass, Ex[(q - 2) * blockDim.x + threadIdx.x] for q = 2..ncv
-    double *yfa = sg, *idcv = sg + ncv + 2;
-    float *yfa32 = (float *)(idcv + ncv + 1), *idcv32 = yfa32 + ncv + 2;
-    double *Ex = sg + eq_exp_off(ncv) + threadIdx.x;
-    const int exs = blockDim.x;
-    const bool keep_ex = ep.mixed && ncv <= EQ_EXP_NCV;
-    for (int q = threadIdx.x; q < ncv + 2; q += blockDim.x) {
-        yfa[q] = q >= 1 && q <= ncv + 1 ? grid[ncv + q] : 0.0;
-        yfa32[q] = (float)yfa[q];
-    }
-    for (int q = threadIdx.x; q < ncv + 1; q += blockDim.x) {
-        idcv[q] = (q >= 1 && q <= ncv - 1) ? 1.0 / (grid[q + 1] - grid[q]) : 0.0;
-        idcv32[q] = (float)idcv[q];
+    const int ncv = ep.ncv, nt = ncv - 1;  // terms with a mixing-length viscosity
+    // y and g of term m = 0 .. nt-1 (face m + 2), FP32 copies after them, then the kept exponentials
+    double *y64 = sg, *g64 = sg + ncv;
+    float *y32 = (float *)(sg + 2 * ncv), *g32 = y32 + ncv;
+    double *Ex = sg + eq_grid_doubles(ncv) + threadIdx.x;
+    for (int m = threadIdx.x; m < nt; m += EQ_T) {
+        y64[m] = grid[ncv + m + 2];
+        g64[m] = grid[m + 2] - grid[m + 1];
+        y32[m] = (float)y64[m];
+        g32[m] = (float)g64[m];
     }
     __syncthreads();
-    const double rw = 1.0 / (grid[1] - grid[ncv + 1]);
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    long npts = (long)ep.nx * ep.nzg * 2;
-    if (t >= npts) return;
+    const double g0 = grid[1] - grid[ncv + 1], ymax = y64[nt - 1];
+    const int part = threadIdx.x % P;
+    const long npts = (long)ep.nx * ep.nzg * 2;
+    long t = ((long)blockIdx.x * EQ_T + threadIdx.x) / P;
+    const bool act = t < npts;
+    if (!act) t = npts - 1;  // whole warps stay: the lanes of a point add by shuffles
     const WallPt pt = wall_point(t, ep);
     const int i = pt.i, w = pt.w, k = pt.k;
     const int nxg = ep.nxg, nyg = ep.nyg;
     double Uv, wv;
-    const double u_les = wall_ules(pt, ep, Ud, Uf32, use_f32, sy, sz, t1, xst, xw, &Uv, &wv);
+    const double u_les = wall_ules(pt, ep, Ud, Uf32, MIXED, sy, sz, t1, xst, xw, &Uv, &wv);
     const long toff = pt.toff;
     const bool served = wm.mode == 1 && wm.inside[toff] != 0;
     const bool check = wm.mode == 1 && wm.check_every > 0 && (*wm.calls % wm.check_every) == 0;
     double tau = tau0[toff];
-    if (!served || check) {
+    const bool solve = act && (!served || check);
+    if (__any_sync(0xffffffffu, solve)) {
         // solve_u_eqwm(u_les, nu, 1.0, yg(jref), ncv, stretch, tau, iter, tau_in)
-        const double kappa = 0.41, Aplus = 17.0, tol = 0.0000001, mu_lam = ep.nu, rho = 1.0;
+        const double nu = ep.nu, rnu = 1.0 / nu, kn = 0.41 * rnu, cA = rnu / 17.0;  // kappa / nu, 1 / (nu A+)
         const int max_iter = 100;
-        double tau_lam = mu_lam * u_les / ep.h_wm;
+        const double tol = 0.0000001 * (nu * u_les / ep.h_wm);  // 1e-7 of the laminar stress
+        const double nuu = nu * u_les;
+        auto psum = [](auto v) {
+#pragma unroll
+            for (int o = 1; o < P; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            return v;
+        };
         int iter = 0;
         bool mixed_ok = false;  // the FP32 passes gave the FP64 ones their start
-        if (ep.mixed) {
-            // Split path: the same Picard passes in FP32 (at most 50) until
-            // the change is below 1e-5 of tau (FP32 resolves about 1e-7), the
-            // unconverged ones counted like FP64 passes; the FP64 passes
-            // below then start next to the fixed point and reach the
-            // reference's criterion after a few passes, instead of all of
-            // them in FP64 (each FP64 pass costs dozens of FP32 ones here).
-            // A non-finite or non-positive FP32 result starts the FP64
-            // passes from the initial tau instead.
-            const float mu32 = (float)mu_lam, ul32 = (float)u_les, rw32 = (float)rw;
-            const float c0 = (float)(rho * kappa), cdf = (float)(1.0 / (mu_lam / rho) / Aplus);
-            float t = (float)tau;
+        float slope = 0.f;
+        if constexpr (MIXED) {
+            const float nuu32 = (float)nuu, g00 = (float)g0, kn32 = (float)kn, cA32 = (float)cA;
+            float tq = (float)tau;
             int it = 0;
-            while (it < 50) {
-                const float tp = t, ut = sqrtf(t), c1 = c0 * ut, cd = ut * cdf;
-                float al = ul32, be = 0.f, yf = yfa32[ncv];
-                float D = 1.f - __expf(-(yf * cd));
-                float mu_up = mu32 + c1 * yf * (D * D);
-                for (int q = ncv - 1; q >= 2; q--) {
-                    yf = yfa32[q];
-                    D = 1.f - __expf(-(yf * cd));
-                    const float mu_q = mu32 + c1 * yf * (D * D);
-                    const float sup = mu_up * idcv32[q], sub = mu_q * idcv32[q - 1];
-                    const float rm = 1.f / (-(sup + sub) + sup * be);
-                    al = -sup * al * rm;
-                    be = -sub * rm;
-                    mu_up = mu_q;
+            bool run = solve;
+            // lanes whose point has converged idle until their warp's others have
+            while (__any_sync(0xffffffffu, run)) {
+                const float ut = sqrtf(tq), c = kn32 * ut, cd = ut * cA32;
+                float r = 0.f, sl = 0.f;
+                for (int m = part; m < nt; m += P) {
+                    const float y = y32[m], x = y * cd, E = __expf(-x), D = 1.f - E, cyD = c * y * D;
+                    const float q = 1.f / fmaf(cyD, D, 1.f), gq = g32[m] * q;
+                    r += gq;
+                    sl = fmaf(gq * q, cyD * fmaf(2.f * x, E, D), sl);
                 }
-                const float sup = mu_up * idcv32[1];
-                const float x1 = -sup * al / (-(sup + mu32 * rw32) + sup * be);
-                t = mu32 * x1 * rw32;
-                if (fabsf(t - tp) < 1e-5f * fabsf(t)) break;
-                it++;
+                r = g00 + psum(r);
+                sl = psum(sl);
+                const float tn = nuu32 / r;
+                if (run) {
+                    const float tp = tq;
+                    tq = tn;
+                    slope = 0.5f * sl / r;
+                    if (fabsf(tq - tp) < 1e-5f * fabsf(tq)) run = false;
+                    else if (++it >= 50) run = false;
+                }
             }
-            if (isfinite(t) && t > 0.f) {
-                tau = (double)t;
+            if (isfinite(tq) && tq > 0.f) {
+                tau = (double)tq;
                 iter = it;
                 mixed_ok = true;
             }
         }
-        // one FP64 Picard pass of solve_u_eqwm (eqwm.f90:121-205): tau from
-        // the mixing-length viscosity of the previous tau.  In the split path
-        // (keep_ex) a pass whose factor cd differs from the last pass's by
-        // |dcd| yfa[ncv] <= 1e-3 takes exp(-(y cd)) as the last pass's value
-        // times exp(-(y dcd)), the latter as its degree-4 Taylor polynomial
-        // (truncation below 1e-17 relative), instead of evaluating exp; and
-        // the elimination runs in continuant form (below), as accurate as the
-        // division per cell of the reference's Thomas sweep (both within a
-        // few 1e-14 of exact rational elimination on the same coefficients
-        // at ncv 30).
+        // one FP64 Picard pass of solve_u_eqwm (eqwm.f90:121-205)
         double cd_last = -1.0;  // no exponentials kept yet
         auto pass64 = [&](double tau) -> double {
-            double nu_eq = mu_lam / rho;
-            double utau = sqrt(tau / rho);
-            double c1 = rho * kappa * utau;
-            // y utau / nu / A+ of eqwm.f90:134-136 with the per-pass factor
-            // formed once (two FP64 divisions less per cell)
-            const double cd = utau / nu_eq / Aplus;
-            const double dcd = cd - cd_last;
-            const double xmax = fabs(dcd) * yfa[ncv];
-            const bool upd = keep_ex && cd_last >= 0.0 && xmax <= 1e-3, low = xmax <= 1e-6;
-            if (keep_ex) cd_last = cd;
-            auto ex = [&](int q, double yf) -> double {
-                double e;
-                if (upd) {
-                    // |x| <= 1e-6: degree 2 (truncation x^3/6 < 2e-19)
-                    const double x = -(yf * dcd);
-                    const double p = low ? 1.0 + x * (1.0 + 0.5 * x)
-                                         : 1.0 + x * (1.0 + x * (0.5 + x * (1.0 / 6.0 + x * (1.0 / 24.0))));
-                    e = Ex[(q - 2) * exs] * p;
-                } else {
-                    e = exp(-(yf * cd));
+            const double ut = sqrt(tau), c = kn * ut, cd = ut * cA;
+            const double dcd = cd - cd_last, xmax = fabs(dcd) * ymax;
+            // the polynomial of the warp's largest step (3: exp)
+            int lev = (cd_last >= 0.0 && xmax <= 2e-2) ? (xmax <= 1e-6 ? 0 : (xmax <= 1e-3 ? 1 : 2)) : 3;
+            lev = keep_ex ? __reduce_max_sync(0xffffffffu, lev) : 3;
+            cd_last = cd;
+            double N = 0.0, Dn = 1.0;
+            auto sweep = [&](auto &&ex) {
+                int s = 0;
+                for (int m = part; m < nt; m += P, s++) {
+                    const double y = y64[m], E = ex(y, s), D = 1.0 - E;
+                    if (keep_ex) Ex[s * EQ_T] = E;
+                    const double mu = fma(c * y, D * D, 1.0);
+                    N = fma(g64[m], Dn, N * mu);
+                    Dn *= mu;
+                    if ((s & 7) == 7) {  // powers of two out (exact), well before the range ends
+                        const int e = ((__double2hiint(Dn) >> 20) & 0x7ff) - 1023;
+                        if (e > 128 && e < 1024) {
+                            const double sc = __hiloint2double((1023 - e) << 20, 0);  // 2^-e
+                            N *= sc;
+                            Dn *= sc;
+                        }
+                    }
                 }
-                if (keep_ex) Ex[(q - 2) * exs] = e;
-                return e;
             };
-            double yf = yfa[ncv];
-            double D = 1.0 - ex(ncv, yf);
-            double mu_up = mu_lam + c1 * yf * (D * D);
-            if (!ep.mixed) {
-                double al = u_les, be = 0.0;
-                for (int q = ncv - 1; q >= 2; q--) {
-                    yf = yfa[q];
-                    D = 1.0 - ex(q, yf);
-                    double mu_q = mu_lam + c1 * yf * (D * D);
-                    double sup = mu_up * idcv[q];
-                    double sub = mu_q * idcv[q - 1];
-                    double m = -1.0 * (sup + sub) + sup * be;
-                    double rm = 1.0 / m;
-                    al = -sup * al * rm;
-                    be = -sub * rm;
-                    mu_up = mu_q;
-                }
-                double sup = mu_up * idcv[1];
-                double diag = -1.0 * (sup + mu_lam * rw);
-                double x1 = -sup * al / (diag + sup * be);
-                return mu_lam * (x1 - 0.0) * rw;
+            if (lev == 3) {
+                sweep([&](double y, int) { return exp(-(y * cd)); });
+            } else if (lev == 2) {
+                sweep([&](double y, int s) {
+                    const double x = y * -dcd;
+                    double p = fma(x, 1.0 / 5040.0, 1.0 / 720.0);
+                    p = fma(x, p, 1.0 / 120.0);
+                    p = fma(x, p, 1.0 / 24.0);
+                    p = fma(x, p, 1.0 / 6.0);
+                    p = fma(x, p, 0.5);
+                    p = fma(x, p, 1.0);
+                    const double e = Ex[s * EQ_T];
+                    return fma(e * x, p, e);
+                });
+            } else if (lev == 1) {
+                sweep([&](double y, int s) {
+                    const double x = y * -dcd;
+                    double p = fma(x, 1.0 / 24.0, 1.0 / 6.0);
+                    p = fma(x, p, 0.5);
+                    p = fma(x, p, 1.0);
+                    const double e = Ex[s * EQ_T];
+                    return fma(e * x, p, e);
+                });
+            } else {
+                sweep([&](double y, int s) {
+                    const double x = y * -dcd, p = fma(x, 0.5, 1.0), e = Ex[s * EQ_T];
+                    return fma(e * x, p, e);
+                });
             }
-            // Split path: the same elimination without a division per cell.
-            // With the pivots m_q = Dn_q / Dn_{q+1} (Dn_ncv = 1) the
-            // continuants follow Dn_q = -(sup_q + sub_q) Dn_{q+1} -
-            // sup_q sub_{q+1} Dn_{q+2}, and A_q = al_q Dn_q = -sup_q A_{q+1};
-            // be_2 = -sub_2 Dn_3 / Dn_2, al_2 = A_2 / Dn_2, so the first cell's
-            // unknown is one quotient.  sup_q = sub_{q+1} (both mu_{q+1} /
-            // (y_cv(q+1) - y_cv(q))).  Dn, A are rescaled by powers of two
-            // (exact) every 8 cells to stay in range.
-            double Dn1 = 1.0, Dn2 = 0.0, A = u_les, subp = 0.0;
-            double sup = mu_up * idcv[ncv - 1];
-            for (int q = ncv - 1; q >= 2; q--) {
-                yf = yfa[q];
-                D = 1.0 - ex(q, yf);
-                const double mu_q = mu_lam + c1 * yf * (D * D);
-                const double sub = mu_q * idcv[q - 1];
-                const double Dn = fma(-(sup + sub), Dn1, -(sup * subp) * Dn2);
-                A = -sup * A;
-                Dn2 = Dn1;
-                Dn1 = Dn;
-                subp = sub;
-                sup = sub;
-                if ((q & 7) == 0) {
-                    const int e = ((__double2hiint(Dn1) >> 20) & 0x7ff) - 1023;
-                    if (e > 512 || e < -512) {
-                        const double sc = __hiloint2double((1023 - e) << 20, 0);  // 2^-e
-                        Dn1 *= sc;
-                        Dn2 *= sc;
-                        A *= sc;
+            return nuu / (g0 + psum(N / Dn));
+        };
+        bool run = solve;
+        if constexpr (MIXED) {
+            if (__any_sync(0xffffffffu, run && mixed_ok)) {
+                const double t0 = tau, tn = pass64(t0);
+                if (run && mixed_ok) {
+                    if (fabs(tn - t0) < tol) {
+                        tau = tn;
+                        run = false;
+                    } else {
+                        iter = iter + 1;
+                        const double ta = t0 + (tn - t0) / (1.0 - (double)slope);
+                        tau = (slope < 0.9f && isfinite(ta) && ta > 0.0) ? ta : tn;
                     }
                 }
             }
-            // sup = mu_2 / (y_cv(2) - y_cv(1)) of the first cell
-            const double diag = -1.0 * (sup + mu_lam * rw);
-            const double x1 = -sup * A / (diag * Dn1 - sup * subp * Dn2);
-            return mu_lam * x1 * rw;
-        };
-        bool fin = false;
-        if (ep.mixed && mixed_ok) {
-            // Split path, from the FP32 iterate: two FP64 passes (checked and
-            // counted like the reference's), then Aitken's extrapolation of
-            // the linearly converging sequence; the reference passes below
-            // take it from there to the reference's criterion.
-            const double t0 = tau, t1 = pass64(t0);
-            if (fabs((t1 - t0) / tau_lam) < tol) {
-                tau = t1;
-                fin = true;
-            } else {
-                iter = iter + 1;
-                const double t2 = pass64(t1);
-                if (fabs((t2 - t1) / tau_lam) < tol) {
-                    tau = t2;
-                    fin = true;
-                } else {
-                    iter = iter + 1;
-                    const double d1 = t1 - t0, d2 = t2 - t1, den = d2 - d1;
-                    const double ta = den != 0.0 ? t2 - d2 * d2 / den : t2;
-                    tau = (isfinite(ta) && ta > 0.0) ? ta : t2;
-                }
+        }
+        while (__any_sync(0xffffffffu, run)) {
+            const double tn = pass64(tau);
+            if (run) {
+                if (fabs(tn - tau) < tol) run = false;
+                else if (++iter > max_iter) run = false;
+                tau = tn;
             }
         }
-        while (!fin) {
-            double tau_prev = tau;
-            tau = pass64(tau);
-            int done = 0;
-            if (fabs((tau - tau_prev) / tau_lam) < tol) done = 1;
-            if (done == 0) iter = iter + 1;
-            if (iter > max_iter) done = 1;
-            if (done) break;
-        }
         // wallmodel.f90:620-640
-        if (isnan(tau)) {
-            atomicAdd(&counters[0], 1);
-            tau = ep.tau_mean;
+        if (solve) {
+            if (isnan(tau)) {
+                if (part == 0) atomicAdd(&counters[0], 1);
+                tau = ep.tau_mean;
+            }
+            if (iter == 100) {
+                tau = ep.tau_mean;
+                if (part == 0) atomicAdd(&counters[1], 1);
+            }
+            if (check && part == 0) wm.tau_eq[toff] = tau;
         }
-        if (iter == 100) {
-            tau = ep.tau_mean;
-            atomicAdd(&counters[1], 1);
-        }
-        if (check) wm.tau_eq[toff] = tau;
     }
+    if (!act || part != 0) return;
     if (served) tau = wm.tau_nn[toff];
     tau0[toff] = tau;
-    double tx = tau * Uv / u_les, tz = tau * wv / u_les;
-    int ja = w == 0 ? 1 : nyg, jb = w == 0 ? 2 : nyg - 1;
-    long cs = (long)nxg * nyg;
+    const int ja = w == 0 ? 1 : nyg, jb = w == 0 ? 2 : nyg - 1;
+    const long cs = (long)nxg * nyg;
     auto NT = [&](int ii, int j) -> double {
-        long o = (long)(ii - 1) + (long)nxg * (j - 1) + cs * (k - 1);
-        return nut_f32 ? (double)((const float *)nut)[o] : nut[o];
+        const long o = (long)(ii - 1) + (long)nxg * (j - 1) + cs * (k - 1);
+        return MIXED ? (double)((const float *)nut)[o] : ((const double *)nut)[o];
     };
-    double nu_t_ik = 0.5 * (0.5 * (NT(i, ja) + NT(i + 1, ja)) + 0.5 * (NT(i, jb) + NT(i + 1, jb)));
-    alpha_x[toff] = tx / (ep.nu + nu_t_ik);
-    alpha_zt[toff] = tz / (ep.nu + nu_t_ik);
+    const double nu_t_ik = 0.25 * ((NT(i, ja) + NT(i + 1, ja)) + (NT(i, jb) + NT(i + 1, jb)));
+    const double f = tau / (u_les * (ep.nu + nu_t_ik));
+    alpha_x[toff] = f * Uv;
+    alpha_zt[toff] = f * wv;
+}
+
+// lanes per point: the count that minimises (warps on the busiest
+// sub-partition) x (45 + 16 per cell of a lane) FP64 instructions of a pass
+static int eq_parts(long npts, int ncv) {
+    int best = 1;
+    double best_cost = 1e300;
+    for (int p = 1; p <= 8; p *= 2) {
+        const double cost = (double)cdiv(cdiv(npts * p, 32), 4 * 152) * (45.0 + 16.0 * cdiv(ncv - 1, p));
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = p;
+        }
+    }
+    return best;
+}
+
+template <int P, bool MIXED>
+static void eq_launch(cf_ctx *ctx, const Fld<double> &Ud, const EqParams &ep, int b, const WmState &wm) {
+    const long npts = (long)ep.nx * ep.nzg * 2;
+    const size_t base = (size_t)eq_grid_doubles(ep.ncv) * sizeof(double),
+                 ex = (size_t)cdiv(ep.ncv - 1, P) * EQ_T * sizeof(double);
+    const int keep = base + ex <= EQ_SMEM;
+    k_eq_solve<P, MIXED><<<cdiv(npts * P, EQ_T), EQ_T, base + (keep ? ex : 0), ctx->st>>>(
+        Ud, (const float *)ctx->U[b], ep.nx, ep.nx * ep.nyg, ctx->wtemp1, ctx->eq_xst, ctx->eq_xw, ctx->eq_grid, ep,
+        ctx->nut, keep, ctx->tau0, ctx->alpha_x, ctx->alpha_zt, (int *)ctx->d_red, wm);
+}
+
+template <bool MIXED>
+static void eq_launch_parts(cf_ctx *ctx, const Fld<double> &Ud, const EqParams &ep, int b, const WmState &wm) {
+    switch (eq_parts((long)ep.nx * ep.nzg * 2, ep.ncv)) {
+    case 1: eq_launch<1, MIXED>(ctx, Ud, ep, b, wm); break;
+    case 2: eq_launch<2, MIXED>(ctx, Ud, ep, b, wm); break;
+    case 4: eq_launch<4, MIXED>(ctx, Ud, ep, b, wm); break;
+    default: eq_launch<8, MIXED>(ctx, Ud, ep, b, wm);
+    }
+}
+
+// shared-memory opt-in (called at context creation)
+int eqwm_setup() {
+#define CF_EQ_ATTR(P)                                                                                           \
+    cudaFuncSetAttribute(k_eq_solve<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EQ_SMEM); \
+    cudaFuncSetAttribute(k_eq_solve<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EQ_SMEM);
+    CF_EQ_ATTR(1) CF_EQ_ATTR(2) CF_EQ_ATTR(4) CF_EQ_ATTR(8)
+#undef CF_EQ_ATTR
+    return 0;
 }
 
 // The error record of checked calls: max and mean |tau_nn/tau_eq - 1| over
@@ -409,11 +430,8 @@ int launch_eqwm(cf_ctx *ctx, int b) {
     ep.nu = ctx->prm.nu;
     ep.h_wm = ctx->hyg[ep.jref];
     ep.tau_mean = ctx->hs.tau_mean_eqwm;
-    ep.mixed = sizeof(T) == 4;
     CF_CUDA(cudaMemsetAsync(ctx->d_red, 0, 2 * sizeof(int), ctx->st));
     long npts = (long)nx * nzg * 2;
-    size_t sh = (size_t)eq_exp_off(ep.ncv) * sizeof(double);
-    if (ep.mixed && ep.ncv <= EQ_EXP_NCV) sh += (size_t)(ep.ncv - 1) * 128 * sizeof(double);
     Fld<double> Ud = make_fld<double>(ctx->U[b], nx, nyg);
     WmState wm = {};
     if (ctx->wmlp) {
@@ -429,10 +447,7 @@ int launch_eqwm(cf_ctx *ctx, int b) {
         wm.mode = 1;
         wm.tau_eq = ctx->wm_tau_eq;
     }
-    k_eq_solve<<<cdiv(npts, 128), 128, sh, ctx->st>>>(Ud, (const float *)ctx->U[b], sizeof(T) == 4, nx, nx * nyg,
-                                                     ctx->wtemp1, ctx->eq_xst, ctx->eq_xw, ctx->eq_grid, ep,
-                                                     (const double *)ctx->nut, sizeof(T) == 4, ctx->tau0, ctx->alpha_x,
-                                                     ctx->alpha_zt, (int *)ctx->d_red, wm);
+    eq_launch_parts<sizeof(T) == 4>(ctx, Ud, ep, b, wm);
     count_launch(ctx, "k_eq_solve");
     if (ctx->wmlp) {
         k_wm_audit<<<1, 1024, 0, ctx->st>>>(npts, ctx->wm_tau, ctx->wm_inside, ctx->wm_tau_eq, ctx->wm_calls,

@@ -111,3 +111,66 @@ def test_rhs_segments_rows_and_chunks(dims, les, wall, vary, kw):
     ch.close()
     o.close()
 
+
+def eqwm_stress(u_les, h, nu, ncv, stretch, tau):
+    """The wall stress of solve_u_eqwm (eqwm.f90:20-223) in extended precision:
+    the same Picard passes to the same criterion, each from the resistances of
+    the faces in series, which is what the tridiagonal system solves."""
+    L = np.longdouble
+    fa = np.concatenate([[0.0], np.cumsum(np.cumprod(np.r_[1.0, np.full(ncv - 1, stretch)]))])
+    cv = (fa[1:] + fa[:-1]) / 2
+    fa, cv = (fa / cv[-1] * h).astype(L), (cv / cv[-1] * h).astype(L)
+    u_les, nu, tau = u_les.astype(L), L(nu), tau.astype(L)
+    tol, run = L("1e-7") * nu * u_les / L(h), np.full(tau.shape, True)
+    for _ in range(101):
+        ut = np.sqrt(tau)
+        r = (cv[0] - fa[0]) / nu + np.zeros_like(tau)
+        for q in range(1, ncv):
+            y = fa[q]
+            r += (cv[q] - cv[q - 1]) / (nu + L("0.41") * ut * y * (1 - np.exp(-y * ut / nu / 17)) ** 2)
+        new = u_les / r
+        tau, run = np.where(run, new, tau), run & ~(np.abs(new - tau) < tol)
+        if not run.any():
+            break
+    return tau.astype(float)
+
+
+@pytest.mark.parametrize("dims,ncv,stretch", [((18, 9, 18), 30, 1.10), ((18, 9, 18), 100, 1.10), ((18, 9, 18), 3, 1.10),
+                                              ((18, 9, 18), 2000, 1.001), ((50, 9, 50), 45, 1.10),
+                                              ((66, 9, 82), 30, 1.10), ((130, 9, 130), 30, 1.10)])
+def test_eqwm_lanes_per_point(dims, ncv, stretch):
+    """The FP64 equilibrium wall model with one to eight lanes per wall point
+    (the count falls with the number of points), few and many ODE cells, with
+    and without room for the kept exponentials; a first call from the mean
+    stress and a second one from the first's result.  Both iterate the same
+    map to the same criterion, so that they stop at the same pass and agree to
+    rounding: 1e-12, counters equal.  With 2000 cells the oracle's Thomas sweep
+    is itself 1e-12 to 1e-11 from the exact solution of its system (its
+    rounding grows as the square of the cells), so that the stress is held to
+    the same passes in extended precision and alpha_x to the oracle's
+    alpha_x / stress."""
+    case = channel_case(*dims, stretch=0.0, wall=3, retau=2000.0, profile="plug", jref=3, ncv=ncv)
+    case["prm"]["eqwm_stretch"] = stretch
+    from channelflow.wallmlp import wall_model_inputs
+    o, ch = pair(case)
+    for d in (o, ch):
+        d.apply_boundary_conditions()
+        d.compute_eddy_viscosity()
+    for _ in range(2):
+        if ncv > 1000:
+            u_les, h, nu = (v.cpu().numpy() if hasattr(v, "cpu") else v for v in wall_model_inputs(ch))
+            tau_in = ch.download_wall()["tau_eqwm_initial"]
+            want = eqwm_stress(u_les.reshape(tau_in.shape, order="F"), h, nu, ncv, stretch, tau_in)
+        o.compute_wall_model()
+        ch.compute_wall_model()
+        w = ch.download_wall()
+        if ncv > 1000:
+            tau, t0 = w["tau_eqwm_initial"], o.array("tau_eqwm_initial")
+            assert_close(tau, want, 1e-12, "tau_eqwm_initial")
+            assert_close(w["alpha_x"] / tau, o.array("alpha_x") / t0, 1e-12, "alpha_x / tau")
+        else:
+            for n in ("alpha_x", "alpha_z", "tau_eqwm_initial"):
+                assert_close(w[n], o.array(n), 1e-12, n)
+        assert ch.eqwm_counters() == (int(o.scalar("n_nan_eqwm")), int(o.scalar("n_iter_eqwm")))
+    ch.close()
+    o.close()
