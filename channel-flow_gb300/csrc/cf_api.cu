@@ -510,19 +510,7 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
         if (ctx->esz == 8) {
             ctx->rhs_nkc = rhs64_plan(nxp, ctx->nym, nzp, dev_sms);
         } else {
-            // fused RHS: 32 x 8 column tiles; z chunks: the count that
-            // minimises (waves of resident blocks) x (planes per chunk + the
-            // 2 halo planes a chunk loads again)
-            long rt = (long)cdiv(ctx->nxp, 32) * cdiv(ctx->nyg - 2, 8);
-            const long res = (long)rhs3_blocks_per_sm() * dev_sms;
-            long best = 1;
-            double best_cost = 1e300;
-            for (long n = 1; n <= std::max(1L, (long)ctx->nzp / 4); n++) {
-                const double waves = (double)((rt * n + res - 1) / res);
-                const double cost = waves * ((double)cdiv(ctx->nzp, n) + 2.0);
-                if (cost < best_cost - 1e-9) { best_cost = cost; best = n; }
-            }
-            ctx->rhs_nkc = (int)best;
+            ctx->rhs_nkc = rhs32_plan(nxp, ctx->nym, nzp, dev_sms);
         }
         if (p->LES_model == 3) amd_plan(p->precision == CF_PREC_SPLIT ? 4 : 8, nxp, ctx->nym, nzp, dev_sms, &ctx->amd_nkc, &amd_parts);
     }
@@ -1611,7 +1599,7 @@ static int capture_batched_step(cf_ensemble *e, int *extra) {
             }
             if (!rc && !rm.empty()) {
                 if (esz == 4) {
-                    rc = launch_rhs3_batch<float>(e->st, rm.data(), s, rs.data(), rd.data(), (int)rm.size());
+                    rc = launch_rhs32_batch(e->st, rm.data(), s, rs.data(), rd.data(), (int)rm.size());
                     *extra += 1;
                 } else {  // FP64 members: their own launches, one after the other
                     for (size_t q = 0; q < rm.size() && !rc; q++) {

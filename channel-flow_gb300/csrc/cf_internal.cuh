@@ -47,6 +47,21 @@ __host__ __device__ static inline Fld<T> make_fld(void *p, int n1, int n2) {
     return f;
 }
 
+// rk_coef (initialization.f90:408-416)
+struct RkCoef {
+    double c[4][4];
+};
+inline RkCoef rk_coefs() {
+    RkCoef c = {};
+    c.c[1][1] = 8.0 / 15.0;
+    c.c[2][1] = 1.0 / 4.0;
+    c.c[2][2] = 5.0 / 12.0;
+    c.c[3][1] = 1.0 / 4.0;
+    c.c[3][2] = 0.0;
+    c.c[3][3] = 3.0 / 4.0;
+    return c;
+}
+
 // one field per velocity component
 template <typename T>
 struct Trio {
@@ -282,7 +297,8 @@ int cf_fail(cf_ctx *ctx, int code, const std::string &msg);
 // ---- launchers (kernels in the .cu files), all enqueue on ctx->st -------
 template <typename T> int launch_bc(cf_ctx *ctx, int buf, bool lo = true);  // apply_boundary_conditions (lo: low words too)
 template <typename T> int launch_rhs(cf_ctx *ctx, int comp, int slot);     // store F slot
-int rhs3_blocks_per_sm();
+int rhs32_plan(int nxp, int nym, int nzp, int sms);                         // z chunks of the fused right-hand side
+int launch_rhs32(cf_ctx *ctx, int s, int src, int dst);                     // FP32 right-hand sides + RK update of substep s
 int rhs64_plan(int nxp, int nym, int nzp, int sms);                        // z chunks of the FP64 right-hand side
 int launch_rhs64(cf_ctx *ctx, cudaStream_t st, int s, int src, int dst);    // FP64 RHS + RK update
 int launch_rhs64_comp(cf_ctx *ctx, int comp, int slot);                     // one FP64 right-hand side into slot
@@ -297,7 +313,7 @@ void dsm64_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
 int dsm64_slots(int nxp, int nzp, int kc);                                 // its partials per row with chunks of kc planes
 constexpr int CF_ENS_MAXM = 32;  // channels per batched ensemble launch at most
 // fused right-hand sides + RK update of substep s of n split-path channels in one launch
-template <typename T> int launch_rhs3_batch(cudaStream_t st, cf_ctx *const *m, int s, const int *src, const int *dst, int n);
+int launch_rhs32_batch(cudaStream_t st, cf_ctx *const *m, int s, const int *src, const int *dst, int n);
 template <typename T> int launch_nut_zero(cf_ctx *ctx);
 template <typename T> int launch_nut_materialize(cf_ctx *ctx);       // fill nut if held lazily
 int launch_nut_rhs64(cf_ctx *ctx, cudaStream_t st, void **field);    // nu_t for the FP64 right-hand side

@@ -141,25 +141,11 @@ int launch_bc(cf_ctx *ctx, int b, bool lo) {
 // ---------------------------------------------------------------------------
 // Momentum right-hand sides, equations.f90:24-498, one thread per point.
 // ---------------------------------------------------------------------------
-struct RkCoef {
-    double c[4][4];
-};
-
 // The spacings enter as reciprocals (rc): 1/(xg(i+1)-xg(i)) = rc.dxg[i+1],
 // 1/(x(i)-x(i-1)) = rc.dx[i], and so on.
-//
-// ZC (the z-marching fused kernel): the z-face terms of a cell -- its
-// advective and viscous fluxes through the faces k-1/2 and k+1/2 -- are
-// taken as rdz3 * (F(k+1/2) - F(k-1/2)) with F = viscous flux less advective
-// flux; *fz holds F(k-1/2) on entry (carried from the cell below, or formed
-// by rhs_*_zflux_dn for the first plane of a chunk) and F(k+1/2) as the
-// next cell's F(k-1/2) on return (for u with the spacing 1/(x(i)-x(i-1))
-// that the reference's lower face uses, rdx1; the cell's own upper face
-// uses rdx2).
-template <typename T, typename A, typename RC, bool ZC = false>
+template <typename T, typename A, typename RC>
 __device__ __forceinline__ T rhs_u_point(const GeoT<T> &g, const RC &rc, const A &U, const A &V, const A &W,
-                                         const A &nt, T nu, T dPdx, T Om, bool rot, int i, int j, int k,
-                                         T *fz = nullptr) {
+                                         const A &nt, T nu, T dPdx, T Om, bool rot, int i, int j, int k) {
     const T *w0 = g.w0, *w1 = g.w1;
     const T h = T(0.5), q = T(0.25);
     const T rdx1 = rc.dx[i], rdx2 = rc.dx[i + 1], rdx3 = rc.dxg[i + 1];
@@ -178,11 +164,9 @@ __device__ __forceinline__ T rhs_u_point(const GeoT<T> &g, const RC &rc, const A
     // 3) -duw/dz   (:84-101)
     T uz1 = h * (U(i, j, k) + U(i, j, k + 1));
     T wx1 = h * (W(i, j, k) + W(i + 1, j, k));
-    if constexpr (!ZC) {
-        T uz0 = h * (U(i, j, k - 1) + U(i, j, k));
-        T wx0 = h * (W(i, j, k - 1) + W(i + 1, j, k - 1));
-        r += -(uz1 * wx1 - uz0 * wx0) * rdz3;
-    }
+    T uz0 = h * (U(i, j, k - 1) + U(i, j, k));
+    T wx0 = h * (W(i, j, k - 1) + W(i + 1, j, k - 1));
+    r += -(uz1 * wx1 - uz0 * wx0) * rdz3;
     // 4) viscous   (:108-163)
     T t2j = (U(i, j + 1, k) - U(i, j, k)) * rc.dyg[j + 1];
     T t2jm = (U(i, j, k) - U(i, j - 1, k)) * rc.dyg[j];
@@ -195,17 +179,10 @@ __device__ __forceinline__ T rhs_u_point(const GeoT<T> &g, const RC &rc, const A
     T visc = T(2) * rdx3 * (nu_x2 * (U(i + 1, j, k) - U(i, j, k)) * rdx2 - nu_x1 * (U(i, j, k) - U(i - 1, j, k)) * rdx1) +
              rdy3 * (nu_y2 * (t2j + (V(i + 1, j, k) - V(i, j, k)) * rdx2) -
                      nu_y1 * (t2jm + (V(i + 1, j - 1, k) - V(i, j - 1, k)) * rdx1));
-    if constexpr (!ZC) {
-        T nu_z1 = nu + q * (nt(i, j, k) + nt(i, j, k - 1) + nt(i + 1, j, k) + nt(i + 1, j, k - 1));
-        visc += rdz3 * (nu_z2 * ((U(i, j, k + 1) - U(i, j, k)) * rdz2 + (W(i + 1, j, k) - W(i, j, k)) * rdx2) -
-                        nu_z1 * ((U(i, j, k) - U(i, j, k - 1)) * rdz1 + (W(i + 1, j, k - 1) - W(i, j, k - 1)) * rdx1));
-        r += visc;
-    } else {
-        r += visc;
-        const T gz = (U(i, j, k + 1) - U(i, j, k)) * rdz2, dw = W(i + 1, j, k) - W(i, j, k), a = uz1 * wx1;
-        r += rdz3 * ((nu_z2 * (gz + dw * rdx2) - a) - *fz);
-        *fz = nu_z2 * (gz + dw * rdx1) - a;
-    }
+    T nu_z1 = nu + q * (nt(i, j, k) + nt(i, j, k - 1) + nt(i + 1, j, k) + nt(i + 1, j, k - 1));
+    visc += rdz3 * (nu_z2 * ((U(i, j, k + 1) - U(i, j, k)) * rdz2 + (W(i + 1, j, k) - W(i, j, k)) * rdx2) -
+                    nu_z1 * ((U(i, j, k) - U(i, j, k - 1)) * rdz1 + (W(i + 1, j, k - 1) - W(i, j, k - 1)) * rdx1));
+    r += visc;
     r += dPdx;  // :166
     if (rot) {  // |Om| > 1e-6, :169-177
         T tv0 = h * (V(i, j - 1, k) + V(i, j, k));
@@ -215,9 +192,9 @@ __device__ __forceinline__ T rhs_u_point(const GeoT<T> &g, const RC &rc, const A
     return r;
 }
 
-template <typename T, typename A, typename RC, bool ZC = false>
+template <typename T, typename A, typename RC>
 __device__ __forceinline__ T rhs_v_point(const GeoT<T> &g, const RC &rc, const A &U, const A &V, const A &W,
-                                         const A &nt, T nu, T Om, bool rot, int i, int j, int k, T *fz = nullptr) {
+                                         const A &nt, T nu, T Om, bool rot, int i, int j, int k) {
     const T *w0 = g.w0, *w1 = g.w1;
     const T h = T(0.5);
     const T rdx1 = rc.dxg[i], rdx2 = rc.dxg[i + 1], rdx3 = rc.dx[i];
@@ -236,11 +213,9 @@ __device__ __forceinline__ T rhs_v_point(const GeoT<T> &g, const RC &rc, const A
     // 3) -dvw/dz (:250-267)
     T vz1 = h * (V(i, j, k) + V(i, j, k + 1));
     T wy1 = w0[j] * W(i, j, k) + w1[j] * W(i, j + 1, k);
-    if constexpr (!ZC) {
-        T vz0 = h * (V(i, j, k - 1) + V(i, j, k));
-        T wy0 = w0[j] * W(i, j, k - 1) + w1[j] * W(i, j + 1, k - 1);
-        r += -(vz1 * wy1 - vz0 * wy0) * rdz3;
-    }
+    T vz0 = h * (V(i, j, k - 1) + V(i, j, k));
+    T wy0 = w0[j] * W(i, j, k - 1) + w1[j] * W(i, j + 1, k - 1);
+    r += -(vz1 * wy1 - vz0 * wy0) * rdz3;
     // 4) viscous (:276-331)
     T nu_x1 = nu + h * (w0[j] * nt(i - 1, j, k) + w1[j] * nt(i - 1, j + 1, k) + w0[j] * nt(i, j, k) + w1[j] * nt(i, j + 1, k));
     T nu_x2 = nu + h * (w0[j] * nt(i, j, k) + w1[j] * nt(i, j + 1, k) + w0[j] * nt(i + 1, j, k) + w1[j] * nt(i + 1, j + 1, k));
@@ -250,17 +225,10 @@ __device__ __forceinline__ T rhs_v_point(const GeoT<T> &g, const RC &rc, const A
     T visc = rdx3 * (nu_x2 * ((V(i + 1, j, k) - V(i, j, k)) * rdx2 + (U(i, j + 1, k) - U(i, j, k)) * rdy3) -
                      nu_x1 * ((V(i, j, k) - V(i - 1, j, k)) * rdx1 + (U(i - 1, j + 1, k) - U(i - 1, j, k)) * rdy3)) +
              T(2) * rdy3 * (nu_y2 * (V(i, j + 1, k) - V(i, j, k)) * rdy2 - nu_y1 * (V(i, j, k) - V(i, j - 1, k)) * rdy1);
-    if constexpr (!ZC) {
-        T nu_z1 = nu + h * (w0[j] * nt(i, j, k - 1) + w1[j] * nt(i, j + 1, k - 1) + w0[j] * nt(i, j, k) + w1[j] * nt(i, j + 1, k));
-        visc += rdz3 * (nu_z2 * ((V(i, j, k + 1) - V(i, j, k)) * rdz2 + (W(i, j + 1, k) - W(i, j, k)) * rdy3) -
-                        nu_z1 * ((V(i, j, k) - V(i, j, k - 1)) * rdz1 + (W(i, j + 1, k - 1) - W(i, j, k - 1)) * rdy3));
-        r += visc;
-    } else {
-        r += visc;
-        const T f = nu_z2 * ((V(i, j, k + 1) - V(i, j, k)) * rdz2 + (W(i, j + 1, k) - W(i, j, k)) * rdy3) - vz1 * wy1;
-        r += rdz3 * (f - *fz);
-        *fz = f;
-    }
+    T nu_z1 = nu + h * (w0[j] * nt(i, j, k - 1) + w1[j] * nt(i, j + 1, k - 1) + w0[j] * nt(i, j, k) + w1[j] * nt(i, j + 1, k));
+    visc += rdz3 * (nu_z2 * ((V(i, j, k + 1) - V(i, j, k)) * rdz2 + (W(i, j + 1, k) - W(i, j, k)) * rdy3) -
+                    nu_z1 * ((V(i, j, k) - V(i, j, k - 1)) * rdz1 + (W(i, j + 1, k - 1) - W(i, j, k - 1)) * rdy3));
+    r += visc;
     if (rot) {  // :334-342
         T tu0 = h * (U(i - 1, j, k) + U(i, j, k));
         T tu1 = h * (U(i - 1, j + 1, k) + U(i, j + 1, k));
@@ -269,9 +237,9 @@ __device__ __forceinline__ T rhs_v_point(const GeoT<T> &g, const RC &rc, const A
     return r;
 }
 
-template <typename T, typename A, typename RC, bool ZC = false>
+template <typename T, typename A, typename RC>
 __device__ __forceinline__ T rhs_w_point(const GeoT<T> &g, const RC &rc, const A &U, const A &V, const A &W,
-                                         const A &nt, T nu, T dPdz, int i, int j, int k, T *fz = nullptr) {
+                                         const A &nt, T nu, T dPdz, int i, int j, int k) {
     const T *w0 = g.w0, *w1 = g.w1;
     const T h = T(0.5), q = T(0.25);
     const T rdx1 = rc.dxg[i], rdx2 = rc.dxg[i + 1], rdx3 = rc.dx[i];
@@ -280,10 +248,8 @@ __device__ __forceinline__ T rhs_w_point(const GeoT<T> &g, const RC &rc, const A
     // 1) -dw^2/dz (equations.f90:370-384)
     T a = h * (W(i, j, k) + W(i, j, k + 1));
     T r = T(0);
-    if constexpr (!ZC) {
-        T b = h * (W(i, j, k - 1) + W(i, j, k));
-        r = -(a * a - b * b) * rdz3;
-    }
+    T b = h * (W(i, j, k - 1) + W(i, j, k));
+    r = -(a * a - b * b) * rdz3;
     // 2) -duw/dx (:389-406)
     T uz1 = h * (U(i, j, k) + U(i, j, k + 1));
     T uz0 = h * (U(i - 1, j, k) + U(i - 1, j, k + 1));
@@ -309,46 +275,11 @@ __device__ __forceinline__ T rhs_w_point(const GeoT<T> &g, const RC &rc, const A
                      nu_x1 * ((W(i, j, k) - W(i - 1, j, k)) * rdx1 + (U(i - 1, j, k + 1) - U(i - 1, j, k)) * rdz1)) +
              rdy3 * (nu_y2 * (t2j + (V(i, j, k + 1) - V(i, j, k)) * rdz2) -
                      nu_y1 * (t2jm + (V(i, j - 1, k + 1) - V(i, j - 1, k)) * rdz1));
-    if constexpr (!ZC) {
-        T nu_z1 = nu + nt(i, j, k);
-        visc += T(2) * rdz3 * (nu_z2 * (W(i, j, k + 1) - W(i, j, k)) * rdz2 - nu_z1 * (W(i, j, k) - W(i, j, k - 1)) * rdz1);
-        r += visc;
-    } else {
-        r += visc;
-        const T f = T(2) * (nu_z2 * (W(i, j, k + 1) - W(i, j, k)) * rdz2) - a * a;
-        r += rdz3 * (f - *fz);
-        *fz = f;
-    }
+    T nu_z1 = nu + nt(i, j, k);
+    visc += T(2) * rdz3 * (nu_z2 * (W(i, j, k + 1) - W(i, j, k)) * rdz2 - nu_z1 * (W(i, j, k) - W(i, j, k - 1)) * rdz1);
+    r += visc;
     r += dPdz;  // :496
     return r;
-}
-
-// F(k-1/2) of the u, v and w cells at (i, j, k) as the reference's lower
-// z faces take them (the first plane of a z-marching chunk; later planes
-// carry it from the cell below, see ZC above).
-template <typename T, typename A, typename RC>
-__device__ __forceinline__ void rhs_zflux_dn(const GeoT<T> &g, const RC &rc, const A &U, const A &V, const A &W,
-                                             const A &nt, T nu, int i, int j, int k, T &fu, T &fv, T &fw) {
-    const T *w0 = g.w0, *w1 = g.w1;
-    const T h = T(0.5), q = T(0.25);
-    {
-        const T uz0 = h * (U(i, j, k - 1) + U(i, j, k)), wx0 = h * (W(i, j, k - 1) + W(i + 1, j, k - 1));
-        const T nu_z1 = nu + q * (nt(i, j, k) + nt(i, j, k - 1) + nt(i + 1, j, k) + nt(i + 1, j, k - 1));
-        fu = nu_z1 * ((U(i, j, k) - U(i, j, k - 1)) * rc.dzg[k] + (W(i + 1, j, k - 1) - W(i, j, k - 1)) * rc.dx[i]) -
-             uz0 * wx0;
-    }
-    {
-        const T vz0 = h * (V(i, j, k - 1) + V(i, j, k)), wy0 = w0[j] * W(i, j, k - 1) + w1[j] * W(i, j + 1, k - 1);
-        const T nu_z1 =
-            nu + h * (w0[j] * nt(i, j, k - 1) + w1[j] * nt(i, j + 1, k - 1) + w0[j] * nt(i, j, k) + w1[j] * nt(i, j + 1, k));
-        fv = nu_z1 * ((V(i, j, k) - V(i, j, k - 1)) * rc.dzg[k] + (W(i, j + 1, k - 1) - W(i, j, k - 1)) * rc.dyg[j + 1]) -
-             vz0 * wy0;
-    }
-    {
-        const T b = h * (W(i, j, k - 1) + W(i, j, k));
-        const T nu_z1 = nu + nt(i, j, k);
-        fw = T(2) * (nu_z1 * (W(i, j, k) - W(i, j, k - 1)) * rc.dz[k]) - b * b;
-    }
 }
 
 // one right-hand side into its slot
@@ -364,17 +295,6 @@ __global__ void k_rhs(GeoT<T> g, RcpT<T> rc, Fld<T> U, Fld<T> V, Fld<T> W, Fld<T
     else if (COMP == 1) r = rhs_v_point<T, Fld<T>>(g, rc, U, V, W, nt, nu, Om, rot, i, j, k);
     else r = rhs_w_point<T, Fld<T>>(g, rc, U, V, W, nt, nu, ds_dpdz<T>(ds), i, j, k);
     out(i, j, k) = r;
-}
-
-static RkCoef rk_coefs() {
-    RkCoef c = {};
-    c.c[1][1] = 8.0 / 15.0;
-    c.c[2][1] = 1.0 / 4.0;
-    c.c[2][2] = 5.0 / 12.0;
-    c.c[3][1] = 1.0 / 4.0;
-    c.c[3][2] = 0.0;
-    c.c[3][3] = 3.0 / 4.0;
-    return c;
 }
 
 template <typename T>
@@ -402,424 +322,6 @@ static int rhs_launch(cf_ctx *ctx, int comp, int slot) {
     return 0;
 }
 
-// ---------------------------------------------------------------------------
-// Fused right-hand sides of u, v and w with the RK update, one launch per
-// substep.  A block owns a TX x TY tile of (i, j) columns and marches along z
-// over a chunk of planes, keeping planes k-1, k, k+1 of U, V, W and nu_t (tile
-// plus one halo cell) in a shared-memory ring; the per-point formulas above
-// read them through an accessor with the Fld interface.
-// ---------------------------------------------------------------------------
-template <typename T, int TX, int TY>
-struct RingAcc {
-    static constexpr int SX = TX + 2, SY = TY + 2;
-    const T *b[3];  // planes k-1, k, k+1 of one field
-    int i0, j0, kc;
-    __device__ __forceinline__ T operator()(int i, int j, int k) const {
-        return b[k - kc + 1][(j - j0 + 1) * SX + (i - i0 + 1)];
-    }
-};
-
-// nu_t held as |S| on canonical cells and the plane coefficient C(j):
-// nu_t(i,j,k) = max(-C(jj)|S|(wrap i, jj, wrap k)/2, 0), jj = j clamped to
-// the interior, negated on the wall ghost rows for Dirichlet_nu_t
-// (subgrid.f90:521-536).  S == nullptr: read the nut field instead.
-template <typename T>
-struct NutSrc {
-    const T *S;
-    const T *C;  // 1-based rows
-    int nxp, nym, nzp, dirichlet;
-};
-
-// planes per z chunk of the fused RHS (its z spacings sit in shared memory)
-constexpr int RHS_ZMAX = RHS_ZMAX_HOST;
-// resident blocks per SM the fused RHS is compiled for.  With u, v and w
-// computed before any store, the shared-memory reads common to them are
-// issued once but more values stay live; with the per-thread index and mask
-// set-up hoisted out of the march and the substep and low words compile-time,
-// the FP32 kernel fits three blocks of 256 threads (85 registers): 24 warps
-// per SM instead of 16, 133 -> 105 us per launch at Re_tau 550.  FP64 keeps two.
-template <typename T> struct RhsMinB { static constexpr int v = sizeof(T) == 4 ? 3 : 2; };
-
-// Everything one launch of the fused right-hand side needs for one channel
-// (the grid of blocks is ntx x nty x nkc).
-template <typename T>
-struct Rhs3Args {
-    GeoT<T> g;
-    RcpT<T> rc;
-    Fld<T> U, V, W, nt;
-    NutSrc<T> ns;
-    const DevScal *ds;
-    T nu, Om, ca, cb;
-    int rot, s, kc_len, ilim, klim, ntx, nty, nkc;
-    Trio<T> out, F1, Uo, Uolo, Unlo;
-};
-
-// The RK update of one point for substep S (time_integration.f90:108-145):
-// S = 1 stores the right-hand side as F1; LO: the split path's low words
-// (u^n = hi + lo; substep 3 stores the new state as hi + lo, the others the
-// rounded sum).  o: the point's index, the same in every field of its
-// component.
-template <typename T, int S, bool LO>
-__device__ __forceinline__ void rk_apply_at(T r, T f1, T uo, T uolo, int o, T *out, T *F1, T *Unlo, T ca, T cb, T dt) {
-    T inc;
-    if constexpr (S == 1) {
-        F1[o] = r;
-        inc = dt * ca * r;
-    } else {
-        inc = dt * (ca * f1 + cb * r);
-    }
-    if constexpr (sizeof(T) == 4 && LO) {
-        float hi = uo, lo = uolo;
-        if constexpr (S == 3) {
-            ff_add(hi, lo, inc);
-            out[o] = hi;
-            Unlo[o] = lo;
-        } else {
-            out[o] = hi + (lo + inc);
-        }
-    } else {
-        out[o] = uo + inc;
-    }
-}
-
-// The tile (bx, by, bz) of one channel: a block of the single-channel launch
-// or of the ensemble launch (k_rhs3_batch below), for substep S (LO: low
-// words of u^n present).  Every per-point index is formed once per thread
-// (the (i, j) part, planes follow by adding the plane stride), the ring's
-// loads are predicated by masks fixed for the march.
-template <typename T, int TX, int TY, int S, bool LO>
-__device__ __forceinline__ void rhs3_tile(const Rhs3Args<T> &args, int bx, int by, int bz) {
-    const GeoT<T> g = args.g;
-    const RcpT<T> rc = args.rc;
-    const Fld<T> U = args.U, V = args.V, W = args.W, nt = args.nt;
-    const NutSrc<T> ns = args.ns;
-    const DevScal *const ds = args.ds;
-    const T nu = args.nu, Om = args.Om, ca = args.ca, cb = args.cb;
-    const int rot = args.rot, kc_len = args.kc_len, ilim = args.ilim, klim = args.klim;
-    const Trio<T> out = args.out, F1 = args.F1, Uo = args.Uo, Uolo = args.Uolo, Unlo = args.Unlo;
-    constexpr int SX = TX + 2, SY = TY + 2, NP = SX * SY, NT = TX * TY, NL = (NP + NT - 1) / NT;
-    __shared__ T ring[3][4][NP];  // [plane slot][field U V W nu_t][tile]
-    const int nx = g.nx, ny = g.ny, nz = g.nz, nxg = g.nxg, nyg = g.nyg, nzg = g.nzg;
-    const int i0 = 2 + bx * TX, j0 = 2 + by * TY;
-    const int kb = 2 + bz * kc_len, ke = min(kb + kc_len - 1, klim);
-    const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-    const int i = i0 + tx, j = j0 + ty;
-    const T dt = ds_dt<T>(ds), dPdx = ds_dpdx<T>(ds), dPdz = ds_dpdz<T>(ds);
-    // the tile's x and y reciprocal spacings and interpolation weights, and
-    // the chunk's z reciprocal spacings, in shared memory; gl and rcs index
-    // them with the global 1-based indices
-    __shared__ T gxs[2][TX + 3], gys[4][TY + 3], gzs[2][RHS_ZMAX + 2];
-    for (int t = threadIdx.x; t < TX + 3; t += TX * TY) {
-        const int ii = i0 - 1 + t;
-        gxs[0][t] = rc.dx[min(ii, nx + 1)];
-        gxs[1][t] = rc.dxg[min(ii, nxg + 1)];
-    }
-    for (int t = threadIdx.x; t < TY + 3; t += TX * TY) {
-        const int jj = j0 - 1 + t;
-        gys[0][t] = rc.dy[min(jj, ny + 1)];
-        gys[1][t] = rc.dyg[min(jj, nyg + 1)];
-        gys[2][t] = g.w0[min(jj, ny)];
-        gys[3][t] = g.w1[min(jj, ny)];
-    }
-    for (int t = threadIdx.x; t < ke - kb + 2; t += TX * TY) {
-        const int kk = kb + t;
-        gzs[0][t] = rc.dz[min(kk, nz + 1)];
-        gzs[1][t] = rc.dzg[min(kk, nzg + 1)];
-    }
-    GeoT<T> gl = g;
-    gl.w0 = gys[2] - (j0 - 1);
-    gl.w1 = gys[3] - (j0 - 1);
-    RcpT<T> rcs;
-    rcs.dx = gxs[0] - (i0 - 1);
-    rcs.dxg = gxs[1] - (i0 - 1);
-    rcs.dy = gys[0] - (j0 - 1);
-    rcs.dyg = gys[1] - (j0 - 1);
-    rcs.dz = gzs[0] - kb;
-    rcs.dzg = gzs[1] - kb;
-    const bool du = i <= nx - 1 && j <= nyg - 1, dv = i <= ilim && j <= ny - 1, dw = i <= ilim && j <= nyg - 1;
-    // this thread's tile elements (same for every plane and field)
-    int eia[NL], eja[NL], erem[NL];
-#pragma unroll
-    for (int q = 0; q < NL; q++) {
-        int rem = threadIdx.x + q * NT;
-        erem[q] = rem;
-        int sy = rem / SX, sx = rem - sy * SX;
-        eia[q] = i0 + sx - 1;
-        eja[q] = j0 + sy - 1;
-    }
-    // nu_t from |S|: per element the plane coefficient (with the ghost-row
-    // sign folded in; 0 outside the field) and the (i, j) part of the
-    // canonical index are fixed for the whole march
-    T ncf[NL], nsg[NL];
-    int nbase[NL];
-    const long nplane = (long)ns.nxp * ns.nym;
-    if (ns.S) {
-#pragma unroll
-        for (int q = 0; q < NL; q++) {
-            const int ia = eia[q], ja = eja[q];
-            const bool ok = erem[q] < NP && ia <= nxg && ja <= nyg;
-            const int jj = ja == 1 ? 2 : (ja == nyg ? nyg - 1 : ja);
-            nsg[q] = ok ? ((jj != ja && ns.dirichlet) ? T(-1) : T(1)) : T(0);
-            ncf[q] = ok ? T(-0.5) * ns.C[jj] : T(0);
-            nbase[q] = ok ? (wrapn(ia, ns.nxp) - 2) + ns.nxp * (jj - 2) : 0;
-        }
-    }
-    // all loads of one plane are issued before any of them is used; the
-    // (i, j) part of every element's index and its in-field mask are fixed
-    int oU[NL], oV[NL], oW[NL], oN[NL];
-    bool mU[NL], mV[NL], mW[NL], mN[NL];
-#pragma unroll
-    for (int q = 0; q < NL; q++) {
-        const int ia = eia[q], ja = eja[q];
-        const bool in = erem[q] < NP;
-        mU[q] = in && ia <= nx && ja <= nyg;
-        mV[q] = in && ia <= nxg && ja <= ny;
-        mW[q] = in && ia <= nxg && ja <= nyg;
-        mN[q] = ns.S ? nsg[q] != T(0) : mW[q];
-        oU[q] = mU[q] ? U.idx(ia, ja, 0) : 0;
-        oV[q] = mV[q] ? V.idx(ia, ja, 0) : 0;
-        oW[q] = mW[q] ? W.idx(ia, ja, 0) : 0;
-        oN[q] = ns.S ? nbase[q] : (mW[q] ? nt.idx(ia, ja, 0) : 0);
-    }
-    T pre[4][NL];
-    auto fetch = [&](int k) {
-        const bool kz = k <= nzg, kw = k <= nz;
-        const int koff = ns.S ? (int)(nplane * (wrapn(k, ns.nzp) - 2)) : k * nt.sz;
-        const T *Np = ns.S ? ns.S : nt.p;
-#pragma unroll
-        for (int q = 0; q < NL; q++) {
-            pre[0][q] = (mU[q] && kz) ? U.p[oU[q] + k * U.sz] : T(0);
-            pre[1][q] = (mV[q] && kz) ? V.p[oV[q] + k * V.sz] : T(0);
-            pre[2][q] = (mW[q] && kw) ? W.p[oW[q] + k * W.sz] : T(0);
-            pre[3][q] = (mN[q] && kz) ? Np[oN[q] + koff] : T(0);  // |S| (formed at commit) or nu_t
-        }
-    };
-    auto commit = [&](int slot) {
-#pragma unroll
-        for (int q = 0; q < NL; q++)
-            if (erem[q] < NP) {
-#pragma unroll
-                for (int f = 0; f < 3; f++) ring[slot][f][erem[q]] = pre[f][q];
-                T n = pre[3][q];
-                if (ns.S) {
-                    // max(-C|S|/2, 0), negated on Dirichlet ghost rows (nsg = -1), 0 outside (nsg = 0)
-                    const T v = ncf[q] * n;
-                    n = nsg[q] * (v > T(0) ? v : T(0));
-                }
-                ring[slot][3][erem[q]] = n;
-            }
-    };
-    fetch(kb - 1);
-    commit(0);
-    fetch(kb);
-    commit(1);
-    fetch(kb + 1);
-    commit(2);
-    __syncthreads();
-    // the z-face fluxes below the chunk's first plane, carried up the march
-    T fzu, fzv, fzw;
-    {
-        RingAcc<T, TX, TY> aU, aV, aW, aN;
-        aU.b[0] = ring[0][0]; aU.b[1] = ring[1][0]; aU.b[2] = ring[2][0];
-        aV.b[0] = ring[0][1]; aV.b[1] = ring[1][1]; aV.b[2] = ring[2][1];
-        aW.b[0] = ring[0][2]; aW.b[1] = ring[1][2]; aW.b[2] = ring[2][2];
-        aN.b[0] = ring[0][3]; aN.b[1] = ring[1][3]; aN.b[2] = ring[2][3];
-        aU.i0 = aV.i0 = aW.i0 = aN.i0 = i0;
-        aU.j0 = aV.j0 = aW.j0 = aN.j0 = j0;
-        aU.kc = aV.kc = aW.kc = aN.kc = kb;
-        rhs_zflux_dn<T, RingAcc<T, TX, TY>>(gl, rcs, aU, aV, aW, aN, nu, i, j, kb, fzu, fzv, fzw);
-    }
-    // the ring slots of planes k-1, k, k+1 rotate at run time: one copy of
-    // the plane's code (a march unrolled by three, with compile-time slots,
-    // triples the code of this large loop body and ran 5 % slower)
-    const int bu = out.u.idx(i, j, 0), bv = out.v.idx(i, j, 0), bw = out.w.idx(i, j, 0);
-    const int szu = out.u.sz, szv = out.v.sz, szw = out.w.sz;
-    int sm1 = 0, s0 = 1, sp1 = 2;
-    for (int k = kb; k <= ke; k++) {
-        if (k + 1 <= ke) fetch(k + 2);  // in flight during this plane's work
-        // RK operands of this plane, loaded before the stencil work; every
-        // field of a component has that component's shape
-        const bool cu = du && k <= klim, cv = dv && k <= klim, cw = dw && k <= nz - 1;
-        const int iu = bu + k * szu, iv = bv + k * szv, iw = bw + k * szw;
-        T fu = T(0), fv = T(0), fw = T(0), ou = T(0), ov = T(0), ow = T(0), lu = T(0), lv = T(0), lw = T(0);
-        if (cu) { ou = Uo.u.p[iu]; if constexpr (LO) lu = Uolo.u.p[iu]; if constexpr (S > 1) fu = F1.u.p[iu]; }
-        if (cv) { ov = Uo.v.p[iv]; if constexpr (LO) lv = Uolo.v.p[iv]; if constexpr (S > 1) fv = F1.v.p[iv]; }
-        if (cw) { ow = Uo.w.p[iw]; if constexpr (LO) lw = Uolo.w.p[iw]; if constexpr (S > 1) fw = F1.w.p[iw]; }
-        RingAcc<T, TX, TY> aU, aV, aW, aN;
-        aU.b[0] = ring[sm1][0]; aU.b[1] = ring[s0][0]; aU.b[2] = ring[sp1][0];
-        aV.b[0] = ring[sm1][1]; aV.b[1] = ring[s0][1]; aV.b[2] = ring[sp1][1];
-        aW.b[0] = ring[sm1][2]; aW.b[1] = ring[s0][2]; aW.b[2] = ring[sp1][2];
-        aN.b[0] = ring[sm1][3]; aN.b[1] = ring[s0][3]; aN.b[2] = ring[sp1][3];
-        aU.i0 = aV.i0 = aW.i0 = aN.i0 = i0;
-        aU.j0 = aV.j0 = aW.j0 = aN.j0 = j0;
-        aU.kc = aV.kc = aW.kc = aN.kc = k;
-        // the three right-hand sides first, every thread (the ring holds the
-        // tile and its halo, so the reads stay inside it; points outside the
-        // field are not stored): with no store between them the shared-memory
-        // reads common to u, v and w are issued once
-        const T ru = rhs_u_point<T, RingAcc<T, TX, TY>, RcpT<T>, true>(gl, rcs, aU, aV, aW, aN, nu, dPdx, Om, rot, i,
-                                                                          j, k, &fzu);
-        const T rv = rhs_v_point<T, RingAcc<T, TX, TY>, RcpT<T>, true>(gl, rcs, aU, aV, aW, aN, nu, Om, rot, i, j, k,
-                                                                          &fzv);
-        const T rw = rhs_w_point<T, RingAcc<T, TX, TY>, RcpT<T>, true>(gl, rcs, aU, aV, aW, aN, nu, dPdz, i, j, k,
-                                                                          &fzw);
-        if (cu) rk_apply_at<T, S, LO>(ru, fu, ou, lu, iu, out.u.p, F1.u.p, Unlo.u.p, ca, cb, dt);
-        if (cv) rk_apply_at<T, S, LO>(rv, fv, ov, lv, iv, out.v.p, F1.v.p, Unlo.v.p, ca, cb, dt);
-        if (cw) rk_apply_at<T, S, LO>(rw, fw, ow, lw, iw, out.w.p, F1.w.p, Unlo.w.p, ca, cb, dt);
-        __syncthreads();            // plane k-1 no longer read
-        if (k + 1 <= ke) commit(sm1);  // plane k+2 into the freed slot
-        __syncthreads();
-        const int t0 = sm1;
-        sm1 = s0;
-        s0 = sp1;
-        sp1 = t0;
-    }
-}
-
-template <typename T, int TX, int TY, int S, bool LO>
-__global__ void __launch_bounds__(TX *TY, RhsMinB<T>::v) k_rhs3(const __grid_constant__ Rhs3Args<T> a) {
-    rhs3_tile<T, TX, TY, S, LO>(a, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-// One launch over the tiles of several channels (an ensemble): member m owns
-// blocks first[m] .. first[m+1]-1, in the order of its own launch's grid.
-template <typename T>
-struct Rhs3Batch {
-    int n;
-    int first[CF_ENS_MAXM + 1];
-    Rhs3Args<T> a[CF_ENS_MAXM];
-};
-
-template <typename T, int TX, int TY, int S, bool LO>
-__global__ void __launch_bounds__(TX *TY, RhsMinB<T>::v) k_rhs3_batch(const __grid_constant__ Rhs3Batch<T> B) {
-    const int bid = blockIdx.x;
-    int m = 0;
-    while (m + 1 < B.n && bid >= B.first[m + 1]) m++;
-    const int l = bid - B.first[m], ntx = B.a[m].ntx, nty = B.a[m].nty;
-    rhs3_tile<T, TX, TY, S, LO>(B.a[m], l % ntx, (l / ntx) % nty, l / (ntx * nty));
-}
-
-template <typename T>
-static Rhs3Args<T> rhs3_args(cf_ctx *ctx, int s, int src, int dst) {
-    constexpr int TX = 32, TY = 8;
-    Rhs3Args<T> A;
-    GeoT<T> g = geo_of<T>(ctx);
-    Fld<T> U = make_fld<T>(ctx->U[src], ctx->nx, ctx->nyg);
-    Fld<T> V = make_fld<T>(ctx->V[src], ctx->nxg, ctx->ny);
-    Fld<T> W = make_fld<T>(ctx->W[src], ctx->nxg, ctx->nyg);
-    Fld<T> nt = make_fld<T>(ctx->nut, ctx->nxg, ctx->nyg);
-    auto trio = [&](void *a, void *b, void *c) {
-        Trio<T> t;
-        t.u = make_fld<T>(a, ctx->nx, ctx->nyg);
-        t.v = make_fld<T>(b, ctx->nxg, ctx->ny);
-        t.w = make_fld<T>(c, ctx->nxg, ctx->nyg);
-        return t;
-    };
-    const int o = ctx->old;
-    Trio<T> out = trio(ctx->U[dst], ctx->V[dst], ctx->W[dst]);
-    Trio<T> F1 = trio(ctx->F[0][0], ctx->F[0][1], ctx->F[0][2]);
-    Trio<T> Uo = trio(ctx->U[o], ctx->V[o], ctx->W[o]);
-    Trio<T> Uolo = trio(ctx->Ulo[o], ctx->Vlo[o], ctx->Wlo[o]);
-    Trio<T> Unlo = s == 3 ? trio(ctx->Ulo[dst], ctx->Vlo[dst], ctx->Wlo[dst]) : trio(nullptr, nullptr, nullptr);
-    // canonical cells only (i <= nxp+1, k <= nzp+1): the periodic duplicate
-    // column of V, W and plane of U, V are rewritten by the boundary
-    // conditions after the projection and read by nothing before them (the
-    // divergence takes canonical cells only)
-    const int ilim = ctx->nxp + 1, klim = ctx->nzp + 1;
-    int ntx = cdiv(ilim - 1, TX), nty = cdiv(ctx->nyg - 2, TY);
-    int nkc = std::max(ctx->rhs_nkc > 0 ? ctx->rhs_nkc : 1, cdiv(ctx->nzp, RHS_ZMAX));
-    int kc_len = cdiv(klim - 1, nkc);
-    const RkCoef rk = rk_coefs();  // F1 and r weights of substep s, rounded to T
-    NutSrc<T> ns = {};
-    if (ctx->nut_lazy) {
-        ns.S = (const T *)ctx->dsm_q + 15 * ctx->nCan;  // |S| slot of the canonical scratch
-        ns.C = sizeof(T) == 8 ? (const T *)ctx->avg_nu_t : (const T *)(ctx->avg_nu_t + ctx->nyg + 2);
-        ns.nxp = ctx->nxp;
-        ns.nym = ctx->nym;
-        ns.nzp = ctx->nzp;
-        ns.dirichlet = ctx->prm.Dirichlet_nu_t == 1;
-    }
-    A.g = g;
-    A.rc = rcp_of<T>(ctx);
-    A.U = U; A.V = V; A.W = W; A.nt = nt;
-    A.ns = ns;
-    A.ds = ctx->ds;
-    A.nu = (T)ctx->prm.nu;
-    A.Om = (T)ctx->omega_z;
-    A.rot = fabs(ctx->omega_z) > 1e-6 ? 1 : 0;
-    A.out = out; A.F1 = F1; A.Uo = Uo; A.Uolo = Uolo; A.Unlo = Unlo;
-    A.s = s;
-    A.ca = T(s == 1 ? rk.c[1][1] : (s == 2 ? rk.c[2][1] : rk.c[3][1]));
-    A.cb = T(s == 1 ? 0.0 : (s == 2 ? rk.c[2][2] : rk.c[3][3]));
-    A.kc_len = kc_len;
-    A.ilim = ilim;
-    A.klim = klim;
-    A.ntx = ntx;
-    A.nty = nty;
-    A.nkc = cdiv(klim - 1, kc_len);
-    return A;
-}
-
-template <typename T>
-int launch_rhs3(cf_ctx *ctx, int s, int src, int dst) {
-    constexpr int TX = 32, TY = 8;
-    const Rhs3Args<T> A = rhs3_args<T>(ctx, s, src, dst);
-    const dim3 grd(A.ntx, A.nty, A.nkc);
-    const bool lo = sizeof(T) == 4 && A.Uolo.u.p != nullptr;
-#define CF_RHS3(SS, LL) k_rhs3<T, TX, TY, SS, LL><<<grd, TX * TY, 0, ctx->st>>>(A)
-    if constexpr (sizeof(T) == 4) {
-        if (lo) {
-            if (s == 1) CF_RHS3(1, true); else if (s == 2) CF_RHS3(2, true); else CF_RHS3(3, true);
-        }
-    }
-    if (!lo) {
-        if (s == 1) CF_RHS3(1, false); else if (s == 2) CF_RHS3(2, false); else CF_RHS3(3, false);
-    }
-#undef CF_RHS3
-    count_launch(ctx, "k_rhs3");
-    CF_CUDA(cudaGetLastError());
-    return 0;
-}
-
-// The fused right-hand sides + RK update of substep s of n split-path channels (state
-// buffers src[q] -> dst[q]) in one launch: per channel exactly the
-// arithmetic of launch_rhs3.
-template <typename T>
-int launch_rhs3_batch(cudaStream_t st, cf_ctx *const *m, int s, const int *src, const int *dst, int n) {
-    constexpr int TX = 32, TY = 8;
-    if (n < 1 || n > CF_ENS_MAXM) return CF_ERR_INVALID;
-    Rhs3Batch<T> B;
-    B.n = n;
-    B.first[0] = 0;
-    for (int q = 0; q < n; q++) {
-        B.a[q] = rhs3_args<T>(m[q], s, src[q], dst[q]);
-        B.first[q + 1] = B.first[q] + B.a[q].ntx * B.a[q].nty * B.a[q].nkc;
-    }
-    // one variant for all members: the substep is common, the low words
-    // must be too
-    const bool lo = sizeof(T) == 4 && B.a[0].Uolo.u.p != nullptr;
-    for (int q = 1; q < n; q++)
-        if ((sizeof(T) == 4 && B.a[q].Uolo.u.p != nullptr) != lo) return CF_ERR_INVALID;
-#define CF_RHS3B(SS, LL) k_rhs3_batch<T, TX, TY, SS, LL><<<B.first[n], TX * TY, 0, st>>>(B)
-    if constexpr (sizeof(T) == 4) {
-        if (lo) {
-            if (s == 1) CF_RHS3B(1, true); else if (s == 2) CF_RHS3B(2, true); else CF_RHS3B(3, true);
-        }
-    }
-    if (!lo) {
-        if (s == 1) CF_RHS3B(1, false); else if (s == 2) CF_RHS3B(2, false); else CF_RHS3B(3, false);
-    }
-#undef CF_RHS3B
-    return cudaGetLastError() == cudaSuccess ? 0 : CF_ERR_CUDA;
-}
-
-// resident fused-RHS blocks per SM (for the z-chunk plan)
-int rhs3_blocks_per_sm() {
-    int n = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_rhs3<float, 32, 8, 2, true>, 256, 0);
-    return n < 1 ? 1 : n;
-}
-
 template <typename T>
 int launch_rhs(cf_ctx *ctx, int comp, int slot) {
     if constexpr (sizeof(T) == 8) {
@@ -837,7 +339,7 @@ int launch_rhs_update(cf_ctx *ctx, int s, int src, int dst) {
         count_launch(ctx, "k_rhs64");
         return 0;
     } else {
-        return launch_rhs3<T>(ctx, s, src, dst);
+        return launch_rhs32(ctx, s, src, dst);
     }
 }
 
@@ -1458,4 +960,3 @@ int launch_div_check(cf_ctx *ctx, int b, double *d_out) {
     template int launch_div_check<T>(cf_ctx *, int, double *);
 INST(double)
 INST(float)
-template int launch_rhs3_batch<float>(cudaStream_t, cf_ctx *const *, int, const int *, const int *, int);

@@ -46,18 +46,13 @@
 #include <algorithm>
 
 #include "cf_internal.cuh"
+#include "f32x2.cuh"
 
 namespace {
 
 constexpr int D32_T = 128;  // threads per block
 constexpr int D32_NB = 3;   // planes of a tile in shared memory: two on their way, one worked on
 
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ float2 sp(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, sp(-1.f), a); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 // the test filter in one direction over its weight 1/6; a one-sided end
 // (2/3, 1/3) is the inner neighbour taken twice
 __device__ __forceinline__ float2 wf(float2 a, float2 b, float2 c) { return fma2(sp(4.f), b, add2(a, c)); }
@@ -91,15 +86,6 @@ constexpr float SC_M = float(4.0 * FS / 256.0);   // 4 |Sf| Sf_ij
 constexpr float SC_A = 0.00212636287f, SC_B = 0.00212622364f;  // (sum of two faces' Uf)^2
 constexpr float SC_P = float(65536.0 * FS * FS);  // partials
 
-template <int B>
-__device__ __forceinline__ void copy_async(float *sm, const float *gm) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(sm);
-    if constexpr (B == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gm) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(gm), "n"(B) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(D32_NB - 2) : "memory"); }
-
 // canonical arrays of dsm_q, n apart: centre velocities, |S| S_ij, |S| (slot
 // 15, where every reader of the lazily formed nu_t expects it); slots 9-14:
 // Uf, Vf, Wf as [k][row][nxp] with rows 1..nyg (V: ny), then their one-sided
@@ -123,18 +109,6 @@ __device__ __forceinline__ float2 s_mag(float2 d0, float2 d1, float2 d2, float2 
     // unlike sqrtf without a branch, which would part the march's body
     const float2 e = f2(rsqrtf(fmaxf(y.x, 1e-37f)), rsqrtf(fmaxf(y.y, 1e-37f))), r = mul2(y, e);
     return fma2(fma2(mul2(r, sp(-1.f)), r, y), mul2(e, sp(0.5f)), r);
-}
-
-// columns i-1, i, i+1, i+2 of one row as two pairs
-struct Quad {
-    float2 p, q;
-    __device__ __forceinline__ float2 c() const { return f2(p.y, q.x); }  // columns i, i+1
-};
-__device__ __forceinline__ Quad quad(const float *s) {
-    Quad r;
-    r.p = *(const float2 *)s;
-    r.q = *(const float2 *)(s + 2);
-    return r;
 }
 
 // strain rates of two cells in the march: what plane p of the velocities
@@ -180,17 +154,9 @@ __device__ __forceinline__ void strain_plane(Strain &s, const SGeo &g, const Qua
     s.y = y;
 }
 
-// tile of the first kernel: R rows of 2 LS columns and one halo cell
+// tile of the first kernel
 template <int LS>
-struct QTile {
-    static constexpr int WS = 2 * LS, R = D32_T / LS, SX = WS + 2, SY = R + 2, NP = SX * SY, NL = (NP + D32_T - 1) / D32_T;
-    // the thread's row: with LS = 8 the two rows that half a warp reads at
-    // once are 8 apart, 8 SX = 144 words or 16 banks
-    static __device__ __forceinline__ int row() {
-        const int t = threadIdx.x / LS;
-        return LS == 8 ? (t & 1) * 8 + (t >> 1) : t;
-    }
-};
+using QTile = HaloTile<LS, D32_T>;
 
 // A block's march.  The loop's body has no branch but the one around the
 // copies, so that the strain rates' chain and the filters are interleaved:
@@ -278,7 +244,7 @@ __device__ __forceinline__ void q_march(const D32 &a, float (*st)[3][QTile<LS>::
     for (int d = 0; d < D32_NB - 1; d++) fetch(kb - 1 + d, d);
     float dzg = 0.f, dzw = 0.f;
     for (int p = kb - 1, b = 0; p <= ke + 1; p++, b = b + 1 == D32_NB ? 0 : b + 1) {
-        copy_wait();
+        copy_wait<D32_NB - 2>();
         __syncthreads();  // plane p is in; the buffer of p-1 is no longer read
         const int bn = b == 0 ? D32_NB - 1 : b - 1;
         if (p + D32_NB - 1 <= ke + 1) fetch(p + D32_NB - 1, bn);
@@ -450,7 +416,7 @@ __global__ void __launch_bounds__(D32_T, 3) k_dsm32_lm(const __grid_constant__ D
     for (int d = 0; d < D32_NB - 1; d++) fetch(kb - 1 + d, d);
     float dzg = 0.f, dzw = 0.f;
     for (int r = kb - 1, b = 0; r <= ke + 1; r++, b = b + 1 == D32_NB ? 0 : b + 1) {
-        copy_wait();
+        copy_wait<D32_NB - 2>();
         __syncthreads();  // plane r is in; the buffer of r-1 is no longer read
         const int bn = b == 0 ? D32_NB - 1 : b - 1;
         if (r + D32_NB - 1 <= ke + 1) fetch(r + D32_NB - 1, bn);
@@ -557,15 +523,6 @@ __global__ void __launch_bounds__(D32_T, 3) k_dsm32_lm(const __grid_constant__ D
     }
 }
 
-// lanes per tile row: the width that leaves the fewest idle columns, the
-// widest of them
-int d32_ls(int nxp) {
-    int best = 32;
-    for (int ls : {16, 8})
-        if (cdiv(nxp, 2 * ls) * ls < cdiv(nxp, 2 * best) * best) best = ls;
-    return best;
-}
-
 template <int LS>
 int lm_blocks_per_sm(int nxp) {
     int per = 1;
@@ -602,7 +559,7 @@ int dsm32_setup() {
 // (waves of resident blocks of the filter kernel) x (planes per chunk + 1.5
 // for the halo planes)
 void dsm32_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
-    const int ls = d32_ls(nxp), ntx = cdiv(nxp, 2 * ls);
+    const int ls = tile_lanes(nxp), ntx = cdiv(nxp, 2 * ls);
     const int per = ls == 32 ? lm_blocks_per_sm<32>(nxp) : (ls == 16 ? lm_blocks_per_sm<16>(nxp) : lm_blocks_per_sm<8>(nxp));
     const long blocks = (long)ntx * cdiv(nym, D32_T / ls), res = (long)per * sms;
     double best_cost = 1e300;
@@ -619,7 +576,7 @@ void dsm32_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
     *nchunk = (size_t)ntx * cdiv(nzp, best);
 }
 
-int dsm32_slots(int nxp, int nzp, int kc) { return cdiv(nxp, 2 * d32_ls(nxp)) * cdiv(nzp, kc); }
+int dsm32_slots(int nxp, int nzp, int kc) { return cdiv(nxp, 2 * tile_lanes(nxp)) * cdiv(nzp, kc); }
 
 // |S| into the canonical scratch, the plane partials into dsm_part
 int launch_dsm32(cf_ctx *ctx, int b, int *nchunk) {
@@ -640,7 +597,7 @@ int launch_dsm32(cf_ctx *ctx, int b, int *nchunk) {
     a.part = (float4 *)ctx->dsm_part;
     a.ny = ctx->ny; a.nz = ctx->nz; a.nyg = ctx->nyg;
     a.nxp = ctx->nxp; a.nym = ctx->nym; a.nzp = ctx->nzp;
-    const int ls = d32_ls(ctx->nxp);
+    const int ls = tile_lanes(ctx->nxp);
     a.ntx = cdiv(ctx->nxp, 2 * ls);
     a.kc_len = ctx->dsm_kc;
     a.nkc = cdiv(ctx->nzp, ctx->dsm_kc);
