@@ -345,6 +345,9 @@ template <typename T> int launch_pressure(cf_ctx *ctx, int buf);  // actual pres
 template <typename T> int launch_amd(cf_ctx *ctx, int buf);  // AMD eddy viscosity (subgrid.f90:639)
 void amd_plan(int esz, int nxp, int nym, int nzp, int sms, int *nkc, int *nparts);  // z chunks of the AMD pass
 int launch_avg_nu_t_flush(cf_ctx *ctx);  // AMD plane means of the last pass, if not formed yet
+int launch_amd32(cf_ctx *ctx, int buf);       // the split path's pass
+int amd32_plan(int nxp, int nym, int nzp, int sms);
+int amd32_parts(int nxp, int nzp, int nkc);
 int amd_partials_for(cf_ctx *ctx, int nkc);  // plane partials per row of an AMD pass with nkc z chunks
 constexpr int RHS_ZMAX_HOST = 256;           // planes per z chunk of the fused RHS at most
 template <typename T> int launch_div_check(cf_ctx *ctx, int buf, double *d_out);

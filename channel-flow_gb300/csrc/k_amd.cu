@@ -1,5 +1,5 @@
 // k_amd.cu -- anisotropic minimum dissipation eddy viscosity,
-// subgrid.f90:639-881, in one pass.
+// subgrid.f90:639-881, in one pass (FP64; the split path's is in k_amd32.cu).
 //
 // The reference builds the model from whole-array and array-section
 // operations on the temporaries term, term_1..term_4 (squared or plain
@@ -15,30 +15,36 @@
 // positions that copy it.
 //
 // A block owns a TX x TY tile of (i, j) columns and marches along z over a
-// chunk of planes with planes k-1, k, k+1 of U, V, W (tile plus one halo
-// cell) in a shared-memory ring, like the fused right-hand side.
+// chunk of planes with planes k, k+1 of U, V, W (tile plus one halo cell) in
+// a shared-memory ring of three, the third being filled; what a cell takes
+// from plane k-1 is carried up the march.
 #include "cf_internal.cuh"
 
 namespace {
 
 constexpr int AMD_TX = 32, AMD_TY = 8;
 
-template <typename T>
 struct AmdRing {
     static constexpr int SX = AMD_TX + 2;
-    const T *b[3];  // planes k-1, k, k+1
+    const double *b[2];  // planes k, k+1
     int i0, j0, kc;
-    __device__ __forceinline__ T operator()(int i, int j, int k) const {
-        return b[k - kc + 1][(j - j0 + 1) * SX + (i - i0 + 1)];
+    __device__ __forceinline__ double operator()(int i, int j, int k) const {
+        return b[k - kc][(j - j0 + 1) * SX + (i - i0 + 1)];
     }
+};
+
+// What a cell takes from the plane below: sums and sums of squares of the z
+// differences of U and V through the face below it, W there and its x and y
+// differences.
+struct AmdCarry {
+    double puz, quz, pvz, qvz, w, wx[2], wy[2];
 };
 
 // Reciprocal spacings of one column and plane and their squares: faces (x, y,
 // z: the cell's own spacing) and centres on its two sides (g0 below, g1 above).
-template <typename T>
 struct AmdGeo {
-    T x, y, z, xg[2], yg[2], zg[2];
-    T x2, y2, z2, xg2[2], yg2[2], zg2[2];
+    double x, y, z, xg[2], yg[2], zg[2];
+    double x2, y2, z2, xg2[2], yg2[2], zg2[2];
 };
 
 // -C num/den at one canonical centre (subgrid.f90:658-868), clipped with
@@ -60,26 +66,39 @@ struct AmdGeo {
 // reciprocals formed once (54 of them per cell: as FP64 divisions they were
 // three quarters of the FP64 instructions, and FP64 instructions are what
 // the FP64 pass is bound by).
-template <typename T, typename A>
-__device__ __forceinline__ T amd_point(const AmdGeo<T> &g, const A &U, const A &V, const A &W, int i, int j, int k) {
-    const T q4 = T(0.25), two = T(2);
-    const T ux = U(i, j, k) - U(i - 1, j, k);
-    const T vy = V(i, j, k) - V(i, j - 1, k);
-    const T wz = W(i, j, k) - W(i, j, k - 1);
-    // sums and sums of squares of the two differences of each side
-    T puy[2], puz[2], pvx[2], pvz[2], pwx[2], pwy[2], quy[2], quz[2], qvx[2], qvz[2], qwx[2], qwy[2];
-    auto pair = [](T a, T b, T &p, T &q) {
-        p = a + b;
-        q = a * a + b * b;
-    };
+__device__ __forceinline__ void amd_pair(double a, double b, double &p, double &q) {
+    p = a + b;
+    q = a * a + b * b;
+}
+// the carry for plane k + 1
+__device__ __forceinline__ void amd_carry(const AmdRing &U, const AmdRing &V, const AmdRing &W, int i, int j, int k, AmdCarry &c) {
+    amd_pair(U(i - 1, j, k + 1) - U(i - 1, j, k), U(i, j, k + 1) - U(i, j, k), c.puz, c.quz);
+    amd_pair(V(i, j - 1, k + 1) - V(i, j - 1, k), V(i, j, k + 1) - V(i, j, k), c.pvz, c.qvz);
+    c.w = W(i, j, k);
 #pragma unroll
     for (int s = 0; s < 2; s++) {
-        pair(U(i - 1, j + s, k) - U(i - 1, j + s - 1, k), U(i, j + s, k) - U(i, j + s - 1, k), puy[s], quy[s]);
-        pair(U(i - 1, j, k + s) - U(i - 1, j, k + s - 1), U(i, j, k + s) - U(i, j, k + s - 1), puz[s], quz[s]);
-        pair(V(i + s, j - 1, k) - V(i + s - 1, j - 1, k), V(i + s, j, k) - V(i + s - 1, j, k), pvx[s], qvx[s]);
-        pair(V(i, j - 1, k + s) - V(i, j - 1, k + s - 1), V(i, j, k + s) - V(i, j, k + s - 1), pvz[s], qvz[s]);
-        pair(W(i + s, j, k - 1) - W(i + s - 1, j, k - 1), W(i + s, j, k) - W(i + s - 1, j, k), pwx[s], qwx[s]);
-        pair(W(i, j + s, k - 1) - W(i, j + s - 1, k - 1), W(i, j + s, k) - W(i, j + s - 1, k), pwy[s], qwy[s]);
+        c.wx[s] = W(i + s, j, k) - W(i + s - 1, j, k);
+        c.wy[s] = W(i, j + s, k) - W(i, j + s - 1, k);
+    }
+}
+__device__ __forceinline__ double amd_point(const AmdGeo &g, const AmdRing &U, const AmdRing &V, const AmdRing &W, AmdCarry &c,
+                                            int i, int j, int k) {
+    typedef double T;
+    const T q4 = T(0.25), two = T(2);
+    const AmdCarry m = c;
+    amd_carry(U, V, W, i, j, k, c);
+    const T ux = U(i, j, k) - U(i - 1, j, k);
+    const T vy = V(i, j, k) - V(i, j - 1, k);
+    const T wz = c.w - m.w;
+    // sums and sums of squares of the two differences of each side
+    T puy[2], pvx[2], pwx[2], pwy[2], quy[2], qvx[2], qwx[2], qwy[2];
+    const T puz[2] = {m.puz, c.puz}, quz[2] = {m.quz, c.quz}, pvz[2] = {m.pvz, c.pvz}, qvz[2] = {m.qvz, c.qvz};
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        amd_pair(U(i - 1, j + s, k) - U(i - 1, j + s - 1, k), U(i, j + s, k) - U(i, j + s - 1, k), puy[s], quy[s]);
+        amd_pair(V(i + s, j - 1, k) - V(i + s - 1, j - 1, k), V(i + s, j, k) - V(i + s - 1, j, k), pvx[s], qvx[s]);
+        amd_pair(m.wx[s], c.wx[s], pwx[s], qwx[s]);
+        amd_pair(m.wy[s], c.wy[s], pwy[s], qwy[s]);
     }
     const T ux2 = ux * ux, vy2 = vy * vy, wz2 = wz * wz;
     T den = quy[0] * g.yg2[0] + quy[1] * g.yg2[1] + quz[0] * g.zg2[0] + quz[1] * g.zg2[1] + qvx[0] * g.xg2[0] +
@@ -103,16 +122,14 @@ __device__ __forceinline__ T amd_point(const AmdGeo<T> &g, const A &U, const A &
     return v > T(0) ? v : T(0);
 }
 
-template <typename T> struct AmdMinB { static constexpr int v = 2; };
-
 // nu_t at the canonical cells and at every duplicate / ghost position that
 // the periodic copies (boundary_conditions.f90:87-244) and the wall rule
 // (subgrid.f90:866-876) fill from them; one partial sum of the canonical
 // values per (row j, block) for avg_nu_t (subgrid.f90:877-879).
-template <typename T>
-__global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g, RcpT<T> rc, Fld<T> U, Fld<T> V,
-                                                                      Fld<T> W, Fld<T> nt, int wall_rule,
-                                                                      const DevScal *ds, double *part, int kc_len) {
+__global__ void __launch_bounds__(AMD_TX *AMD_TY, 2) k_amd(GeoT<double> g, RcpT<double> rc, Fld<double> U, Fld<double> V,
+                                                            Fld<double> W, Fld<double> nt, int wall_rule,
+                                                            const DevScal *ds, double *part, int kc_len) {
+    typedef double T;
     constexpr int TX = AMD_TX, TY = AMD_TY, SX = TX + 2, SY = TY + 2, NP = SX * SY, NT = TX * TY;
     constexpr int NL = (NP + NT - 1) / NT;
     __shared__ T ring[3][3][NP];  // [plane slot][field U V W][tile]
@@ -124,7 +141,7 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
     const bool on = i <= nxp + 1 && j <= nyg - 1;
     // this column's reciprocal spacings (the last entries of the tables stand
     // in for columns and rows past the field, whose results are not stored)
-    AmdGeo<T> ag;
+    AmdGeo ag;
     {
         const int ii = min(i, nx - 1), jj = min(j, nyg - 1);
         ag.x = rc.dx[ii];
@@ -179,11 +196,14 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
     fetch(kb + 1);
     commit(2);
     __syncthreads();
+    AmdCarry carry = {};
+    if (on) amd_carry({{ring[0][0], ring[1][0]}, i0, j0, kb - 1}, {{ring[0][1], ring[1][1]}, i0, j0, kb - 1},
+                      {{ring[0][2], ring[1][2]}, i0, j0, kb - 1}, i, j, kb - 1, carry);
+    __syncthreads();  // plane kb-1 no longer read
     // duplicate / ghost images of this column
     const int ix1 = i + nxp <= nxp + 3 ? i + nxp : 0, ix2 = i - nxp >= 1 ? i - nxp : 0;
     const int jg = j == 2 ? 1 : (j == nyg - 1 ? nyg : 0);
-    float accf = 0.f;
-    double accd = 0.0;
+    double acc = 0.0;
     int sm1 = 0, s0 = 1, sp1 = 2;
     for (int k = kb; k <= ke; k++) {
         if (k + 1 <= ke) fetch(k + 2);  // in flight during this plane's work
@@ -195,16 +215,9 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
         ag.z = rc.dz[k];
         ag.z2 = ag.z * ag.z;
         if (on) {
-            AmdRing<T> aU, aV, aW;
-            aU.b[0] = ring[sm1][0]; aU.b[1] = ring[s0][0]; aU.b[2] = ring[sp1][0];
-            aV.b[0] = ring[sm1][1]; aV.b[1] = ring[s0][1]; aV.b[2] = ring[sp1][1];
-            aW.b[0] = ring[sm1][2]; aW.b[1] = ring[s0][2]; aW.b[2] = ring[sp1][2];
-            aU.i0 = aV.i0 = aW.i0 = i0;
-            aU.j0 = aV.j0 = aW.j0 = j0;
-            aU.kc = aV.kc = aW.kc = k;
-            const T v = amd_point<T, AmdRing<T>>(ag, aU, aV, aW, i, j, k);
-            if constexpr (sizeof(T) == 8) accd += v;
-            else accf += v;
+            const T v = amd_point(ag, {{ring[s0][0], ring[sp1][0]}, i0, j0, k}, {{ring[s0][1], ring[sp1][1]}, i0, j0, k},
+                                  {{ring[s0][2], ring[sp1][2]}, i0, j0, k}, carry, i, j, k);
+            acc += v;
             const T gv = wall_rule == 0 ? v : -v + add;
             const int kz1 = k + nzp <= nzp + 3 ? k + nzp : 0, kz2 = k - nzp >= 1 ? k - nzp : 0;
             const int ixs[3] = {i, ix1, ix2}, kzs[3] = {k, kz1, kz2};
@@ -219,15 +232,13 @@ __global__ void __launch_bounds__(AMD_TX *AMD_TY, AmdMinB<T>::v) k_amd(GeoT<T> g
                 }
             }
         }
-        __syncthreads();               // plane k-1 no longer read
-        if (k + 1 <= ke) commit(sm1);  // plane k+2 into the freed slot
-        __syncthreads();
+        if (k + 1 <= ke) commit(sm1);  // plane k+2 into the slot of plane k-1
+        __syncthreads();               // plane k no longer read, k+2 in
         const int t0 = sm1;
         sm1 = s0;
         s0 = sp1;
         sp1 = t0;
     }
-    double acc = sizeof(T) == 8 ? accd : (double)accf;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     const int nparts = gridDim.x * gridDim.z;
@@ -257,8 +268,12 @@ __global__ void k_amd_avg(const double *part, int nparts, int nyg, double norm, 
 // blocks) x (planes per chunk + the 2 halo planes a chunk loads again)
 void amd_plan(int esz, int nxp, int nym, int nzp, int sms, int *nkc, int *nparts) {
     int per = 1;
-    if (esz == 4) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd<float>, AMD_TX * AMD_TY, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd<double>, AMD_TX * AMD_TY, 0);
+    if (esz == 4) {
+        *nkc = amd32_plan(nxp, nym, nzp, sms);
+        *nparts = amd32_parts(nxp, nzp, *nkc);
+        return;
+    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd, AMD_TX * AMD_TY, 0);
     const long tiles = (long)cdiv(nxp, AMD_TX) * cdiv(nym, AMD_TY), res = (long)(per < 1 ? 1 : per) * sms;
     long best = 1;
     double best_cost = 1e300;
@@ -278,26 +293,33 @@ void amd_plan(int esz, int nxp, int nym, int nzp, int sms, int *nkc, int *nparts
 template <typename T>
 int launch_amd(cf_ctx *ctx, int b) {
     ctx->nut_lazy = false;
-    GeoT<T> g = geo_of<T>(ctx);
-    Fld<T> U = make_fld<T>(ctx->U[b], ctx->nx, ctx->nyg);
-    Fld<T> V = make_fld<T>(ctx->V[b], ctx->nxg, ctx->ny);
-    Fld<T> W = make_fld<T>(ctx->W[b], ctx->nxg, ctx->nyg);
-    Fld<T> nt = make_fld<T>(ctx->nut, ctx->nxg, ctx->nyg);
-    const int nkc = ctx->amd_nkc, kc_len = cdiv(ctx->nzp, nkc);
-    const dim3 grd(cdiv(ctx->nxp, AMD_TX), cdiv(ctx->nym, AMD_TY), nkc);
-    k_amd<T><<<grd, AMD_TX * AMD_TY, 0, ctx->st>>>(g, rcp_of<T>(ctx), U, V, W, nt, ctx->prm.Dirichlet_nu_t, ctx->ds,
+    if constexpr (sizeof(T) == 4) {
+        if (int rc = launch_amd32(ctx, b)) return rc;
+    } else {
+        GeoT<T> g = geo_of<T>(ctx);
+        Fld<T> U = make_fld<T>(ctx->U[b], ctx->nx, ctx->nyg);
+        Fld<T> V = make_fld<T>(ctx->V[b], ctx->nxg, ctx->ny);
+        Fld<T> W = make_fld<T>(ctx->W[b], ctx->nxg, ctx->nyg);
+        Fld<T> nt = make_fld<T>(ctx->nut, ctx->nxg, ctx->nyg);
+        const int nkc = ctx->amd_nkc, kc_len = cdiv(ctx->nzp, nkc);
+        const dim3 grd(cdiv(ctx->nxp, AMD_TX), cdiv(ctx->nym, AMD_TY), nkc);
+        k_amd<<<grd, AMD_TX * AMD_TY, 0, ctx->st>>>(g, rcp_of<T>(ctx), U, V, W, nt, ctx->prm.Dirichlet_nu_t, ctx->ds,
                                                     ctx->dsm_part, kc_len);
-    count_launch(ctx, "k_amd");
+        count_launch(ctx, "k_amd");
+        CF_CUDA(cudaGetLastError());
+    }
     // nothing in the step reads avg_nu_t of the AMD model (the reference
     // marks it "not used"): the plane means are formed from the partials of
     // the last pass when they are asked for
-    ctx->amd_nparts = (int)(grd.x * grd.z);
+    ctx->amd_nparts = amd_partials_for(ctx, ctx->amd_nkc);
     ctx->amd_avg_pending = true;
-    CF_CUDA(cudaGetLastError());
     return 0;
 }
 
-int amd_partials_for(cf_ctx *ctx, int nkc) { return cdiv(ctx->nxp, AMD_TX) * cdiv(ctx->nzp, cdiv(ctx->nzp, nkc)); }
+int amd_partials_for(cf_ctx *ctx, int nkc) {
+    if (ctx->esz == 4) return amd32_parts(ctx->nxp, ctx->nzp, nkc);
+    return cdiv(ctx->nxp, AMD_TX) * cdiv(ctx->nzp, cdiv(ctx->nzp, nkc));
+}
 
 int launch_avg_nu_t_flush(cf_ctx *ctx) {
     if (!ctx->amd_avg_pending) return 0;
