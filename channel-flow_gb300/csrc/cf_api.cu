@@ -7,7 +7,7 @@
 
 #include "cf_internal.cuh"
 
-int fft_setup_attrs();
+int fft_setup_attrs(int esz, int nxp, int nzp);
 int dsm_b_setup();
 int dsm32_setup();
 int eqwm_setup();
@@ -554,7 +554,7 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
     CF_CUDA(cudaMalloc(&ctx->ds, sizeof(DevScal)));
     TRY(push_scal(ctx));
     TRY(setup_eqwm(ctx));
-    fft_setup_attrs();
+    fft_setup_attrs(ctx->esz, nxp, nzp);
     CF_CUDA(cudaStreamSynchronize(ctx->st));
     CF_CUDA(cudaGetLastError());
     return CF_OK;

@@ -45,6 +45,42 @@ def test_projection_edges(dims):
     o.close()
 
 
+# every transform length with a compile-time plan (even, factors 2, 3, 5, 16 to
+# 512), and two outside that range
+LENGTHS = sorted(a * b * c for a in (2, 4, 8, 16, 32, 64, 128, 256, 512) for b in (1, 3, 9, 27, 81, 243)
+                 for c in (1, 5, 25, 125) if 16 <= a * b * c <= 512) + [12, 540]
+
+
+@pytest.mark.parametrize("nx,nz", list(zip(LENGTHS, reversed(LENGTHS))))
+def test_projection_lengths(nx, nz):
+    """Transforms of every length in x and in z, in both precisions, with the
+    last block of lines partly full: the FP64 projection within the
+    per-routine 1e-12 of the oracle's (P within 1e-11, as above), the split
+    path's (FP32 transforms) within the 1e-5 (P 1e-3) it is held to elsewhere."""
+    import channelflow as cf
+    case = channel_case(nx + 2, 7, nz + 2)
+    o, ch = pair(case)
+    sp = cf.Channel(case["x"], case["y"], case["z"], precision=cf.PREC_SPLIT, **case["prm"])
+    sp.upload(case["U"], case["V"], case["W"])
+    o.set_scalar("dt", case["dt"])
+    o.set_scalar("rk_step", 1)
+    for d in (ch, sp):
+        d.set_scalars(dt=case["dt"], rk_step=1)
+    for d in (o, ch, sp):
+        d.apply_boundary_conditions()
+        d.compute_projection_step()
+        d.apply_boundary_conditions()
+    f, g, h = o.fields(), ch.download(), sp.download()
+    for n in ("U", "V", "W"):
+        assert_close(g[n], f[n], 1e-12, n)
+        assert_close(h[n], g[n], 1e-5, n)
+    assert_close(g["P"], f["P"], 1e-11, "P")
+    assert_close(h["P"], g["P"], 1e-3, "P")
+    ch.close()
+    sp.close()
+    o.close()
+
+
 @pytest.mark.parametrize("dims,wall,kw", [((6, 5, 6), 0, {}), ((18, 6, 8), 0, {}), ((22, 9, 34), 0, {"dirichlet": 1}),
                                           ((34, 17, 12), 0, {}), ((50, 7, 18), 0, {}), ((66, 12, 20), 0, {}),
                                           ((18, 17, 18), 3, {}), ((34, 8, 22), 3, {}), ((50, 13, 10), 3, {})])
