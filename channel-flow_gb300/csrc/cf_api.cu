@@ -495,6 +495,7 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
     {
         int dev_sms = 152;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device);
+        ctx->sms = dev_sms;
         dsm_b_setup();
         dsm32_setup();
         eqwm_setup();

@@ -219,6 +219,7 @@ struct cf_ctx {
     void *Uf = nullptr, *Vf = nullptr, *Wf = nullptr;  // filtered velocities (layout of the pass that wrote them)
     double *dsm_part = nullptr;        // plane partial sums
     double *avg_nu_t = nullptr;        // (nyg) device
+    int sms = 152;                     // of the device
     int dsm_kc = 0;                    // z-chunk length of the eddy-viscosity pass
     int dsmb_nkc = 0;                  // z chunks of the multi-pass DSM filter kernel
     // tensor map (a CUtensorMap) of the 15 filter quantities of dsm_q for the

@@ -56,6 +56,7 @@ struct D64 {
     Fld<double> U, V, W, Uf, Vf, Wf;  // state and (canonical elements of) the filtered velocities
     RcpT<double> rc;
     double *q;                        // canonical arrays, n apart
+    int ng;  // groups of components
     double *part;
     long n;
     int nx, ny, nz, nxg, nyg, nxp, nym, nzp, nseg, kc_len, nkc;
@@ -214,9 +215,12 @@ __global__ void __launch_bounds__(D64_T) k_dsm64_q(const __grid_constant__ D64 a
     }
 }
 
-template <int W>
-__global__ void __launch_bounds__(D64_T) k_dsm64_lm(const __grid_constant__ D64 a) {
-    constexpr int NQ = 12;
+// Components C0 .. C0+NC-1 of L and M (11, 22, 33, 12, 13, 23); `group` is
+// the slot of their partials among a.ng.
+template <int W, int C0, int NC>
+__device__ __forceinline__ void lm_march(const D64 &a, int group) {
+    constexpr int NQ = 2 * NC;  // filtered quantities: u_i u_j, then |S| S_ij
+    auto qid = [](int q) { return q < NC ? C0 + q : 6 + C0 + q - NC; };
     const Seg<W> sg(a.nym, 2, a.nseg);
     const int nx = a.nx, nyg = a.nyg, nxp = a.nxp, nzp = a.nzp, j = sg.j, l = sg.l;
     const int kb = 2 + blockIdx.y * a.kc_len, ke = min(kb + a.kc_len - 1, a.nz - 1);
@@ -229,7 +233,7 @@ __global__ void __launch_bounds__(D64_T) k_dsm64_lm(const __grid_constant__ D64 
     const long plane = (long)nxp * a.nym, n = a.n;
     // edge lanes of the quantities' y filter: quantity eq, side; W = 32 both
     // sides at once (lanes 0-15 left, 16-31 right), W = 16 one after the other
-    const int eq = min(l & 15, NQ - 1);
+    const int eq = qid(min(l & 15, NQ - 1));
     const int e0 = (W == 32 && l >= 16 ? iR : iL) - 2;
     const double *const EQ = a.q + (D_Q0 + eq) * n + e0 + nxp * (j - 2);
     const int eda = nxp * (ja - j), edc = nxp * (jc - j), edr = iR - iL;
@@ -271,7 +275,8 @@ __global__ void __launch_bounds__(D64_T) k_dsm64_lm(const __grid_constant__ D64 
         double H[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; q++) {
-            const double y = fma(4.0, Q[q1 + q * n], Q[qa + q * n] + Q[qc + q * n]);
+            const long qo = qid(q) * n;
+            const double y = fma(4.0, Q[q1 + qo], Q[qa + qo] + Q[qc + qo]);
             const double x = fma(4.0, y, sg.left(y, yL, q) + sg.right(y, yR, W == 32 ? 16 + q : q));
             H[q] = fma(4.0, h1[q], h0[q] + x);
             h0[q] = h1[q];
@@ -297,17 +302,17 @@ __global__ void __launch_bounds__(D64_T) k_dsm64_lm(const __grid_constant__ D64 
                 const double t13 = p13 + du, t23 = p23 + dv;
                 const double c = s_mag(d0, d1, d2, t12, t13, t23) * (1.0 / 54.0);
                 const double fu = wrow ? hw[0] : u2l, fv = wrow ? hw[1] : v2l, fw = wrow ? hw[2] : w2o;
-                const double bu = fu * (1.0 / 216.0), bv = fv * (1.0 / 216.0), bw = fw * (1.0 / 216.0);
-                const double L0 = fma(-fu, bu, H[0]), L1 = fma(-fv, bv, H[1]), L2 = fma(-fw, bw, H[2]),
-                             L3 = fma(-fu, bv, H[3]), L4 = fma(-fu, bw, H[4]), L5 = fma(-fv, bw, H[5]);
-                const double M0 = fma(c, d0, -H[6]), M1 = fma(c, d1, -H[7]), M2 = fma(c, d2, -H[8]),
-                             M3 = fma(c, t12, -H[9]), M4 = fma(c, t13, -H[10]), M5 = fma(c, t23, -H[11]);
+                const double f[3] = {fu, fv, fw}, S[6] = {d0, d1, d2, t12, t13, t23};
                 const int reps = r - 1 == 2 ? 2 : 1;  // plane 2 stands for its duplicate too
-                for (int t = 0; t < reps; t++) {
-                    lmd = fma(L0, M0, fma(L1, M1, fma(L2, M2, lmd)));
-                    lmo = fma(L3, M3, fma(L4, M4, fma(L5, M5, lmo)));
-                    mmd = fma(M0, M0, fma(M1, M1, fma(M2, M2, mmd)));
-                    mmo = fma(M3, M3, fma(M4, M4, fma(M5, M5, mmo)));
+#pragma unroll
+                for (int q = 0; q < NC; q++) {
+                    constexpr int IA[6] = {0, 1, 2, 0, 0, 1}, IB[6] = {0, 1, 2, 1, 2, 2};
+                    const double L = fma(-f[IA[C0 + q]], f[IB[C0 + q]] * (1.0 / 216.0), H[q]), M = fma(c, S[C0 + q], -H[NC + q]);
+                    double &lm = C0 + q < 3 ? lmd : lmo, &mm = C0 + q < 3 ? mmd : mmo;
+                    for (int t = 0; t < reps; t++) {
+                        lm = fma(L, M, lm);
+                        mm = fma(M, M, mm);
+                    }
                 }
             }
             if (r <= ke) {
@@ -342,10 +347,23 @@ __global__ void __launch_bounds__(D64_T) k_dsm64_lm(const __grid_constant__ D64 
         sm += __shfl_down_sync(FULLM, sm, o, W);
     }
     if (l == 0 && sg.act) {
-        const long slot = (long)(j - 2) * (a.nseg * a.nkc) + sg.s * a.nkc + blockIdx.y;
+        const long slot = ((long)(j - 2) * (a.nseg * a.nkc) + sg.s * a.nkc + blockIdx.y) * a.ng + group;
         a.part[2 * slot] = sl;
         a.part[2 * slot + 1] = sm;
     }
+}
+
+template <int W>
+__global__ void __launch_bounds__(D64_T) k_dsm64_lm(const __grid_constant__ D64 a) {
+    lm_march<W, 0, 6>(a, 0);
+}
+// two components a warp (blockIdx.z): the strain rates of the filtered
+// velocities are formed by three warps instead of one
+template <int W>
+__global__ void __launch_bounds__(D64_T) k_dsm64_lm3(const __grid_constant__ D64 a) {
+    if (blockIdx.z == 0) lm_march<W, 0, 2>(a, 0);
+    else if (blockIdx.z == 1) lm_march<W, 2, 2>(a, 1);
+    else lm_march<W, 4, 2>(a, 2);
 }
 
 // lanes per segment: 16 where a row then has fewer idle columns (a warp
@@ -375,7 +393,8 @@ void dsm64_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
     *nchunk = (size_t)nseg * cdiv(nzp, best);
 }
 
-int dsm64_slots(int nxp, int nzp, int kc) { return cdiv(nxp, d64_w(nxp)) * cdiv(nzp, kc); }
+// (three per segment and chunk where its components are split)
+int dsm64_slots(int nxp, int nzp, int kc) { return 3 * cdiv(nxp, d64_w(nxp)) * cdiv(nzp, kc); }
 
 // |S| into the canonical scratch, the plane partials into dsm_part
 int launch_dsm64(cf_ctx *ctx, int b, int *nchunk) {
@@ -396,15 +415,26 @@ int launch_dsm64(cf_ctx *ctx, int b, int *nchunk) {
     a.nseg = cdiv(ctx->nxp, w);
     a.kc_len = ctx->dsm_kc;
     a.nkc = cdiv(ctx->nzp, ctx->dsm_kc);
-    *nchunk = a.nseg * a.nkc;
+    // Three warps for one where even so every quarter of an SM has at most one
+    // (the smallest grids): about 90 FP64 instructions a plane of the march
+    // instead of 165; 16^3 48 -> 34 us a launch (5 of them the launch).
+    const long warps = cdiv((long)a.nseg * ctx->nym, 32 / w) * (long)a.nkc;
+    a.ng = 3 * warps <= 4L * ctx->sms ? 3 : 1;
+    *nchunk = a.nseg * a.nkc * a.ng;
     if ((size_t)*nchunk > ctx->dsm_part_nch) return cf_fail(ctx, CF_ERR_INVALID, "plane-partial slots");
     const int per = (32 / w) * (D64_T / 32);
     const dim3 gq(cdiv((long)a.nseg * ctx->nyg, per), a.nkc), gl(cdiv((long)a.nseg * ctx->nym, per), a.nkc);
     if (w == 32) k_dsm64_q<32><<<gq, D64_T, 0, ctx->st>>>(a);
     else k_dsm64_q<16><<<gq, D64_T, 0, ctx->st>>>(a);
     count_launch(ctx, "k_dsm64_q");
-    if (w == 32) k_dsm64_lm<32><<<gl, D64_T, 0, ctx->st>>>(a);
-    else k_dsm64_lm<16><<<gl, D64_T, 0, ctx->st>>>(a);
+    const dim3 gl3(gl.x, gl.y, 3);
+    if (a.ng == 3) {
+        if (w == 32) k_dsm64_lm3<32><<<gl3, D64_T, 0, ctx->st>>>(a);
+        else k_dsm64_lm3<16><<<gl3, D64_T, 0, ctx->st>>>(a);
+    } else {
+        if (w == 32) k_dsm64_lm<32><<<gl, D64_T, 0, ctx->st>>>(a);
+        else k_dsm64_lm<16><<<gl, D64_T, 0, ctx->st>>>(a);
+    }
     count_launch(ctx, "k_dsm64_lm");
     CF_CUDA(cudaGetLastError());
     return 0;

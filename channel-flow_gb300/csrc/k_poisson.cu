@@ -261,15 +261,16 @@ __global__ void k_fft_z(typename C2<T>::t *spec, FftPlan pl, const typename C2<T
 
 // ---------------------------------------------------------------------------
 // Compile-time plans, for every admissible length (even, factors 2, 3, 5)
-// from 16 to 512: two Stockham stages of composite radix up to 16 (16 = 4x4,
+// from 16 to 512: two Stockham stages of composite radix up to 16 (itself 4x4;
 // 15 = 3x5, 12 = 4x3, 10 = 2x5, ...) where the length is a product of two
 // such, else three of radix up to 10, each radix-R butterfly a register DFT.
 // The first stage reads its R elements straight from the spectrum and stores
 // to shared memory, the last reads them back and stores its results straight
 // to the spectrum -- one or two shared-memory round trips per element instead
 // of one per radix-2..5 stage plus the copies in and out (90 points, 3900
-// lines, FP32: 8.3 us against 15.0 for the run-time plan).  Natural order in
-// and out.  Of the splits with the smallest radices the one whose first radix
+// lines, FP32: 8.3 us against 15.0 for the run-time plan; 16 points as 4 x 4,
+// 144 lines, FP64: 9.2 us against 17.7 as one 16-point butterfly a thread).
+// Natural order in and out.  Of the splits with the smallest radices the one whose first radix
 // is a multiple of 8, then the larger first radix; the first radix is even
 // (the x transforms' padding).
 // ---------------------------------------------------------------------------
@@ -277,7 +278,6 @@ constexpr bool fft_radix(int r, int most) {
     return r <= most && (r == 3 || r == 4 || r == 5 || r == 6 || r == 8 || r == 9 || r == 10 || r == 12 || r == 15 || r == 16);
 }
 constexpr int zr_r0(int n) {
-    if (n == 16) return 16;
     int best = 0, cost = 1 << 20;
     for (int r = 16; r >= 4 && n <= 256; r -= 2) {
         if (!fft_radix(r, 16) || n % r || !fft_radix(n / r, 16)) continue;
@@ -295,7 +295,7 @@ constexpr int zr_r1(int n) { return zr_r0(n) ? n / zr_r0(n) : 0; }
 // measured better: 32, 96 and 128 points.)
 constexpr int ZR_T = 256;  // threads per block
 constexpr int zr_lines(int n) {
-    if (zr_r1(n) <= 1) return ZR_T;
+    if (zr_r0(n) == 0) return 1;
     if (n == 32 || n == 96) return 64;
     if (n == 128) return 32;
     return ZR_T / (zr_r0(n) > zr_r1(n) ? zr_r0(n) : zr_r1(n));
@@ -366,44 +366,32 @@ __global__ void __launch_bounds__(ZR_T) k_fft_zr(typename C2<T>::t *__restrict__
     }
     for (int e = threadIdx.x; e < N; e += ZR_T) stw[e] = tw_g[e];
     __syncthreads();
-    if constexpr (R1 == 1) {
-        // one stage (N = R0): the DFT of the line, stored in natural order
+    C *bl = buf + l * LS;
 #pragma unroll
-        for (int it = 0; it < I0; it++) {
+    for (int it = 0; it < I0; it++) {
+        const int j = t + it * G;
+        if (t < G && j < NB0) {
             reg_dft<R0, N, INV>(v[it], stw);
-            if (act && t + it * G < NB0) {
 #pragma unroll
-                for (int r = 0; r < R0; r++) spec[gb + (long)r * nh] = v[it][r];
-            }
+            for (int r = 0; r < R0; r++) bl[j * R0 + r] = v[it][r];
         }
-    } else {
-        C *bl = buf + l * LS;
+    }
+    __syncthreads();
+    // second stage (Ns = R0 = NB1, so k = j, the twiddle step is 1 and
+    // output r of butterfly j goes to j + r R0)
 #pragma unroll
-        for (int it = 0; it < I0; it++) {
-            const int j = t + it * G;
-            if (t < G && j < NB0) {
-                reg_dft<R0, N, INV>(v[it], stw);
+    for (int it = 0; it < I1; it++) {
+        const int j = t + it * G;
+        if (t < G && j < NB1) {
+            C w[R1];
 #pragma unroll
-                for (int r = 0; r < R0; r++) bl[j * R0 + r] = v[it][r];
-            }
-        }
-        __syncthreads();
-        // second stage (Ns = R0 = NB1, so k = j, the twiddle step is 1 and
-        // output r of butterfly j goes to j + r R0)
+            for (int r = 0; r < R1; r++) w[r] = bl[j + r * NB1];
 #pragma unroll
-        for (int it = 0; it < I1; it++) {
-            const int j = t + it * G;
-            if (t < G && j < NB1) {
-                C w[R1];
+            for (int r = 1; r < R1; r++) w[r] = cmul(w[r], stw[r * j]);
+            reg_dft<R1, N, INV>(w, stw);
+            if (act) {
 #pragma unroll
-                for (int r = 0; r < R1; r++) w[r] = bl[j + r * NB1];
-#pragma unroll
-                for (int r = 1; r < R1; r++) w[r] = cmul(w[r], stw[r * j]);
-                reg_dft<R1, N, INV>(w, stw);
-                if (act) {
-#pragma unroll
-                    for (int r = 0; r < R1; r++) spec[gb + (long)(j + r * R0) * nh] = w[r];
-                }
+                for (int r = 0; r < R1; r++) spec[gb + (long)(j + r * R0) * nh] = w[r];
             }
         }
     }
@@ -525,7 +513,7 @@ static size_t zr3_smem() {
 
 template <typename T, int N>
 static size_t zr_smem() {
-    return zr_r1(N) > 1 ? (size_t)zr_lines(N) * (N + 1) * sizeof(typename C2<T>::t) : 0;
+    return (size_t)zr_lines(N) * (N + 1) * sizeof(typename C2<T>::t);
 }
 
 // ---------------------------------------------------------------------------
@@ -671,24 +659,22 @@ __global__ void __launch_bounds__(ZR_T) k_fwd_xr(GeoT<T> g, Fld<T> U, Fld<T> V, 
         __syncthreads();
         xr_mid_stage<N, R1, R0, LP, false>(buf, stw, p);
     }
-    if constexpr (R1 > 1) {
-        __syncthreads();
-        // last stage in place (span NSL = NBL, twiddle step 1): butterfly
-        // jb reads and writes jb + r NSL
+    __syncthreads();
+    // last stage in place (span NSL = NBL, twiddle step 1): butterfly
+    // jb reads and writes jb + r NSL
 #pragma unroll
-        for (int it = 0; it < IL; it++) {
-            const int q = p + it * ZR_T, jb = q % NBL;
-            C *ln = buf + (q / NBL) * LS;
-            if (q < LP * NBL) {
-                C w[RL];
+    for (int it = 0; it < IL; it++) {
+        const int q = p + it * ZR_T, jb = q % NBL;
+        C *ln = buf + (q / NBL) * LS;
+        if (q < LP * NBL) {
+            C w[RL];
 #pragma unroll
-                for (int r = 0; r < RL; r++) w[r] = ln[xr_pos<N>(jb + r * NSL)];
+            for (int r = 0; r < RL; r++) w[r] = ln[xr_pos<N>(jb + r * NSL)];
 #pragma unroll
-                for (int r = 1; r < RL; r++) w[r] = cmul(w[r], stw[r * jb]);
-                reg_dft<RL, N, false>(w, stw);
+            for (int r = 1; r < RL; r++) w[r] = cmul(w[r], stw[r * jb]);
+            reg_dft<RL, N, false>(w, stw);
 #pragma unroll
-                for (int r = 0; r < RL; r++) ln[xr_pos<N>(jb + r * NSL)] = w[r];
-            }
+            for (int r = 0; r < RL; r++) ln[xr_pos<N>(jb + r * NSL)] = w[r];
         }
     }
     __syncthreads();
@@ -754,55 +740,41 @@ __global__ void __launch_bounds__(ZR_T) k_inv_xr(const typename C2<T>::t *__rest
     }
     for (int e = threadIdx.x; e < N; e += ZR_T) stw[e] = tw_g[e];
     __syncthreads();
-    if constexpr (R1 == 1) {
-        int jj, kk;
-        const bool act = line(p, jj, kk);
-        T *p0 = phi + (long)N * (jj + (long)nym * kk), *p1 = phi + (long)N * (jj + (long)nym * (kk + 1));
-        reg_dft<R0, N, true>(v[0], stw);
-        if (act) {
 #pragma unroll
-            for (int r = 0; r < R0; r++) {
-                p0[r] = v[0][r].x * scale;
-                p1[r] = v[0][r].y * scale;
-            }
+    for (int it = 0; it < I0; it++) {
+        const int b = p + it * ZR_T, jb = b % NB0;
+        C *ln = buf + (b / NB0) * LS;
+        if (b < LP * NB0) {
+            reg_dft<R0, N, true>(v[it], stw);
+#pragma unroll
+            for (int r = 0; r < R0; r++) ln[xr_pos<N>(jb * R0 + r)] = v[it][r];
         }
-    } else {
-#pragma unroll
-        for (int it = 0; it < I0; it++) {
-            const int b = p + it * ZR_T, jb = b % NB0;
-            C *ln = buf + (b / NB0) * LS;
-            if (b < LP * NB0) {
-                reg_dft<R0, N, true>(v[it], stw);
-#pragma unroll
-                for (int r = 0; r < R0; r++) ln[xr_pos<N>(jb * R0 + r)] = v[it][r];
-            }
-        }
+    }
+    __syncthreads();
+    if constexpr (R2 > 1) {
+        xr_mid_stage<N, R1, R0, LP, true>(buf, stw, p);
         __syncthreads();
-        if constexpr (R2 > 1) {
-            xr_mid_stage<N, R1, R0, LP, true>(buf, stw, p);
-            __syncthreads();
-        }
-        // last stage (span NSL = NBL, twiddle step 1): phi stored directly
+    }
+    // last stage (span NSL = NBL, twiddle step 1): phi stored directly
 #pragma unroll
-        for (int it = 0; it < IL; it++) {
-            const int b = p + it * ZR_T, jb = b % NBL;
-            const C *ln = buf + (b / NBL) * LS;
-            if (b < LP * NBL) {
-                int jj, kk;
-                const bool act = line(b / NBL, jj, kk);
-                T *p0 = phi + (long)N * (jj + (long)nym * kk), *p1 = phi + (long)N * (jj + (long)nym * (kk + 1));
-                C w[RL];
+    for (int it = 0; it < IL; it++) {
+        const int b = p + it * ZR_T, jb = b % NBL;
+        const C *ln = buf + (b / NBL) * LS;
+        if (b < LP * NBL) {
+            int jj, kk;
+            const bool act = line(b / NBL, jj, kk);
+            T *p0 = phi + (long)N * (jj + (long)nym * kk), *p1 = phi + (long)N * (jj + (long)nym * (kk + 1));
+            C w[RL];
 #pragma unroll
-                for (int r = 0; r < RL; r++) w[r] = ln[xr_pos<N>(jb + r * NSL)];
+            for (int r = 0; r < RL; r++) w[r] = ln[xr_pos<N>(jb + r * NSL)];
 #pragma unroll
-                for (int r = 1; r < RL; r++) w[r] = cmul(w[r], stw[r * jb]);
-                reg_dft<RL, N, true>(w, stw);
-                if (act) {
+            for (int r = 1; r < RL; r++) w[r] = cmul(w[r], stw[r * jb]);
+            reg_dft<RL, N, true>(w, stw);
+            if (act) {
 #pragma unroll
-                    for (int r = 0; r < RL; r++) {
-                        p0[jb + r * NSL] = w[r].x * scale;
-                        p1[jb + r * NSL] = w[r].y * scale;
-                    }
+                for (int r = 0; r < RL; r++) {
+                    p0[jb + r * NSL] = w[r].x * scale;
+                    p1[jb + r * NSL] = w[r].y * scale;
                 }
             }
         }
@@ -811,7 +783,7 @@ __global__ void __launch_bounds__(ZR_T) k_inv_xr(const typename C2<T>::t *__rest
 
 template <typename T, int N>
 static size_t xr_smem() {
-    return xr_r(N, 1) > 1 ? (size_t)xr_lines(N) * xr_ls<N>() * sizeof(typename C2<T>::t) : 0;
+    return (size_t)xr_lines(N) * xr_ls<N>() * sizeof(typename C2<T>::t);
 }
 template <typename T, int N>
 static size_t xr_fwd_smem() {
