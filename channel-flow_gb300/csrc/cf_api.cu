@@ -183,6 +183,10 @@ static int setup_eqwm(cf_ctx *ctx) {
     for (int i = 1; i <= ncv + 1; i++) out[ncv + i] = fa[i];
     CF_CUDA(cudaMalloc(&ctx->eq_grid, out.size() * sizeof(double)));
     CF_CUDA(cudaMemcpy(ctx->eq_grid, out.data(), out.size() * sizeof(double), cudaMemcpyHostToDevice));
+    std::vector<double2> et(EQ_EXPN + 1);
+    for (int n = 0; n <= EQ_EXPN; n++) et[n] = make_double2(n / 32.0, std::exp(-n / 32.0));
+    CF_CUDA(cudaMalloc(&ctx->eq_exp, et.size() * sizeof(double2)));
+    CF_CUDA(cudaMemcpy(ctx->eq_exp, et.data(), et.size() * sizeof(double2), cudaMemcpyHostToDevice));
     std::vector<int> zs, xs;
     std::vector<double> zw, xw;
     stencils_2nd(ctx->hz, ctx->nz, ctx->hzg, ctx->nzg, false, zs, zw);
@@ -571,7 +575,7 @@ extern "C" int cf_destroy(cf_ctx *ctx) {
     void *ptrs[] = {ctx->nut, ctx->P, ctx->dsm_q, ctx->Uf, ctx->Vf, ctx->Wf, ctx->dsm_part, ctx->avg_nu_t,
                     ctx->phi, ctx->spec, ctx->d_tri, ctx->d_tw, ctx->tri_fac, ctx->tri_piv, ctx->tri_l32, ctx->tri_ru32,
                     ctx->tri_du32, ctx->tri_flag, ctx->tri_list, ctx->alpha_x, ctx->alpha_z, ctx->alpha_zt, ctx->tau0,
-                    ctx->wtemp1, ctx->wtemp2, ctx->eq_grid, ctx->eq_zst, ctx->eq_xst, ctx->eq_zw, ctx->eq_xw, ctx->ds,
+                    ctx->wtemp1, ctx->wtemp2, ctx->eq_grid, ctx->eq_exp, ctx->eq_zst, ctx->eq_xst, ctx->eq_zw, ctx->eq_xw, ctx->ds,
                     ctx->d_red, ctx->d_dtmin, ctx->d_mass_c, ctx->d_geo, ctx->d_geo_f, ctx->d_rgeo, ctx->d_rgeo_f, ctx->stage,
                     ctx->wm_u, ctx->wm_tau, ctx->wm_tau_eq, ctx->wm_log, ctx->wm_inside, ctx->wm_calls};
     for (void *q : ptrs)

@@ -185,6 +185,8 @@ __device__ __forceinline__ void sij_point(const GeoT<T> &g, const RcpT<T> &rc, c
 }
 
 
+constexpr int EQ_EXPN = 1280;                // last entry of the wall model's table of exponentials (x = 40)
+
 struct cf_ctx {
     int dev = 0;
     cf_params prm;
@@ -264,6 +266,7 @@ struct cf_ctx {
     int *wm_inside = nullptr, *wm_calls = nullptr;
     int wm_check_every = 0;
     double *eq_grid = nullptr;                      // y_cv(1..ncv), y_fa(1..ncv+1)
+    double2 *eq_exp = nullptr;         // (n/32, exp(-n/32)), n = 0 .. EQ_EXPN
     int *eq_zst = nullptr, *eq_xst = nullptr;       // stencil indices
     double *eq_zw = nullptr, *eq_xw = nullptr;      // stencil weights
     int n_nan = 0, n_iter = 0;

@@ -101,7 +101,7 @@ struct WmState {
 // exp(-y cd) of a pass is the last pass's value (kept per thread in shared
 // memory) times exp(-y dcd) as its Taylor polynomial where |y dcd| <= 2e-2
 // (degree 7; 4 up to 1e-3, 2 up to 1e-6: truncation below 1e-17 relative),
-// 16 FP64 instructions otherwise.
+// from a table otherwise (exp_neg).
 //
 // Split path: the Picard passes in FP32 (at most 50, until the change is below
 // 1e-5 of tau), which also give the slope of the fixed-point map, G'(tau) =
@@ -111,16 +111,35 @@ struct WmState {
 // which the first of them meets.  (Two passes and Aitken's extrapolation
 // instead needed a third FP64 pass, and a pass took a continuant recurrence
 // with seven operations a cell: 567 us per call against 340 at Re_tau 2000,
-// 258 x 258 x 2 points of 30 cells; all-FP64 4.62 ms against 2.32.)
+// 258 x 258 x 2 points of 30 cells, 295 with the table of exponentials;
+// all-FP64 4.62 ms against 2.32 and 2.16.)
 // ---------------------------------------------------------------------------
 constexpr int EQ_T = 128;                 // threads per block
+
+// exp(-x), x >= 0, by table (Tang's method): exp(-n/32) at the nearest n/32
+// times the Taylor polynomial of the rest, |r| <= 1/64 (degree 6: truncation
+// 5e-17).  About 9 FP64 instructions, the library's function 16.  Past x = 40
+// the value is below half an ulp of the 1 it is taken from: 0.
+__device__ __forceinline__ double exp_neg(double x, const double2 *__restrict__ tab) {
+    const float xf = (float)x;
+    const double2 t = __ldg(&tab[min((int)fmaf(xf, 32.f, 0.5f), EQ_EXPN)]);  // (n/32, exp(-n/32))
+    const double r = t.x - x;
+    double p = fma(r, 1.0 / 720.0, 1.0 / 120.0);
+    p = fma(r, p, 1.0 / 24.0);
+    p = fma(r, p, 1.0 / 6.0);
+    p = fma(r, p, 0.5);
+    p = fma(r, p, 1.0);
+    const double e = fma(t.y * r, p, t.y);
+    return xf > 40.f ? 0.0 : e;
+}
 constexpr size_t EQ_SMEM = 100 * 1024;    // shared memory of a block at most
 __host__ __device__ __forceinline__ int eq_grid_doubles(int ncv) { return 2 * ncv + (ncv + 1); }
 
 template <int P, bool MIXED>
 __global__ void __launch_bounds__(EQ_T) k_eq_solve(const Fld<double> Ud, const float *Uf32, int sy, int sz,
                                                    const double *t1, const int *xst, const double *xw,
-                                                   const double *grid, EqParams ep, const void *nut, int keep_ex,
+                                                   const double *grid, const double2 *etab, EqParams ep,
+                                                   const void *nut, int keep_ex,
                                                    double *tau0, double *alpha_x, double *alpha_zt, int *counters,
                                                    WmState wm) {
     extern __shared__ double sg[];
@@ -227,7 +246,7 @@ __global__ void __launch_bounds__(EQ_T) k_eq_solve(const Fld<double> Ud, const f
                 }
             };
             if (lev == 3) {
-                sweep([&](double y, int) { return exp(-(y * cd)); });
+                sweep([&](double y, int) { return exp_neg(y * cd, etab); });
             } else if (lev == 2) {
                 sweep([&](double y, int s) {
                     const double x = y * -dcd;
@@ -331,8 +350,8 @@ static void eq_launch(cf_ctx *ctx, const Fld<double> &Ud, const EqParams &ep, in
                  ex = (size_t)cdiv(ep.ncv - 1, P) * EQ_T * sizeof(double);
     const int keep = base + ex <= EQ_SMEM;
     k_eq_solve<P, MIXED><<<cdiv(npts * P, EQ_T), EQ_T, base + (keep ? ex : 0), ctx->st>>>(
-        Ud, (const float *)ctx->U[b], ep.nx, ep.nx * ep.nyg, ctx->wtemp1, ctx->eq_xst, ctx->eq_xw, ctx->eq_grid, ep,
-        ctx->nut, keep, ctx->tau0, ctx->alpha_x, ctx->alpha_zt, (int *)ctx->d_red, wm);
+        Ud, (const float *)ctx->U[b], ep.nx, ep.nx * ep.nyg, ctx->wtemp1, ctx->eq_xst, ctx->eq_xw, ctx->eq_grid, ctx->eq_exp,
+        ep, ctx->nut, keep, ctx->tau0, ctx->alpha_x, ctx->alpha_zt, (int *)ctx->d_red, wm);
 }
 
 template <bool MIXED>
