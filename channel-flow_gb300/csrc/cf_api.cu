@@ -849,9 +849,13 @@ extern "C" int cf_compute_dt(cf_ctx *ctx, double *dt) {
     return CF_OK;
 }
 
-static int eddy(cf_ctx *ctx, int b) {
+// again: not the first of a step.  Without a model only the first one sets
+// nu_t to zero: nothing else in a step writes it (eight fills of the field
+// and its row means a step were 10 % of a step at 128 x 96 x 128).
+static int eddy(cf_ctx *ctx, int b, bool again = false) {
     if (ctx->prm.LES_model == 2) return DISPATCH(launch_dsm<double>(ctx, b), launch_dsm<float>(ctx, b));
     if (ctx->prm.LES_model == 3) return DISPATCH(launch_amd<double>(ctx, b), launch_amd<float>(ctx, b));
+    if (again) return 0;
     return DISPATCH(launch_nut_zero<double>(ctx), launch_nut_zero<float>(ctx));
 }
 
@@ -1075,9 +1079,9 @@ static int enqueue_seg(cf_ctx *ctx, int seg, bool tri) {
         TRY(eddy(ctx, X));
         if (ctx->prm.iwall_model == 3) {
             TRY(wall_model(ctx, X));
-            if (ctx->prm.sgs_recompute) TRY(eddy(ctx, X));
+            if (ctx->prm.sgs_recompute) TRY(eddy(ctx, X, true));
         } else if (ctx->prm.sgs_recompute) {
-            TRY(eddy(ctx, X));
+            TRY(eddy(ctx, X, true));
         }
         // substeps 1 and 2 hold intermediate stages: the split path keeps a low
         // word only for u^n and the new state of substep 3.  The boundary
@@ -1095,7 +1099,7 @@ static int enqueue_seg(cf_ctx *ctx, int seg, bool tri) {
     if (seg == 1) {
         TRY(launch_projection<T>(ctx, a, true, false, canon, POISSON_INV, true));
         // substep 2 (:118-131)
-        TRY(eddy(ctx, a));
+        TRY(eddy(ctx, a, true));
         TRY(launch_rhs_update<T>(ctx, 2, a, b));
         ctx->cur = b;
         return launch_projection<T>(ctx, b, false, false, canon, fwd);
@@ -1103,7 +1107,7 @@ static int enqueue_seg(cf_ctx *ctx, int seg, bool tri) {
     if (seg == 2) {
         TRY(launch_projection<T>(ctx, b, false, false, canon, POISSON_INV, true));
         // substep 3 (:134-150)
-        TRY(eddy(ctx, b));
+        TRY(eddy(ctx, b, true));
         TRY(launch_rhs_update<T>(ctx, 3, b, a));
         ctx->cur = a;
         return launch_projection<T>(ctx, a, false, true, canon, fwd);
@@ -1167,13 +1171,13 @@ static int ens_pre_t(cf_ctx *ctx, int s) {
         TRY(launch_dt<T>(ctx, X, true));
         TRY(eddy(ctx, X));
         if (ctx->prm.iwall_model == 3) TRY(wall_model(ctx, X));
-        if (ctx->prm.sgs_recompute) TRY(eddy(ctx, X));
+        if (ctx->prm.sgs_recompute) TRY(eddy(ctx, X, true));
         return 0;
     }
     const int X = ctx->seg_base, a = (X + 1) % 3, b = (X + 2) % 3;
     const int p = s == 2 ? a : b;  // the state the previous substep's projection acts on
     TRY(launch_projection<T>(ctx, p, s == 2, false, canon, POISSON_INV, true));
-    return eddy(ctx, p);
+    return eddy(ctx, p, true);
 }
 
 template <typename T>
