@@ -806,26 +806,27 @@ struct TriFac {
     const unsigned char *piv;        // [nym][NM]
 };
 
-// FP64 replay, one thread per mode, 32 adjacent modes per block: a warp's
-// accesses to a row are coalesced, and the rows of the next TRI_RB are loaded
-// while the recurrence works on the current ones (a row costs one dependent
-// FP64 operation forward and two backward).  The eliminated right-hand side
-// stays in place in the spectrum.  PIV: some mode of the warp pivots; without,
-// zgtsv's elimination leaves the upper diagonal at Dyy's (duc, the same for
-// every mode), dl is zero and the flags need not be read, so that a mode and
-// row moves 80 bytes instead of 97.  Six FP64 instructions per mode and row
-// (2.4 M mode-rows at Re_tau 550: 23 us of the FP64 pipe); one lane per
-// 32-thread block running the recurrence issued as many per warp as this
-// does for 32 modes.
+// FP64 replay, two threads per mode (real and imaginary part), 16 adjacent
+// modes per block: a warp's accesses to a row are coalesced, and the rows of
+// the next TRI_RB are loaded while the recurrence works on the current ones
+// (a row costs one dependent FP64 operation forward and two backward).  The
+// eliminated right-hand side stays in place in the spectrum.  PIV: some mode
+// of the warp pivots; without, zgtsv's elimination leaves the upper diagonal
+// at Dyy's (duc, the same for every mode), dl is zero and the flags need not
+// be read, so that a mode and row moves 80 bytes instead of 97.  Three FP64
+// instructions per thread and row: with one thread for both parts the six of
+// a warp were the time where the modes do not fill the chip (2112 modes of 64
+// rows; 57 -> 47 us at 18624 modes of 128 rows, 13 -> 11 at 144 of 16).
 constexpr int TRI_RB = 8;
 
 template <bool PIV>
-__device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const TriFac &f, const double *__restrict__ duc,
-                                           int nym, long NM, long mo) {
-    double2 *const sp = spec + mo;
+__device__ __forceinline__ void tri_replay(double *__restrict__ spec, const TriFac &f, const double *__restrict__ duc,
+                                           int nym, long NM, long mo, int part) {
+    double *const sp = spec + 2 * mo + part;
+    const long NS = 2 * NM;  // row stride of the spectrum
     const double *const fm = f.m + mo, *const frd = f.rd + mo, *const fdu = f.du + mo, *const fdl = f.dl + mo;
     const unsigned char *const fp = f.piv + mo;
-    double2 nb[TRI_RB];
+    double nb[TRI_RB];
     double nm[TRI_RB];
     unsigned char np[TRI_RB];
     // rows q0+1 .. q0+TRI_RB of the right-hand side and the multipliers above them
@@ -834,16 +835,16 @@ __device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const Tri
         for (int r = 0; r < TRI_RB; r++) {
             const int q = q0 + r;
             if (q < nym - 1) {
-                nb[r] = sp[(long)(q + 1) * NM];
+                nb[r] = sp[(long)(q + 1) * NS];
                 nm[r] = fm[(long)q * NM];
                 if constexpr (PIV) np[r] = fp[(long)q * NM];
             }
         }
     };
-    double2 c = sp[0];
+    double c = sp[0];
     load_f(0);
     for (int q0 = 0; q0 < nym - 1; q0 += TRI_RB) {
-        double2 b[TRI_RB];
+        double b[TRI_RB];
         double m[TRI_RB];
         unsigned char p[TRI_RB];
 #pragma unroll
@@ -857,29 +858,27 @@ __device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const Tri
         for (int r = 0; r < TRI_RB; r++) {
             const int q = q0 + r;
             if (q < nym - 1) {
-                double2 o = c, x = b[r];
+                double o = c, x = b[r];
                 if constexpr (PIV) {
                     if (p[r]) {
                         o = b[r];
                         x = c;
                     }
                 }
-                sp[(long)q * NM] = o;
-                c.x = x.x - m[r] * o.x;
-                c.y = x.y - m[r] * o.y;
+                sp[(long)q * NS] = o;
+                c = x - m[r] * o;
             }
         }
     }
-    double rl = frd[(long)(nym - 1) * NM];
-    double2 x1 = make_double2(c.x * rl, c.y * rl), x2 = make_double2(0.0, 0.0);
-    sp[(long)(nym - 1) * NM] = x1;
+    double x1 = c * frd[(long)(nym - 1) * NM], x2 = 0.0;
+    sp[(long)(nym - 1) * NS] = x1;
     double nu[TRI_RB], nl[TRI_RB];
     auto load_b = [&](int q0) {  // rows q0, q0 - 1, ..
 #pragma unroll
         for (int r = 0; r < TRI_RB; r++) {
             const int q = q0 - r;
             if (q >= 0) {
-                nb[r] = sp[(long)q * NM];
+                nb[r] = sp[(long)q * NS];
                 nm[r] = frd[(long)q * NM];
                 if constexpr (PIV) {
                     nu[r] = fdu[(long)q * NM];
@@ -892,7 +891,7 @@ __device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const Tri
     };
     load_b(nym - 2);
     for (int q0 = nym - 2; q0 >= 0; q0 -= TRI_RB) {
-        double2 b[TRI_RB];
+        double b[TRI_RB];
         double rd[TRI_RB], du[TRI_RB], dl[TRI_RB];
 #pragma unroll
         for (int r = 0; r < TRI_RB; r++) {
@@ -906,31 +905,29 @@ __device__ __forceinline__ void tri_replay(double2 *__restrict__ spec, const Tri
         for (int r = 0; r < TRI_RB; r++) {
             const int q = q0 - r;
             if (q >= 0) {
-                double2 y;
+                double y;
                 if constexpr (PIV) {
-                    y.x = ((b[r].x - du[r] * x1.x) - dl[r] * x2.x) * rd[r];
-                    y.y = ((b[r].y - du[r] * x1.y) - dl[r] * x2.y) * rd[r];
+                    y = ((b[r] - du[r] * x1) - dl[r] * x2) * rd[r];
                     x2 = x1;
                 } else {
-                    y.x = (b[r].x - du[r] * x1.x) * rd[r];
-                    y.y = (b[r].y - du[r] * x1.y) * rd[r];
+                    y = (b[r] - du[r] * x1) * rd[r];
                 }
-                sp[(long)q * NM] = y;
+                sp[(long)q * NS] = y;
                 x1 = y;
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(32) k_tri_mode(double2 *__restrict__ spec, TriFac f,
+__global__ void __launch_bounds__(32) k_tri_mode(double *__restrict__ spec, TriFac f,
                                                  const unsigned char *__restrict__ flag,
                                                  const double *__restrict__ duc, int nym, long NM) {
-    const long mo = (long)blockIdx.x * 32 + threadIdx.x;
+    const long mo = (long)blockIdx.x * 16 + threadIdx.x / 2;
     const bool act = mo < NM;
     const bool piv = __any_sync(0xffffffffu, act && flag[act ? mo : 0]);
     if (!act) return;
-    if (piv) tri_replay<true>(spec, f, duc, nym, NM, mo);
-    else tri_replay<false>(spec, f, duc, nym, NM, mo);
+    if (piv) tri_replay<true>(spec, f, duc, nym, NM, mo, threadIdx.x & 1);
+    else tri_replay<false>(spec, f, duc, nym, NM, mo, threadIdx.x & 1);
 }
 
 // The tridiagonal systems of many channels in one launch (ensembles): the
@@ -1702,7 +1699,7 @@ static int poisson_solve(cf_ctx *ctx, Fld<T> U, Fld<T> V, Fld<T> W, int phases) 
         else k_tri_split<32><<<nb, tb, sm, ctx->st>>>((float2 *)spec, tf, ts, nym, NM, npb, pw);
         count_launch(ctx, "k_tri_split");
     } else {
-        k_tri_mode<<<(unsigned)cdiv(NM, 32), 32, 0, ctx->st>>>(spec, tf, ctx->tri_flag, ctx->d_tri + 2 * nym, nym, NM);
+        k_tri_mode<<<(unsigned)cdiv(NM, 16), 32, 0, ctx->st>>>((double *)spec, tf, ctx->tri_flag, ctx->d_tri + 2 * nym, nym, NM);
         count_launch(ctx, "k_tri_mode");
     }
     }
