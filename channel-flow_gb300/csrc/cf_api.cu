@@ -505,11 +505,11 @@ extern "C" int cf_create(int nx, int ny, int nz, const double *x, const double *
         eqwm_setup();
         // eddy viscosity: chunks of planes; room for the partials of any chunk length
         if (ctx->esz == 4) {
-            dsm32_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_dsm);
+            ctx->dsm_kc = dsm32_plan(nxp, ctx->nym, nzp, dev_sms);
             nch_dsm = (size_t)dsm32_slots(nxp, nzp, 1);
             ctx->dsmb_nkc = dsm_b_plan(nxp, ctx->nym, nzp, dev_sms);
         } else {
-            dsm64_plan(nxp, ctx->nym, nzp, dev_sms, &ctx->dsm_kc, &nch_dsm);
+            ctx->dsm_kc = dsm64_plan(nxp, ctx->nym, nzp, dev_sms);
             nch_dsm = (size_t)dsm64_slots(nxp, nzp, 1);
         }
         if (ctx->esz == 8) {
@@ -1826,7 +1826,7 @@ static int tune_t(cf_ctx *ctx, int reps, double *rep) {
         double best = 1e300;
         int best_n = keep;
         int last_len = -1;
-        for (int nn = 1; nn <= std::max(1, nzp / 4) && !rc; nn++) {
+        for (int nn = 1; nn <= nzp && !rc; nn++) {
             const int len = cdiv(nzp, nn);
             if (len == last_len) continue;
             last_len = len;
@@ -1845,7 +1845,7 @@ static int tune_t(cf_ctx *ctx, int reps, double *rep) {
         const int keep = ctx->dsm_kc;
         double best = 1e300;
         int best_kc = keep, last_len = -1;
-        for (int nn = 1; nn <= std::max(1, nzp / 4) && !rc; nn++) {
+        for (int nn = 1; nn <= nzp && !rc; nn++) {
             const int len = cdiv(nzp, nn);
             if (len == last_len) continue;
             last_len = len;
@@ -1862,7 +1862,7 @@ static int tune_t(cf_ctx *ctx, int reps, double *rep) {
         const int keep = ctx->amd_nkc;
         double best = 1e300;
         int best_n = keep, last_len = -1;
-        for (int nn = 1; nn <= std::max(1, nzp / 4) && !rc; nn++) {
+        for (int nn = 1; nn <= nzp && !rc; nn++) {
             const int len = cdiv(nzp, nn);
             if (len == last_len || (size_t)amd_partials_for(ctx, nn) > 2 * ctx->dsm_part_nch) continue;
             last_len = len;

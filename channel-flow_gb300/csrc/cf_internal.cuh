@@ -310,10 +310,10 @@ template <typename T> int launch_rhs_update(cf_ctx *ctx, int s, int src, int dst
 template <typename T> int launch_rk_update(cf_ctx *ctx, int s);            // from stored F slots
 template <typename T> int launch_dsm(cf_ctx *ctx, int buf);                // eddy viscosity
 int launch_dsm32(cf_ctx *ctx, int buf, int *nchunk);                       // FP32 pass: |S| and the plane partials
-void dsm32_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
+int dsm32_plan(int nxp, int nym, int nzp, int sms);                         // its z-chunk length
 int dsm32_slots(int nxp, int nzp, int kc);                                 // its partials per row with chunks of kc planes
 int launch_dsm64(cf_ctx *ctx, int buf, int *nchunk);                       // FP64 pass: |S| and the plane partials
-void dsm64_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk);
+int dsm64_plan(int nxp, int nym, int nzp, int sms);                         // its z-chunk length
 int dsm64_slots(int nxp, int nzp, int kc);                                 // its partials per row with chunks of kc planes
 constexpr int CF_ENS_MAXM = 32;  // channels per batched ensemble launch at most
 // fused right-hand sides + RK update of substep s of n split-path channels in one launch

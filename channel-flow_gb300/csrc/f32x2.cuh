@@ -52,3 +52,26 @@ inline int tile_lanes(int nxp) {
         if (cdiv(nxp, 2 * ls) * ls < cdiv(nxp, 2 * best) * best) best = ls;
     return best;
 }
+
+// z-chunk length of a marching kernel with `blocks` tiles and `per` resident
+// blocks per SM: the one that minimises (waves of blocks) x (planes per chunk
+// + 1.5, the planes below and above and the first copies) x (1 + 0.3 for each
+// resident block of an SM past the first: where one wave is not full, fewer
+// blocks run faster; 64^3 right-hand side: 256 blocks of 4 planes 8.6 us, 352
+// of 3 planes 10.4).
+inline int chunk_len(long blocks, int per, int sms, int nzp) {
+    if (per < 1) per = 1;
+    double best_cost = 1e300;
+    int best = nzp;
+    for (int n = 1; n <= nzp; n++) {
+        const int len = cdiv(nzp, n);
+        const long tot = blocks * cdiv(nzp, len);
+        const int b = (int)(tot < (long)per * sms ? cdiv(tot, sms) : per);
+        const double cost = (double)cdiv(tot, (long)per * sms) * (len + 1.5) * (1.0 + 0.3 * (b - 1));
+        if (cost < best_cost - 1e-9) {
+            best_cost = cost;
+            best = len;
+        }
+    }
+    return best;
+}

@@ -264,29 +264,28 @@ __global__ void k_amd_avg(const double *part, int nparts, int nyg, double norm, 
 
 }  // namespace
 
-// z chunks of the AMD pass: the count that minimises (waves of resident
-// blocks) x (planes per chunk + the 2 halo planes a chunk loads again)
+// z chunks of the AMD pass.  FP64: an SM works its blocks off at the FP64
+// pipe's rate, so the count that minimises the mean work of an SM (0.1 plane
+// extra a chunk) and half a chunk for the uneven end (120 x 81 x 96: 6 chunks
+// for one full wave 337 us, 32 to 48 chunks 295 to 299).
 void amd_plan(int esz, int nxp, int nym, int nzp, int sms, int *nkc, int *nparts) {
-    int per = 1;
     if (esz == 4) {
         *nkc = amd32_plan(nxp, nym, nzp, sms);
         *nparts = amd32_parts(nxp, nzp, *nkc);
         return;
     }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd, AMD_TX * AMD_TY, 0);
-    const long tiles = (long)cdiv(nxp, AMD_TX) * cdiv(nym, AMD_TY), res = (long)(per < 1 ? 1 : per) * sms;
-    long best = 1;
+    const double tiles = (double)cdiv(nxp, AMD_TX) * cdiv(nym, AMD_TY);
     double best_cost = 1e300;
-    for (long n = 1; n <= std::max(1L, (long)nzp / 4); n++) {
-        const double waves = (double)((tiles * n + res - 1) / res);
-        const double cost = waves * ((double)cdiv(nzp, n) + 2.0);
+    int best = nzp;
+    for (int n = 1; n <= nzp; n++) {
+        const int len = cdiv(nzp, n);
+        const double cost = tiles * (nzp + 0.1 * cdiv(nzp, len)) / sms + 0.5 * (len + 0.1);
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
-            best = n;
+            best = len;
         }
     }
-    const int kc_len = cdiv(nzp, best);
-    *nkc = cdiv(nzp, kc_len);
+    *nkc = cdiv(nzp, best);
     *nparts = cdiv(nxp, AMD_TX) * *nkc;
 }
 

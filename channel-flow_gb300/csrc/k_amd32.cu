@@ -192,32 +192,16 @@ __global__ void __launch_bounds__(A32_T, 4) k_amd32(const __grid_constant__ A32 
     if (l == 0 && rowok) a.part[(long)(j - 2) * (gridDim.x * gridDim.z) + blockIdx.z * gridDim.x + blockIdx.x] = s;
 }
 
-template <int LS>
-int amd32_blocks_per_sm() {
-    int per = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd32<LS>, A32_T, 0);
-    return std::max(per, 1);
-}
-
 }  // namespace
 
-// z chunks: the count that minimises (waves of resident blocks) x (planes per
-// chunk + 1.5: the plane below the chunk and the first copies)
+// z chunks
 int amd32_plan(int nxp, int nym, int nzp, int sms) {
     const int ls = tile_lanes(nxp);
-    const int per = ls == 32 ? amd32_blocks_per_sm<32>() : (ls == 16 ? amd32_blocks_per_sm<16>() : amd32_blocks_per_sm<8>());
-    const long blocks = (long)cdiv(nxp, 2 * ls) * cdiv(nym, A32_T / ls), res = (long)per * sms;
-    double best_cost = 1e300;
-    int best = 1;
-    for (int n = 1; n <= std::max(1, nzp / 4); n++) {
-        const int len = cdiv(nzp, n);
-        const double cost = (double)cdiv(blocks * cdiv(nzp, len), res) * (len + 1.5);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = n;
-        }
-    }
-    return cdiv(nzp, cdiv(nzp, best));
+    int per = 1;
+    if (ls == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd32<32>, A32_T, 0);
+    else if (ls == 16) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd32<16>, A32_T, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amd32<8>, A32_T, 0);
+    return cdiv(nzp, chunk_len((long)cdiv(nxp, 2 * ls) * cdiv(nym, A32_T / ls), per, sms, nzp));
 }
 
 // partials per row with nkc chunks

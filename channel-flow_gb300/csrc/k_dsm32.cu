@@ -555,25 +555,12 @@ int dsm32_setup() {
     return 0;
 }
 
-// z-chunk length and plane-partial slots per row: the count that minimises
-// (waves of resident blocks of the filter kernel) x (planes per chunk + 1.5
-// for the halo planes)
-void dsm32_plan(int nxp, int nym, int nzp, int sms, int *kc, size_t *nchunk) {
-    const int ls = tile_lanes(nxp), ntx = cdiv(nxp, 2 * ls);
+// z-chunk length (of the filter kernel's blocks; the first kernel's time is
+// within 3 % over a factor of two around it)
+int dsm32_plan(int nxp, int nym, int nzp, int sms) {
+    const int ls = tile_lanes(nxp);
     const int per = ls == 32 ? lm_blocks_per_sm<32>(nxp) : (ls == 16 ? lm_blocks_per_sm<16>(nxp) : lm_blocks_per_sm<8>(nxp));
-    const long blocks = (long)ntx * cdiv(nym, D32_T / ls), res = (long)per * sms;
-    double best_cost = 1e300;
-    int best = 1;
-    for (int n = 1; n <= nzp; n++) {
-        const int len = cdiv(nzp, n);
-        const double cost = (double)cdiv(blocks * cdiv(nzp, len), res) * (len + 1.5);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = len;
-        }
-    }
-    *kc = best;
-    *nchunk = (size_t)ntx * cdiv(nzp, best);
+    return chunk_len((long)cdiv(nxp, 2 * ls) * cdiv(nym, D32_T / ls), per, sms, nzp);
 }
 
 int dsm32_slots(int nxp, int nzp, int kc) { return cdiv(nxp, 2 * tile_lanes(nxp)) * cdiv(nzp, kc); }

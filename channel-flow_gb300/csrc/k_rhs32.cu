@@ -381,27 +381,14 @@ void rhs32_ls(cf_ctx *ctx, const R32 &a, int s) {
 
 }  // namespace
 
-// z chunks: the count that minimises (waves of resident blocks) x (planes per
-// chunk + 1.5: the plane below the chunk, whose upper z fluxes are formed
-// again, and the first copies)
+// z chunks
 int rhs32_plan(int nxp, int nym, int nzp, int sms) {
     const int ls = tile_lanes(nxp);
     int per = 1;
     if (ls == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rhs32<32, 2, true>, R32_T, 0);
     else if (ls == 16) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rhs32<16, 2, true>, R32_T, 0);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rhs32<8, 2, true>, R32_T, 0);
-    const long blocks = (long)cdiv(nxp, 2 * ls) * cdiv(nym, R32_T / ls), res = (long)std::max(per, 1) * sms;
-    double best_cost = 1e300;
-    int best = 1;
-    for (int n = 1; n <= std::max(1, nzp / 4); n++) {
-        const int len = cdiv(nzp, n);
-        const double cost = (double)cdiv(blocks * cdiv(nzp, len), res) * (len + 1.5);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = n;
-        }
-    }
-    return best;
+    return cdiv(nzp, chunk_len((long)cdiv(nxp, 2 * ls) * cdiv(nym, R32_T / ls), per, sms, nzp));
 }
 
 int launch_rhs32(cf_ctx *ctx, int s, int src, int dst) {
