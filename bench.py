@@ -67,10 +67,15 @@ def algorithmic_bytes(kernel: str, c, es: int) -> float | None:
     cs = 2 * es                  # complex spectrum element
     nh = (c.nxp // 2 + 1) * c.nym * c.nzp
     tab = {
-        # the dynamic Smagorinsky pass: read U, V, W, write |S| (4 field accesses per cell)
-        "k_dsm_fused": 4 * nC * es,
+        # the dynamic Smagorinsky pass: U, V, W in, 13 canonical arrays out;
+        # the filtered ones and the filtered velocities in, plane sums out
+        "k_dsm32_q": (3 + 13) * nC * es,
+        "k_dsm32_lm": 12 * nC * es,
+        "k_dsm64_q": (3 + 19) * nC * es,
+        "k_dsm64_lm": 15 * nC * es,
         # the AMD pass: read U, V, W, write nu_t
         "k_amd": 4 * nC * es,
+        "k_amd32": 4 * nC * es,
         # 3 velocity components in, |S| Sij (6), products (6), centre velocities (3), |S| out
         "k_dsm_a": (3 + 16) * nC * es,
         # 15 filtered quantities and Uf, Vf, Wf in (L, M and the plane sums formed in place)
@@ -78,7 +83,10 @@ def algorithmic_bytes(kernel: str, c, es: int) -> float | None:
         # one velocity component in and out
         "k_dsm_c_t": 2 * nC * es,
         "k_dsm_f": 2 * nC * es,
-        # U, V, W, nu_t, Uo (+ lo), F1 in; out + F1 (substep 1 of 3 stores it)
+        # U, V, W, nu_t, u^n (two words in the split path), F1 in, the new
+        # velocities out
+        "k_rhs32": (3 + 1 + 6 + 3 + 3) * nC * es,
+        "k_rhs64": (3 + 1 + 3 + 3 + 3) * nC * es,
         # one component: U, V, W, nu_t, Uo (+ its low word) and F1 in, the new
         # component out (F1 written in substep 1 instead of read)
         "k_rhs": 8 * nC * es,

@@ -462,9 +462,9 @@ class Channel:
 class Ensemble:
     """Independent channels advanced together: one CUDA graph per ensemble
     step with a branch per member (cf_ensemble_*), the tridiagonal systems of
-    all members solved by one FP64 launch per substep (batched_tri), the fused
-    dynamic Smagorinsky passes and fused right-hand sides of all members as
-    one launch each per substep (batched_stencils).  The members stay usable
+    all members solved by one FP64 launch per substep (batched_tri), the
+    right-hand sides of the split-path members as one launch per substep
+    (batched_stencils).  The members stay usable
     as Channel objects between steps."""
 
     def __init__(self, members, batched_tri: bool = True, batched_stencils: bool = False):

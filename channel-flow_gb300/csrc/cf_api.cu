@@ -672,6 +672,7 @@ extern "C" int cf_upload_fields(cf_ctx *ctx, const double *U, const double *V, c
     TRY(put(ctx, ctx->W[b], ctx->Wlo[b], W, ctx->nW));
     ctx->old = ctx->cur;
     CF_CUDA(cudaStreamSynchronize(ctx->st));  // the host arrays may be reused
+    ctx->nut_renew = true;
     return CF_OK;
 }
 
@@ -1214,7 +1215,8 @@ extern "C" int cf_time_step_rk3(cf_ctx *ctx, int nsteps, int sync) {
     CF_CUDA(cudaSetDevice(ctx->dev));
     for (int s = 0; s < nsteps; s++) {
         int X = ctx->cur;
-        if (!ctx->graphs[X]) {
+        const bool renew = ctx->nut_renew, first = !ctx->graphs[X];
+        if (first) {
             // first step from this buffer: count launches eagerly-captured
             cudaGraph_t g = nullptr;
             ctx->launches = 0;
@@ -1243,6 +1245,9 @@ extern "C" int cf_time_step_rk3(cf_ctx *ctx, int nsteps, int sync) {
         CF_CUDA(cudaGraphLaunch(ctx->graphs[X], ctx->st));
         ctx->cur = ctx->next_buf[X];
         ctx->old = ctx->cur;
+        if (ctx->prm.LES_model == 2 && (renew || ctx->cap_renew[X])) ctx->nut_lazy = true;
+        ctx->cap_renew[X] = first && renew;
+        ctx->nut_renew = false;
     }
     if (sync) {
         CF_CUDA(cudaStreamSynchronize(ctx->st));
@@ -1470,12 +1475,14 @@ extern "C" int cf_profile_graph_steps(cf_ctx *ctx, int nsteps, int max_names, ch
 // run concurrently on the GPU, so small grids fill it together.
 // ---------------------------------------------------------------------------
 #include <map>
+#include <set>
 
 struct cf_ensemble {
     std::vector<cf_ctx *> m;
     int dev = 0;
     bool batched_tri = true;          // one FP64 launch for every member's tridiagonal systems
     bool batched_stencils = false;    // one launch for every member's fused DSM pass and fused RHS
+    std::set<std::vector<int>> cap_renew;  // graphs captured by a step whose members' states were just uploaded
     TriMember *dtab = nullptr;        // device table of the members' systems
     double2 *scratch = nullptr;       // FP64 elimination scratch of every member
     long total_modes = 0;             // blocks of the batched launch
@@ -1655,7 +1662,10 @@ extern "C" int cf_ensemble_step(cf_ensemble *e, int nsteps, int sync) {
         std::vector<int> key(n);
         for (int q = 0; q < n; q++) key[q] = e->m[q]->cur;
         auto it = e->graphs.find(key);
-        if (it == e->graphs.end()) {
+        const bool first = it == e->graphs.end();
+        bool renew = false;
+        for (cf_ctx *c : e->m) renew = renew || c->nut_renew;
+        if (first) {
             cudaGraph_t g;
             int total_tri = 0;
             for (cf_ctx *c : e->m) {
@@ -1711,6 +1721,13 @@ extern "C" int cf_ensemble_step(cf_ensemble *e, int nsteps, int sync) {
             e->m[q]->cur = it->second.second[q];
             e->m[q]->old = e->m[q]->cur;
         }
+        // as in cf_time_step_rk3
+        const bool set = renew || e->cap_renew.erase(key) > 0;
+        for (cf_ctx *c : e->m) {
+            if (set && c->prm.LES_model == 2) c->nut_lazy = true;
+            c->nut_renew = false;
+        }
+        if (first && renew) e->cap_renew.insert(key);
     }
     // the members' own streams see the ensemble's work before anything they do next
     ENS_CUDA(cudaEventRecord(e->fork, e->st));

@@ -241,6 +241,12 @@ struct cf_ctx {
     // the plane coefficient <LM>/<MM>: the fused RHS forms nu_t on the fly and
     // the nut buffer is filled only when another reader needs it.
     bool nut_lazy = false;
+    // The state was uploaded and apply_boundary_conditions has not been called
+    // since: the next step leaves nut_lazy set (its replay launches the eddy
+    // viscosity without the host's flag seeing it), and so does the first
+    // replay of a graph captured by such a step.
+    bool nut_renew = true;
+    bool cap_renew[3] = {false, false, false};
     // pressure
     void *phi = nullptr;               // canonical real
     void *spec = nullptr;              // complex spectrum [j][kz][kx]: mode m = kz*nxh + kx contiguous per row

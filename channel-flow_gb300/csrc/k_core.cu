@@ -132,6 +132,7 @@ int launch_bc(cf_ctx *ctx, int b, bool lo) {
     s.dyb = ctx->hyg[2] - ctx->hyg[1];
     s.dyt = ctx->hyg[ctx->nyg] - ctx->hyg[ctx->nyg - 1];
     const int tot = s.f[0].n + s.f[1].n + s.f[2].n;
+    ctx->nut_renew = false;
     k_bc<T><<<cdiv(tot, 256), 256, 0, ctx->st>>>(s);
     count_launch(ctx, "k_bc");
     CF_CUDA(cudaGetLastError());

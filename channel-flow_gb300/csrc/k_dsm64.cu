@@ -5,7 +5,7 @@
 // sub-partitions one per 64-76), whatever the number of resident warps, so
 // the pass costs its FP64 instructions and nothing else: about 240 a cell
 // here, in 4.7 M cells 2.1 ms, against 0.25 ms for the 300 bytes a cell that
-// go through memory.  (The one-pass kernel of the FP32 path in FP64 took
+// go through memory.  (A one-pass tile kernel took
 // 539: the halo of its tiles is computed 1.4 times over, its strain rates
 // take every difference by itself, and its filters a multiply for each
 // weight; 7.0 ms per pass at 192 x 128 x 192 cells, where its tiles also

@@ -58,10 +58,10 @@ typedef struct {
     int sgs_recompute;     /* 1: evaluate the second eddy viscosity of substep 1
                               (time_integration.f90:103) inside cf_time_step_rk3;
                               0: reuse the first one (bit-identical inputs)      */
-    int dsm_unfused;       /* 1: evaluate the dynamic Smagorinsky model with the
-                              multi-pass kernels even where the fused pass applies;
-                              2: the same with the filter kernel's per-element
-                              plane gather instead of tensor copies             */
+    int dsm_unfused;       /* split path: 1: evaluate the dynamic Smagorinsky model
+                              with the multi-pass kernels (a cross-check); 2: the
+                              same with the filter kernel's per-element plane
+                              gather instead of tensor copies.  FP64: no effect */
     int cfl_corrected;     /* 1: convective limit of compute_dt with the minimum
                               over cells of spacing/|u| (the reference takes the
                               maximum, time_integration.f90:191-201, which leaves
@@ -330,12 +330,11 @@ int cf_ensemble_launches_per_step(cf_ensemble *e);
  * their FP32 spectra); 0: each member solves its own systems inside its
  * branch, bit for bit as cf_time_step_rk3. */
 int cf_ensemble_set_batched_tri(cf_ensemble *e, int on);
-/* 1 (up to 32 members; default 0): the fused dynamic Smagorinsky pass of
- * every member that takes it (no wall model) and the fused right-hand sides
- * of all members run as one launch each per substep, every (member, tile) a
- * block of it -- per member the same arithmetic as its own launch; the
- * other kernels stay in the members' branches.  0: every kernel in the
- * members' branches. */
+/* 1 (up to 32 members; default 0): the right-hand sides of all split-path
+ * members run as one launch per substep, every (member, tile) a block of it
+ * -- per member the same arithmetic as its own launch (FP64 members: their
+ * own launches, at the same place of the step); the other kernels stay in
+ * the members' branches.  0: every kernel in the members' branches. */
 int cf_ensemble_set_batched_stencils(cf_ensemble *e, int on);
 /* Empirical choice of how the ensemble runs its stencil passes and its
  * tridiagonal solves: one whole ensemble step per candidate captures its

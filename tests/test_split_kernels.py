@@ -112,3 +112,37 @@ def test_amd_tiles_and_chunks(dims, rule):
     assert rel_err(b.avg_nu_t()[1:-1], a.avg_nu_t()[1:-1]) <= 2e-4
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_nut_of_steps_after_uploads(prec):
+    """nu_t downloaded after each step of a state uploaded without its ghosts
+    filled, and after a step of each of several uploads: bit for bit that of a
+    channel that is stepped once from the upload on and downloaded once."""
+    import channelflow as cf
+    case = channel_case(18, 9, 18, mass=0)
+
+    def make(scale):
+        ch = cf.Channel(case["x"], case["y"], case["z"], precision=prec, **case["prm"])
+        ch.upload(scale * case["U"], scale * case["V"], scale * case["W"])
+        ch.set_fixed_dt(case["dt"])
+        return ch
+
+    ch = make(1.0)
+    for n in range(1, 5):
+        ch.time_step_rk3(1)
+        got = ch.download()["nu_t"]
+        ref = make(1.0)
+        ref.time_step_rk3(n)
+        assert np.array_equal(got, ref.download()["nu_t"]), n
+        ref.close()
+    for n in range(6):
+        scale = 1.0 + 0.1 * n
+        ch.upload(scale * case["U"], scale * case["V"], scale * case["W"])
+        ch.time_step_rk3(1)
+        got = ch.download()["nu_t"]
+        ref = make(scale)
+        ref.time_step_rk3(1)
+        assert np.array_equal(got, ref.download()["nu_t"]), scale
+        ref.close()
+    ch.close()
