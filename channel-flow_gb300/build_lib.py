@@ -48,9 +48,7 @@ def build(verbose: bool = False, extra: list[str] | None = None) -> str:
         src, obj = os.path.join(CSRC, s), os.path.join(BUILD, s + ".o")
         objs.append(obj)
         if _newer(src, obj, hdrs):
-            # the transforms' compile-time lengths are many kernels in one file
-            split = ["--split-compile=0"] if s == "k_poisson.cu" else []
-            jobs.append([NVCC] + ARCH + CU_FLAGS + split + (extra or []) + ["-c", src, "-o", obj])
+            jobs.append([NVCC] + ARCH + CU_FLAGS + (extra or []) + ["-c", src, "-o", obj])
     for s in CXX_SOURCES:
         src, obj = os.path.join(CSRC, s), os.path.join(BUILD, s + ".o")
         objs.append(obj)
