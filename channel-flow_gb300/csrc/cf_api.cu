@@ -1481,7 +1481,7 @@ struct cf_ensemble {
     std::vector<cf_ctx *> m;
     int dev = 0;
     bool batched_tri = true;          // one FP64 launch for every member's tridiagonal systems
-    bool batched_stencils = false;    // one launch for every member's fused DSM pass and fused RHS
+    bool batched_stencils = false;    // one launch for every split-path member's right-hand sides
     std::set<std::vector<int>> cap_renew;  // graphs captured by a step whose members' states were just uploaded
     TriMember *dtab = nullptr;        // device table of the members' systems
     double2 *scratch = nullptr;       // FP64 elimination scratch of every member
@@ -1739,7 +1739,7 @@ extern "C" int cf_ensemble_step(cf_ensemble *e, int nsteps, int sync) {
 // Empirical choice of how an ensemble runs its stencil passes: the whole
 // ensemble step is timed (CUDA events, `steps` steps after one that captures
 // its graph) for every member kernel in its branch with each member's own
-// z-chunk plan, and for the batched DSM / right-hand-side launches with the
+// z-chunk plan, and for the batched right-hand-side launches with the
 // members' plans, with one z chunk per member and with two; the fastest is
 // kept.  The ensemble advances 4 x (steps + 1) steps.  report (4 doubles,
 // may be NULL): ms per step of the four candidates in that order; *choice
