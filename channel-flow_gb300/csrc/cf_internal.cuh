@@ -10,6 +10,7 @@
 // the nxp x nym x nzp unique cells (i = 2..nx-1, j = 2..nyg-1, k = 2..nz-1),
 // read through the periodic wrap  i -> 2 + (i-2) mod nxp.
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -45,6 +46,34 @@ __host__ __device__ static inline Fld<T> make_fld(void *p, int n1, int n2) {
     f.sz = n1 * n2;
     f.off = 1 + f.sy + f.sz;
     return f;
+}
+
+// z-chunk length of an FP64 marching kernel with `blocks` tiles, two blocks
+// resident per SM, `least` chunks at least.  An SM works its blocks off at the
+// FP64 pipe's rate, a block alone at 1/0.6 of its speed beside another; a
+// chunk of len planes costs len + head.  The time of a length is that of
+// dealing its full chunks and then the short last ones to the resident places
+// in order.
+inline int fp64_chunk_len(long blocks, int sms, int nzp, int least, double head) {
+    const long res = 2L * sms;
+    double best_cost = 1e300;
+    int best = 1;
+    for (int n = least; n <= nzp; n++) {
+        const int len = (nzp + n - 1) / n, nn = (nzp + len - 1) / len, last = nzp - (nn - 1) * len;
+        const long full = blocks * (last == len ? nn : nn - 1), rest = last == len ? 0 : blocks;
+        const double d = len + head, e = last + head;
+        const long r = full % res, room = res - r;
+        double tail = r ? d : 0.0;
+        if (rest > room) tail = std::max(tail, std::min(e * ((rest + room - 1) / room), (r * d + rest * e) / res + e));
+        else if (rest) tail = std::max(tail, e);
+        if (r + rest <= sms) tail *= 0.6;
+        const double cost = (double)(full / res) * d + tail;
+        if (cost < best_cost - 1e-9) {
+            best_cost = cost;
+            best = len;
+        }
+    }
+    return best;
 }
 
 // rk_coef (initialization.f90:408-416)

@@ -372,33 +372,11 @@ int d64_w(int nxp) { return cdiv(nxp, 16) * 16 < cdiv(nxp, 32) * 32 ? 16 : 32; }
 
 }  // namespace
 
-// z-chunk length.  An SM works its blocks off at the FP64 pipe's rate however
-// many are resident (two fit), a block alone at 1.6 times its speed beside
-// another; a chunk of len planes costs len + 0.9 (its halo planes).  The time
-// of a length is that of dealing its full chunks and then the short last ones
-// to the resident places in order (192 x 128 x 192: 28 planes, whose last
-// wave is nearly empty, 2.55 ms a pass; 18 to 24 planes 2.36).
+// z-chunk length (192 x 128 x 192: 28 planes, whose last wave is nearly
+// empty, 2.55 ms a pass; 18 to 24 planes 2.36)
 int dsm64_plan(int nxp, int nym, int nzp, int sms) {
     const int w = d64_w(nxp), nseg = cdiv(nxp, w);
-    const long blocks = cdiv((long)nseg * nym, (32 / w) * (D64_T / 32)), res = 2L * sms;
-    double best_cost = 1e300;
-    int best = 1;
-    for (int n = 1; n <= nzp; n++) {
-        const int len = cdiv(nzp, n), nn = cdiv(nzp, len), last = nzp - (nn - 1) * len;
-        const long full = blocks * (last == len ? nn : nn - 1), rest = last == len ? 0 : blocks;
-        const double d = len + 0.9, e = last + 0.9;
-        const long r = full % res, room = res - r;
-        double tail = r ? d : 0.0;
-        if (rest > room) tail = std::max(tail, std::min(e * cdiv(rest, room), (r * d + rest * e) / res + e));
-        else if (rest) tail = std::max(tail, e);
-        if (r + rest <= sms) tail *= 0.62;
-        const double cost = (double)(full / res) * d + tail;
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = len;
-        }
-    }
-    return best;
+    return fp64_chunk_len(cdiv((long)nseg * nym, (32 / w) * (D64_T / 32)), sms, nzp, 1, 0.9);
 }
 
 // (three per segment and chunk where its components are split)

@@ -292,22 +292,11 @@ R64Plan r64_shape(int nxp, int nym) {
 
 }  // namespace
 
-// z chunks: the count that minimises (warps on the busiest SM) x (planes per
-// chunk + 0.5 for the head plane)
+// z chunks (64 x 48 x 64: 10 chunks, one block an SM, 66 us; 22 chunks 60)
 int rhs64_plan(int nxp, int nym, int nzp, int sms) {
     const R64Plan p = r64_shape(nxp, nym);
     const long blocks = (long)cdiv(nxp, p.w) * cdiv(nym, p.rb);
-    int best = cdiv(nzp, R64_ZMAX);
-    double best_cost = 1e300;
-    for (int n = best; n <= nzp; n++) {
-        const int len = cdiv(nzp, n);
-        const double cost = (double)cdiv(blocks * cdiv(nzp, len), sms) * (len + 0.5);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = n;
-        }
-    }
-    return best;
+    return cdiv(nzp, fp64_chunk_len(blocks, sms, nzp, cdiv(nzp, R64_ZMAX), 0.5));
 }
 
 static R64 r64_args(cf_ctx *ctx, int src, const R64Plan &p) {

@@ -342,7 +342,7 @@ int cf_ensemble_set_batched_stencils(cf_ensemble *e, int on);
  * member solves its own tridiagonal systems (as cf_time_step_rk3); 4-7: one
  * FP64 launch for all members' systems.  Within each group: (+0) every
  * kernel in the members' branches with each member's own z-chunk plan, and
- * the batched DSM / right-hand-side launches with (+1) the members' plans,
+ * the batched right-hand-side launches with (+1) the members' plans,
  * (+2) one z chunk per member, (+3) two.  The fastest is kept.  The ensemble
  * advances CF_ENS_TUNE_CANDIDATES (steps + 1) steps.  report
  * (CF_ENS_TUNE_CANDIDATES doubles, may be NULL): ms per step of each
