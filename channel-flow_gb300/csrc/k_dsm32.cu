@@ -76,8 +76,8 @@ __device__ __forceinline__ float2 wz(float2 &h, float2 &l, float2 x) {
 // 1/3 and 2/3 are its double and quadruple).  L is a small difference of
 // hat(u u) and hat(u) hat(u), which those weights, 3e-8 above 1 in sum, move
 // by -9e-8 u u; the factor between the two, FS / 1024, is taken as the product
-// of two FP32 numbers 3e-8 below it (-6e-8 u u; one FP32 number has 1e-7
-// between its neighbours).  Powers of two keep the filtered quantities'
+// of two FP32 numbers 1.8e-8 below it (-7e-8 u u; the nearest FP32 number is
+// 1.9e-8 above it: -11e-8).  Powers of two keep the filtered quantities'
 // squares near their unscaled size.
 constexpr double W6 = double(float(1.0 / 6.0)), FS = W6 * W6 * W6;
 constexpr float SC_U = 1.f / 32.f;                // sum of two faces -> centre velocity / 16

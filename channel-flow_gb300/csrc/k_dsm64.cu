@@ -9,7 +9,7 @@
 // 539: the halo of its tiles is computed 1.4 times over, its strain rates
 // take every difference by itself, and its filters a multiply for each
 // weight; 7.0 ms per pass at 192 x 128 x 192 cells, where its tiles also
-// filled 63 % of the block slots.)
+// filled 63 % of the block slots.  The two kernels: 0.84 + 1.52 ms.)
 //
 // A warp owns a segment of W = 32 or 16 adjacent columns of one row j and
 // marches along z over a chunk of planes; W = 16 packs two rows into a warp

@@ -8,8 +8,8 @@
 // fluxes at the cell centres and, at each edge, the product of the two
 // interpolated velocities, the edge viscosity and the two velocity
 // differences for both components that use them -- about 105 instructions a
-// cell instead of 191 of the tile kernel of the FP32 path in FP64, which
-// forms the x and y fluxes in both neighbouring cells.
+// cell instead of 191 of a tile kernel that forms the x and y fluxes in both
+// neighbouring cells (1691 -> 1075 us a launch at 192 x 128 x 192).
 //
 // A warp owns a segment of W = 32 or 16 columns of one row and marches along
 // z.  Fluxes on a cell's upper faces and edges are formed by its own lane;
