@@ -184,59 +184,65 @@ __device__ __forceinline__ void rhs32_tile(const R32 &a, float (*st)[4][R32_NPMA
         const float2 sb = add2(nbc, nb.q), sn = add2(nnbc, nnb.q);     // nu_t of both cells of an x face
         const float2 zb = add2(nbc, nnbc);                             // of a z face
         auto flux = [](float2 ne, float2 g, float2 A) { return fma2(ne, g, mul2(A, sp(-1.f))); };
+        // difference of two products in x: a b of the pair less those one cell to
+        // the left (aL bL, a.x b.x); in y: a b + c d with c negated.  One of the
+        // two products is not rounded.
+        auto dx = [](float2 a, float2 b, float aL, float bL) {
+            return f2(fmaf(a.x, b.x, -(aL * bL)), fmaf(a.y, b.y, -(a.x * b.x)));
+        };
+        auto dy = [](float2 a, float2 b, float2 c, float2 d) { return fma2(a, b, mul2(c, d)); };
+        const float2 uac = ua.c(), vac = va.c();
+        // minus the quantities of the edges and faces below (nu_t, velocities)
+        const float2 zna = add2(na.c(), nna.c());
         float2 ru, rv, rw;
         {  // xy edge (i+1/2, j+1/2): u through the y face, v through the x face
             const float2 ne = fma2(sp(w1), add2(nc.c(), nc.q), fma2(sp(w0), sb, sp(nu2)));
-            const float2 ucc = uc.c(), A = mul2(fma2(sp(w1), ucc, mul2(sp(w0), u0)), add2(v0, vb.q));
-            const float2 gr = mul2(sub2(ucc, u0), sp(ryg1)), dV = sub2(vb.q, v0);
-            const float2 yu = flux(ne, fma2(dV, rx1, gr), A), xv = flux(ne, fma2(dV, rxg1, gr), A);
+            const float2 ucc = uc.c(), P = fma2(sp(w1), ucc, mul2(sp(w0), u0)), Q = add2(v0, vb.q);
+            const float2 gr = mul2(sub2(ucc, u0), sp(ryg1)), dV = sub2(vb.q, v0), gx = fma2(dV, rxg1, gr);
             // v through the face left of the pair
             const float neL = fmaf(w1, nc.p.x + nc.p.y, fmaf(w0, nb.p.x + nb.p.y, nu2));
-            const float AL = fmaf(w1, uc.p.x, w0 * ub.p.x) * (vb.p.x + vb.p.y);
-            const float xvL = fmaf(neL, fmaf(vb.p.y - vb.p.x, rxg0.x, (uc.p.x - ub.p.x) * ryg1), -AL);
-            rv = mul2(mul2(rx, sp(0.5f)), f2(xv.x - xvL, xv.y - xv.x));
+            const float PL = fmaf(w1, uc.p.x, w0 * ub.p.x), QL = vb.p.x + vb.p.y;
+            const float gL = fmaf(vb.p.y - vb.p.x, rxg0.x, (uc.p.x - ub.p.x) * ryg1);
+            rv = mul2(mul2(rx, sp(0.5f)), sub2(dx(ne, gx, neL, gL), dx(P, Q, PL, QL)));
             // (j-1/2): u through the y face below
-            const float2 nea = fma2(sp(w1m), sb, fma2(sp(w0m), add2(na.c(), na.q), sp(nu2)));
-            const float2 uac = ua.c(), vac = va.c(), Aa = mul2(fma2(sp(w1m), u0, mul2(sp(w0m), uac)), add2(vac, va.q));
-            const float2 yul = flux(nea, fma2(sub2(va.q, vac), rx, mul2(sub2(u0, uac), sp(ryg0))), Aa);
-            ru = mul2(sub2(yu, yul), sp(0.5f * ry));
+            const float2 nea = fma2(sp(-w1m), sb, fma2(sp(-w0m), add2(na.c(), na.q), sp(-nu2)));
+            const float2 Pa = fma2(sp(-w1m), u0, mul2(sp(-w0m), uac)), Qa = add2(vac, va.q);
+            const float2 gy = fma2(dV, rx1, gr), ga = fma2(sub2(va.q, vac), rx, mul2(sub2(u0, uac), sp(ryg0)));
+            ru = mul2(sub2(dy(ne, gy, nea, ga), dy(P, Q, Pa, Qa)), sp(0.5f * ry));
             // v through the centres of rows j+1 and j
             const float2 vcc = vc.c(), s1 = add2(v0, vcc), s0 = add2(vac, v0);
-            const float2 yv = flux(mul2(add2(nc.c(), sp(nu)), sp(8.f * ry1)), sub2(vcc, v0), mul2(s1, s1));
-            const float2 yvl = flux(mul2(add2(nbc, sp(nu)), sp(8.f * ry)), sub2(v0, vac), mul2(s0, s0));
-            rv = fma2(sub2(yv, yvl), sp(0.25f * ryg1), rv);
+            const float2 m1 = mul2(add2(nc.c(), sp(nu)), sp(8.f * ry1)), m0 = mul2(add2(nbc, sp(nu)), sp(-8.f * ry));
+            rv = fma2(sub2(dy(m1, sub2(vcc, v0), m0, sub2(v0, vac)), dy(s1, s1, mul2(s0, sp(-1.f)), s0)), sp(0.25f * ryg1), rv);
         }
         {  // u through the centres of columns i+1 (both cells') and i
-            const float2 s1 = add2(u0, ub.q);
-            const float2 xu = flux(mul2(add2(nb.q, sp(nu)), mul2(rx1, sp(8.f))), sub2(ub.q, u0), mul2(s1, s1));
-            const float s0 = ub.p.x + ub.p.y, xuL = fmaf((nu + nb.p.y) * (8.f * rx.x), ub.p.y - ub.p.x, -(s0 * s0));
-            ru = fma2(mul2(rxg1, sp(0.25f)), f2(xu.x - xuL, xu.y - xu.x), ru);
+            const float2 s1 = add2(u0, ub.q), m1 = mul2(add2(nb.q, sp(nu)), mul2(rx1, sp(8.f)));
+            const float s0 = ub.p.x + ub.p.y, m0 = (nu + nb.p.y) * (8.f * rx.x);
+            ru = fma2(mul2(rxg1, sp(0.25f)), sub2(dx(m1, sub2(ub.q, u0), m0, ub.p.y - ub.p.x), dx(s1, s1, s0, s0)), ru);
         }
         float2 zu, zv, zw;
         {  // xz edge (i+1/2, k+1/2): u through the z face, w through the x face
-            const float2 ne = add2(sp(nu4), add2(sb, sn)), A = mul2(add2(u0, u1), add2(w_0, wb.q));
+            const float2 ne = add2(sp(nu4), add2(sb, sn)), P = add2(u0, u1), Q = add2(w_0, wb.q), A = mul2(P, Q);
             const float2 dU = sub2(u1, u0), dW = sub2(wb.q, w_0), gz = mul2(dU, sp(z3)), gx = mul2(dW, rxg1);
             const float2 zup = flux(ne, fma2(dW, rx1, gz), A);
             zu = flux(ne, fma2(dW, rx, gz), A);
-            const float2 xw = flux(ne, fma2(dU, sp(z2), gx), A);
-            const float xwl = fmaf(ne.x, fmaf(dU.x, z1, gx.x), -A.x);
+            const float2 g = fma2(dU, sp(z2), gx);
             const float neL = nu4 + ((nb.p.x + nb.p.y) + (nnb.p.x + nnb.p.y));
-            const float AL = (ub.p.x + un.p.x) * (wb.p.x + wb.p.y);
-            const float xwL = fmaf(neL, fmaf(un.p.x - ub.p.x, z1, (wb.p.y - wb.p.x) * rxg0.x), -AL);
+            const float PL = ub.p.x + un.p.x, QL = wb.p.x + wb.p.y;
+            const float gL = fmaf(un.p.x - ub.p.x, z1, (wb.p.y - wb.p.x) * rxg0.x);
+            const float2 v = f2(fmaf(ne.x, g.x, -(neL * gL)), fmaf(ne.y, g.y, -(ne.x * fmaf(dU.x, z1, gx.x))));
             ru = fma2(sub2(zup, zu_l), sp(0.25f * z1), ru);
-            rw = mul2(mul2(rx, sp(0.25f)), f2(xw.x - xwL, xw.y - xwl));
+            rw = mul2(mul2(rx, sp(0.25f)), sub2(v, dx(P, Q, PL, QL)));
         }
         {  // yz edges (j+1/2, k+1/2) and (j-1/2, k+1/2): v through the z face, w through the y face
             const float2 ne = fma2(sp(w1), add2(nc.c(), nnc.c()), fma2(sp(w0), zb, sp(nu2)));
-            const float2 A = mul2(add2(v0, v1), fma2(sp(w1), w1c, mul2(sp(w0), w_0)));
+            const float2 P = add2(v0, v1), Q = fma2(sp(w1), w1c, mul2(sp(w0), w_0));
             const float2 dV = sub2(v1, v0), gW = mul2(sub2(w1c, w_0), sp(ryg1));
-            zv = flux(ne, fma2(dV, sp(z3), gW), A);
-            const float2 yw = flux(ne, fma2(dV, sp(z2), gW), A);
-            const float2 nea = fma2(sp(w1m), zb, fma2(sp(w0m), add2(na.c(), nna.c()), sp(nu2)));
-            const float2 vac = va.c(), vnac = vna.c(), Aa = mul2(add2(vac, vnac), fma2(sp(w1m), w_0, mul2(sp(w0m), wac)));
-            const float2 ywl = flux(nea, fma2(sub2(vnac, vac), sp(z1), mul2(sub2(w_0, wac), sp(ryg0))), Aa);
+            zv = flux(ne, fma2(dV, sp(z3), gW), mul2(P, Q));
+            const float2 nea = fma2(sp(-w1m), zb, fma2(sp(-w0m), zna, sp(-nu2)));
+            const float2 vnac = vna.c(), Pa = add2(vac, vnac), Qa = fma2(sp(-w1m), w_0, mul2(sp(-w0m), wac));
+            const float2 ga = fma2(sub2(vnac, vac), sp(z1), mul2(sub2(w_0, wac), sp(ryg0)));
             rv = fma2(sub2(zv, zv_l), sp(0.5f * z1), rv);
-            rw = fma2(sub2(yw, ywl), sp(0.5f * ry), rw);
+            rw = fma2(sub2(dy(ne, fma2(dV, sp(z2), gW), nea, ga), dy(P, Q, Pa, Qa)), sp(0.5f * ry), rw);
         }
         {  // w through the centre of plane k+1
             const float2 wnc = wn.c(), s = add2(w_0, wnc);
@@ -253,7 +259,7 @@ __device__ __forceinline__ void rhs32_tile(const R32 &a, float (*st)[4][R32_NPMA
         nc = nnc;
         if (a.rot) {
             // equations.f90:169-177, 334-342
-            const float2 vac = va.c(), h = sp(0.25f), m = sp(2.f * a.Om);
+            const float2 h = sp(0.25f), m = sp(2.f * a.Om);
             ru = fma2(m, mul2(h, add2(add2(vac, v0), add2(va.q, vb.q))), ru);
             const float2 q = fma2(sp(w0), add2(ub.p, u0), mul2(sp(w1), add2(uc.p, uc.c())));
             rv = fma2(mul2(m, sp(-0.5f)), q, rv);
